@@ -29,6 +29,7 @@
 #include "rt_aerosol.cuh"
 #include "rt_prep.cuh"
 #include "rt_column.cuh"
+#include "rt_stage.cuh"
 #include "tables.h"
 #include <nvtx3/nvToolsExt.h>
 
@@ -37,6 +38,7 @@ __global__ void rt_fp64_kernel(const SegTable *__restrict__ st, const double *__
                                const double *__restrict__ ki, const double *__restrict__ planck,
                                const RtConst K, int max_nl, uint32_t *status,
                                unsigned long long *nsys, double *red_scratch);
+template <bool V>
 __global__ void rt_stage(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                          unsigned char *__restrict__ blocks, size_t stride,
                          const double *__restrict__ planck, const RtConst K, uint32_t *status);
@@ -212,55 +214,40 @@ constexpr int SERVE_JOB_COLS = MGCM_SERVE_JOB_COLS;   // columns per job of a se
 constexpr int SERVE_SLOTS = 4;          // serving slots at most
 
 // ---------------------------------------------------------------- validation
+// A warp per column, lanes along each array (a thread per column walked 35 KB
+// of strided reads by itself).
 __global__ void validate_kernel(const SegTable *__restrict__ st, uint32_t *status) {
-    const int total = st->total_cols;
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        const int si = find_seg(st, g);
-        const SegDev &sg = st->seg[si];
-        const int c = g - sg.col0, L = sg.L, LEV = 2 * L + 3, LEV1 = LEV + 1;
-        uint32_t bad = 0;
-        auto fin = [&](const double *p, size_t n) {
-            if (!p) return;
-            for (size_t i = 0; i < n; ++i)
-                if (!isfinite(p[i])) { bad |= ST_NONFINITE; return; }
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < st->total_cols; g += nwarps) {
+        const SegDev &sg = st->seg[find_seg(st, g)];
+        const size_t c = (size_t)(g - sg.col0);
+        const int L = sg.L, LEV = 2 * L + 3, LEV1 = LEV + 1;
+        Check<true> chk;
+        auto fin = [&](const double *base, int n, int per) {   // n of the column's `per` values
+            if (base)
+                for (int i = lane; i < n; i += 32) chk.finite(base[c * per + i]);
         };
-        fin(sg.plev + (size_t)c * LEV, LEV);
-        fin(sg.tlev + (size_t)c * LEV, LEV);
-        fin(sg.pmid + (size_t)c * LEV, LEV);
-        fin(sg.tmid + (size_t)c * LEV, LEV);
-        fin(sg.qh2o + (size_t)c * LEV, LEV);
-        fin(sg.tauref + (size_t)c * LEV1, sg.dust_band ? LEV : LEV1);   // TAUREF(LEV+1) is 0 then
-        fin(sg.qextrefdst + (size_t)c * LEV1, LEV1);
-        fin(sg.qxvdst + (size_t)c * 7 * LEV1, 7 * LEV1);
-        fin(sg.qsvdst + (size_t)c * 7 * LEV1, 7 * LEV1);
-        fin(sg.gvdst + (size_t)c * 7 * LEV1, 7 * LEV1);
-        fin(sg.qxidst + (size_t)c * 5 * LEV1, 5 * LEV1);
-        fin(sg.qsidst + (size_t)c * 5 * LEV1, 5 * LEV1);
-        fin(sg.gidst + (size_t)c * 5 * LEV1, 5 * LEV1);
+        for (int i = lane; i < LEV; i += 32) {
+            chk.pressure(sg.plev[c * LEV + i]);
+            chk.pressure(sg.pmid[c * LEV + i]);
+            chk.temperature(sg.tlev[c * LEV + i]);
+        }
+        fin(sg.tmid, LEV, LEV);
+        fin(sg.qh2o, LEV, LEV);
+        fin(sg.tauref, sg.dust_band ? LEV : LEV1, LEV1);   // TAUREF(LEV+1) is 0 then
+        fin(sg.qextrefdst, LEV1, LEV1);
+        for (const double *p : {sg.qxvdst, sg.qsvdst, sg.gvdst}) fin(p, 7 * LEV1, 7 * LEV1);
+        for (const double *p : {sg.qxidst, sg.qsidst, sg.gidst}) fin(p, 5 * LEV1, 5 * LEV1);
         if (sg.taurefcld) {
-            fin(sg.taurefcld + (size_t)c * LEV1, LEV1);
-            fin(sg.qextrefcld + (size_t)c * LEV1, LEV1);
-            fin(sg.qxvcld + (size_t)c * 7 * LEV1, 7 * LEV1);
-            fin(sg.qsvcld + (size_t)c * 7 * LEV1, 7 * LEV1);
-            fin(sg.gvcld + (size_t)c * 7 * LEV1, 7 * LEV1);
-            fin(sg.qxicld + (size_t)c * 5 * LEV1, 5 * LEV1);
-            fin(sg.qsicld + (size_t)c * 5 * LEV1, 5 * LEV1);
-            fin(sg.gicld + (size_t)c * 5 * LEV1, 5 * LEV1);
+            fin(sg.taurefcld, LEV1, LEV1);
+            fin(sg.qextrefcld, LEV1, LEV1);
+            for (const double *p : {sg.qxvcld, sg.qsvcld, sg.gvcld}) fin(p, 7 * LEV1, 7 * LEV1);
+            for (const double *p : {sg.qxicld, sg.qsicld, sg.gicld}) fin(p, 5 * LEV1, 5 * LEV1);
         }
-        fin(sg.acosz + c, 1);
-        fin(sg.als + c, 1);
-        fin(sg.albi + c, 1);
-        fin(sg.pcol + c, 1);
-        fin(sg.detau + (size_t)c * 119, 119);
-        const double *pl = sg.plev + (size_t)c * LEV, *pm = sg.pmid + (size_t)c * LEV;
-        for (int k = 0; k < LEV; ++k)
-            if (!(pl[k] > 0.0) || !(pm[k] > 0.0)) bad |= ST_NONFINITE;
-        const double *tl = sg.tlev + (size_t)c * LEV;
-        for (int k = 0; k < LEV; ++k) {
-            const double x = __dsub_rn(__dmul_rn(tl[k], 10.0), 499.0);
-            if (!(x >= 1.0 && x < 8502.0)) bad |= ST_TEMP;
-        }
-        if (bad) atomicOr(status, bad);
+        for (const double *p : {sg.acosz, sg.als, sg.albi, sg.pcol}) fin(p, 1, 1);
+        fin(sg.detau, 119, 119);
+        chk.report(status);
     }
 }
 
@@ -516,6 +503,12 @@ int arena_ensure(mgcm_rt_handle *h, Arena &a, size_t bytes, cudaStream_t s) {
     return MGCM_RT_OK;
 }
 
+// The input checks as a kernel of their own, for the forms without rt_stage.
+void launch_validate(mgcm_rt_handle *h, const SegTable *segs, uint32_t *status, int total, cudaStream_t st) {
+    const int vb = std::max(1, std::min((total + 7) / 8, h->num_sms * 8));
+    validate_kernel<<<vb, 256, 0, st>>>(segs, status);
+}
+
 int slot_init(Slot &s) {
     CK(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&s.aux, cudaStreamNonBlocking));
@@ -604,8 +597,9 @@ size_t pipe_bytes_per_col(int max_nl, size_t *stride_out = nullptr) {
 
 // Three-kernel pipeline (rt_fp64.cu; MIXED swaps in rt_mixed.cu's solver)
 // over chunks of the columns in the slot's segment table.
+// check: the stage validates the inputs as it reads them.
 int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int max_nl, int &nk,
-                    int max_chunk) {
+                    int max_chunk, bool check) {
     auto al = [](size_t b) { return (b + 255) / 256 * 256; };
     size_t stride = 0;
     const size_t per_col = pipe_bytes_per_col(max_nl, &stride);
@@ -640,7 +634,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, mixed ? rt_fp64_screen<true> : rt_fp64_screen<false>,
                                                       SCREEN_THREADS, 0);
         int e = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, rt_stage, STAGE_THREADS, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, rt_stage<true>, STAGE_THREADS, 0);
         sl.occ_stage = std::max(e, 1);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rt_fp64_solve<false>, 128, 0);
         int qo = 1;
@@ -658,8 +652,8 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         const int c1 = std::min(total, c0 + chunk);
         CK(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned int), st));
         const int g0 = std::min((c1 - c0 + 3) / 4, h->num_sms * sl.occ_stage);   // 4 columns per CTA
-        rt_stage<<<g0, STAGE_THREADS, 0, st>>>(sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_planck, h->K,
-                                               sl.d_status);
+        (check ? rt_stage<true> : rt_stage<false>)<<<g0, STAGE_THREADS, 0, st>>>(
+            sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_planck, h->K, sl.d_status);
         const long long items = (long long)(c1 - c0) * SCREEN_GROUPS;
         const int warps = SCREEN_THREADS / 32;
         const int g1 = (int)std::min<long long>((items + warps - 1) / warps, (long long)h->num_sms * sl.occ_screen);
@@ -780,22 +774,24 @@ int launch_fused(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int ncols, int ma
 
 // The radiation kernels of a call: the persistent fused kernel or the
 // multi-kernel pipeline, per the handle's form.
-int launch_body(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int max_nl, int &nk, int max_chunk) {
+int launch_body(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int max_nl, int &nk, int max_chunk,
+                bool check = false) {
     return h->fused ? launch_fused(h, sl, st, total, max_nl, nk)
-                    : launch_pipeline(h, sl, st, total, max_nl, nk, max_chunk);
+                    : launch_pipeline(h, sl, st, total, max_nl, nk, max_chunk, check);
 }
 
-// Status words cleared, optional validation, kernels between ev0 and ev1.
+// Status words cleared, optional validation (the pipeline's stage checks the
+// inputs it reads; the fused form has a kernel for it), kernels between ev0
+// and ev1.
 int launch_all(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int max_nl, int max_chunk) {
     CK(cudaMemsetAsync(sl.d_status, 0, 256, st));
     int nk = 0;
-    if (h->cfg.validate) {
-        const int vb = std::min((total + 255) / 256, h->num_sms * 8);
-        validate_kernel<<<std::max(vb, 1), 256, 0, st>>>(sl.d_segs, sl.d_status);
+    if (h->cfg.validate && h->fused) {
+        launch_validate(h, sl.d_segs, sl.d_status, total, st);
         ++nk;
     }
     CK(cudaEventRecord(sl.ev0, st));
-    const int rc = launch_body(h, sl, st, total, max_nl, nk, max_chunk);
+    const int rc = launch_body(h, sl, st, total, max_nl, nk, max_chunk, h->cfg.validate != 0);
     if (rc) return rc;
     CK(cudaEventRecord(sl.ev1, st));
     sl.kernels = nk;
@@ -1861,7 +1857,7 @@ int mgcm_rt_debug_bins(mgcm_rt_handle *h, const mgcm_rt_batch_in *in, int *mt, i
                             cudaMemcpyHostToDevice, st) ||
             cudaMemsetAsync(sl.d_status, 0, 256, st)) { rc = MGCM_RT_ECUDA; break; }
         const int g0 = std::min<int>(((int)z.ncol + 3) / 4, h->num_sms * 4);
-        rt_stage<<<g0, STAGE_THREADS, 0, st>>>(sl.d_segs, 0, (int)z.ncol, z.nl, blocks, stride, h->d_planck,
+        rt_stage<false><<<g0, STAGE_THREADS, 0, st>>>(sl.d_segs, 0, (int)z.ncol, z.nl, blocks, stride, h->d_planck,
                                                h->K, sl.d_status);
         const long long items = (long long)z.ncol * z.lev;
         const int g1 = (int)std::min<long long>((items + 255) / 256, (long long)h->num_sms * 8);
@@ -2331,10 +2327,8 @@ extern "C" int mgcm_rt_run_noalloc(mgcm_rt_handle *h, const mgcm_rt_batch_in *in
                        cudaMemcpyHostToDevice, stream));
     CK(cudaMemsetAsync(d_status, 0, sizeof(uint32_t), stream));
     CK(cudaMemsetAsync(d_nsys, 0, sizeof(unsigned long long), stream));
-    if (h->cfg.validate) {   // the same input checks as the other entry points
-        const int vb = std::min((int)((z.ncol + 255) / 256), h->num_sms * 8);
-        validate_kernel<<<std::max(vb, 1), 256, 0, stream>>>(d_tab, d_status);
-    }
+    if (h->cfg.validate)   // the same input checks as the other entry points
+        launch_validate(h, d_tab, d_status, (int)z.ncol, stream);
     CK(cudaEventRecord(sl.ev0, stream));
     rt_fp64_kernel<<<grid, BLOCK, smem, stream>>>(d_tab, h->d_kv, h->d_ki, h->d_planck, h->K,
                                                      max_nl, d_status, d_nsys, d_red);

