@@ -46,15 +46,18 @@ template <bool F32>
 __global__ void rt_fp64_screen(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                                unsigned char *__restrict__ blocks, size_t stride,
                                const double *__restrict__ kv, const double *__restrict__ ki,
-                               const RtConst K, int *__restrict__ list_v, int *__restrict__ list_i,
+                               const __grid_constant__ RtConst K, int *__restrict__ list_v, int *__restrict__ list_i,
                                unsigned int *counts, unsigned long long *nsys,
-                               const float *__restrict__ kvf);
-template <bool VIS>
-__global__ void rt_fp64_solve(const SegTable *__restrict__ st, int col_begin, int max_nl,
-                              unsigned char *__restrict__ blocks, size_t stride,
-                              const double *__restrict__ ktab, const RtConst K,
-                              const int *__restrict__ list, const unsigned int *count,
-                              double *__restrict__ fl, double *__restrict__ sc);
+                               const float *__restrict__ kvf, int groups);
+__global__ void rt_fp64_solve_vis(const SegTable *__restrict__ st, int col_begin, int max_nl,
+                                  unsigned char *__restrict__ blocks, size_t stride,
+                                  const double *__restrict__ ktab, const __grid_constant__ RtConst K,
+                                  const int *__restrict__ list, const unsigned int *count,
+                                  double *__restrict__ fl, double *__restrict__ sc);
+__global__ void rt_ir_dense(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
+                            unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ ktab,
+                            const __grid_constant__ RtConst K, double *__restrict__ fl, double *__restrict__ sc,
+                            unsigned long long *nsys);
 template <bool VIS, int R>
 __global__ void rt_quad_solve(const SegTable *__restrict__ st, int col_begin, int max_nl,
                               unsigned char *__restrict__ blocks, size_t stride,
@@ -69,7 +72,7 @@ __global__ void rt_quad_mixed_vis(const SegTable *__restrict__ st, int col_begin
 __global__ void rt_mixed_solve_vis(const SegTable *__restrict__ st, int col_begin, int max_nl,
                                    unsigned char *__restrict__ blocks, size_t stride,
                                    const float *__restrict__ ktabf, const double *__restrict__ ktab,
-                                   const RtConst K, const int *__restrict__ list,
+                                   const __grid_constant__ RtConst K, const int *__restrict__ list,
                                    const unsigned int *count, double *__restrict__ fl,
                                    double *__restrict__ sc);
 template <bool ONE_LEVEL, int RB>
@@ -77,7 +80,7 @@ __global__ void rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, i
                                int max_nl, unsigned char *__restrict__ blocks, size_t stride,
                                const RtConst K, const double *__restrict__ fl_v,
                                const double *__restrict__ sc_v, const double *__restrict__ fl_i,
-                               const double *__restrict__ sc_i);
+                               const double *__restrict__ sc_i, int dense_ir);
 size_t reduce_smem_bytes(int max_nl, int rb);
 const void *reduce_kernel(int max_nl, int rb);
 constexpr int REDUCE_WARPS = 4, REDUCE_THREADS = 32 * REDUCE_WARPS;   // rt_fp64_reduce: warp per column
@@ -581,7 +584,7 @@ int configure_kernels(int device) {
                                     (int)TM_SMEM_CAP));
     // the solvers use no shared memory: the whole unified L1 goes to the
     // per-system arrays
-    for (const void *f : {(const void *)rt_fp64_solve<true>, (const void *)rt_fp64_solve<false>,
+    for (const void *f : {(const void *)rt_fp64_solve_vis, (const void *)rt_ir_dense,
                           (const void *)rt_mixed_solve_vis})
         CK(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0));
     done[device] = true;
@@ -636,7 +639,8 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         int e = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, rt_stage<true>, STAGE_THREADS, 0);
         sl.occ_stage = std::max(e, 1);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rt_fp64_solve<false>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, mixed ? (const void *)rt_mixed_solve_vis : (const void *)rt_fp64_solve_vis,
+                                                      128, 0);
         int qo = 1;
         const int qr = quad_r_for(max_nl);
         if (qr == 7) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qo, rt_quad_solve<false, 7>, 128, 0);
@@ -654,24 +658,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         const int g0 = std::min((c1 - c0 + 3) / 4, h->num_sms * sl.occ_stage);   // 4 columns per CTA
         (check ? rt_stage<true> : rt_stage<false>)<<<g0, STAGE_THREADS, 0, st>>>(
             sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_planck, h->K, sl.d_status);
-        const long long items = (long long)(c1 - c0) * SCREEN_GROUPS;
-        const int warps = SCREEN_THREADS / 32;
-        const int g1 = (int)std::min<long long>((items + warps - 1) / warps, (long long)h->num_sms * sl.occ_screen);
-        if (mixed)
-            rt_fp64_screen<true><<<g1, SCREEN_THREADS, 0, st>>>(sl.d_segs, c0, c1, max_nl, blocks, stride,
-                                                                h->d_kv, h->d_ki, h->K, list_v, list_i,
-                                                                counts, sl.d_nsys, h->d_kvf);
-        else
-            rt_fp64_screen<false><<<g1, SCREEN_THREADS, 0, st>>>(sl.d_segs, c0, c1, max_nl, blocks, stride,
-                                                                 h->d_kv, h->d_ki, h->K, list_v, list_i,
-                                                                 counts, sl.d_nsys, nullptr);
         const int g2 = h->num_sms * (sl.tune.solve_ctas > 0 ? sl.tune.solve_ctas : sl.occ_solve);
-        // MIXED: FP32 visible opacities; the IR family is FP64 in both modes.
-        // The visible solve runs on the slot's second stream beside the IR
-        // solve, so each kernel's last wave overlaps the other's.
-        CK(cudaEventRecord(sl.fork_ev, st));
-        CK(cudaStreamWaitEvent(sl.aux, sl.fork_ev, 0));
-        cudaStream_t vst = sl.aux;
         const int qr = h->quad ? quad_r_for(max_nl) : 0;
         const bool oc = h->onchip || h->tmem;
         const int tv = oc ? oc_threads(true, max_nl) : 0, ti = oc ? oc_threads(false, max_nl) : 0;
@@ -680,6 +667,28 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         for (int q = 1; q < sl.h_segs->nseg; ++q) one_l = one_l && sl.h_segs->seg[q].L == sl.h_segs->seg[0].L;
         const int qv = h->tmem && one_l ? tm_choice(true, max_nl) : -1;
         const int qi = h->tmem && one_l ? tm_choice(false, max_nl) : -1;
+        // thread per system: the IR solve screens its own systems, beside the
+        // visible screen and solve on the slot's second stream; the other
+        // forms solve listed systems of both families after one screen
+        const int dense_ir = !((qv >= 0 && qi >= 0) || (tv > 0 && ti > 0) || qr);
+        const int groups = dense_ir ? SCREEN_GROUPS_V : SCREEN_GROUPS;
+        const long long items = (long long)(c1 - c0) * groups;
+        const int warps = SCREEN_THREADS / 32;
+        const int g1 = (int)std::min<long long>((items + warps - 1) / warps, (long long)h->num_sms * sl.occ_screen);
+        cudaStream_t vst = sl.aux;
+        auto fork = [&]() {
+            CK(cudaEventRecord(sl.fork_ev, st));
+            CK(cudaStreamWaitEvent(vst, sl.fork_ev, 0));
+            return MGCM_RT_OK;
+        };
+        if (dense_ir)
+            if (const int frc = fork()) return frc;
+        (mixed ? rt_fp64_screen<true> : rt_fp64_screen<false>)<<<g1, SCREEN_THREADS, 0, dense_ir ? vst : st>>>(
+            sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_kv, h->d_ki, h->K, list_v, list_i, counts, sl.d_nsys,
+            mixed ? h->d_kvf : nullptr, groups);
+        if (!dense_ir)
+            if (const int frc = fork()) return frc;
+        // MIXED: FP32 visible opacities; the IR family is FP64 in both modes.
         if (qv >= 0 && qi >= 0) {
             const int wv = TM_WARPS[qv], wi = TM_WARPS[qi];
             // at least 116 KB of shared memory each: no two CTAs that hold the
@@ -720,10 +729,11 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
                 rt_mixed_solve_vis<<<g2, 128, 0, vst>>>(sl.d_segs, c0, max_nl, blocks, stride, h->d_kvf, h->d_kv,
                                                         h->K, list_v, counts, fl_v, sc_v);
             else
-                rt_fp64_solve<true><<<g2, 128, 0, vst>>>(sl.d_segs, c0, max_nl, blocks, stride, h->d_kv, h->K,
-                                                         list_v, counts, fl_v, sc_v);
-            rt_fp64_solve<false><<<g2, 128, 0, st>>>(sl.d_segs, c0, max_nl, blocks, stride, h->d_ki, h->K,
-                                                     list_i, counts, fl_i, sc_i);
+                rt_fp64_solve_vis<<<g2, 128, 0, vst>>>(sl.d_segs, c0, max_nl, blocks, stride, h->d_kv, h->K,
+                                                       list_v, counts, fl_v, sc_v);
+            const int gi = ((c1 - c0) * NSYS_I + 127) / 128;
+            rt_ir_dense<<<sl.tune.solve_ctas > 0 ? std::min(gi, g2) : gi, 128, 0, st>>>(
+                sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_ki, h->K, fl_i, sc_i, sl.d_nsys);
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(sl.join_ev, sl.aux));
@@ -734,7 +744,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
             const RtConst &K = h->K;
             void *args[] = {(void *)&segs, (void *)&c0, (void *)&c1, (void *)&max_nl, (void *)&blocks,
                             (void *)&stride, (void *)&K, (void *)&fl_v, (void *)&sc_v, (void *)&fl_i,
-                            (void *)&sc_i};
+                            (void *)&sc_i, (void *)&dense_ir};
             CK(cudaLaunchKernel(reduce_kernel(max_nl, rb), dim3(g3), dim3(REDUCE_THREADS), args, rsm, st));
         }
         nk += 5;
@@ -1602,8 +1612,8 @@ mgcm_rt_handle *mgcm_rt_create(const mgcm_rt_config *cfg, const char *data_dir, 
         // allocating is allowed, through the per-thread stack limit, so that
         // no later call -- mgcm_rt_run_noalloc in particular -- allocates.
         size_t need = 0, cur = 0;
-        for (const void *f : {(const void *)rt_fp64_kernel, (const void *)rt_fp64_solve<true>,
-                              (const void *)rt_fp64_solve<false>, (const void *)rt_mixed_solve_vis,
+        for (const void *f : {(const void *)rt_fp64_kernel, (const void *)rt_fp64_solve_vis,
+                              (const void *)rt_ir_dense, (const void *)rt_mixed_solve_vis,
                               (const void *)rt_fp64_screen<false>, (const void *)rt_fp64_screen<true>}) {
             cudaFuncAttributes fa{};
             if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) { *status = MGCM_RT_ECUDA; return nullptr; }

@@ -30,6 +30,17 @@ struct alignas(16) KLevel {
 };
 static_assert(sizeof(KLevel) == 64, "KLevel is one 64-byte record");
 
+// What the IR systems of a band read per layer: COSBI, the numerator of
+// WBARI, Planck B0 and the numerator of B1 (B1*DTAU), two 16-byte loads.
+struct alignas(16) IrLayer {
+    double cosb, wnum, b0, pdif;
+};
+
+// What the visible systems of a band read per layer in pass A.
+struct alignas(16) VisLayer {
+    double cosb, wnum;
+};
+
 // Shared-memory layout of one column; sized by the launch's largest NL.
 struct ColSmem {
     // per level (1-based k = 1..LEV+1)
@@ -38,18 +49,19 @@ struct ColSmem {
     double *tref_v, *tref_i, *tref_c;   // TAUREF/QEXTREF (vis, IR), TAUREFCLD/QEXTREFCLD
     // per level and band
     double *trayaer;                    // [k][7] visible TRAY+TAEROS+TCLOUD
-    double *taer_i, *tcld_i;            // [k][5] IR TAEROS, TCLOUD
+    double2 *ext_i;                     // [k][5] IR TAEROS, TCLOUD
     // per layer and band
-    double *cosb_v, *wnum_v;            // [l][7]
+    VisLayer *lay_v;                    // [l][7]
     double *cbs_v;                      // [l][7] COSBV/(1+COSBV), the delta-Eddington COSBAR
-    double *cosb_i, *wnum_i;            // [l][5]
-    double *b0_i, *pdif_i;              // [l][5] Planck B0 and B1*DTAU numerator
+    IrLayer *lay_i;                     // [l][5]
     double *bsurf_i, *pltop_i;          // [5]
     // reduction staging
     double *fmp, *fmm;                  // [sys][l]
     double *sc0, *sc1, *sc2;            // [sys] FLUXUP, FLUXDN, DIFFV (vis) / FTOPUP (IR)
     unsigned char *skip;                // [sys] 0 = solved, 1 = TLIMIT skip, 2 = no work
     int *meta;                          // [2*SCREEN_GROUPS] list base/count of kept systems per group
+    int *odd;                           // bands (bit nw-1 visible, 7+nw-1 IR) with a layer outside the
+                                        // range of the solves' fast arithmetic (rt_solve.cuh)
     double *fmnet_v, *fmnet_i;          // [l] reduced net fluxes for the divergences
     double *misc;                       // [4] NFLUXTOPV, NFLUXTOPI
     int day;
@@ -74,7 +86,7 @@ __host__ __device__ inline size_t col_smem_bytes(int nl, bool red_in_smem = true
     if (red_in_smem) b += red_bytes(nl);
     b += 3 * NSYS * sizeof(double);
     b += 2 * (nl + 1) * sizeof(double) + 4 * sizeof(double);
-    b += NSYS + 16 + 2 * SCREEN_GROUPS * sizeof(int) + 16;
+    b += NSYS + 16 + (2 * SCREEN_GROUPS + 1) * sizeof(int) + 16;
     return b;
 }
 
@@ -83,22 +95,21 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
     ColSmem s;
     const int lev1 = 2 * nl + 3;
     s.klev = reinterpret_cast<KLevel *>(base);   // base is 16-byte aligned
-    double *d = reinterpret_cast<double *>(base + (size_t)(lev1 + 1) * sizeof(KLevel));
+    // records first: 16-byte aligned
+    unsigned char *q = base + (size_t)(lev1 + 1) * sizeof(KLevel);
+    s.ext_i = reinterpret_cast<double2 *>(q);
+    q += (size_t)(lev1 + 1) * D_NI * sizeof(double2);
+    s.lay_i = reinterpret_cast<IrLayer *>(q);
+    q += (size_t)(nl + 1) * D_NI * sizeof(IrLayer);
+    s.lay_v = reinterpret_cast<VisLayer *>(q);
+    double *d = reinterpret_cast<double *>(q + (size_t)(nl + 1) * D_NV * sizeof(VisLayer));
     auto take = [&](size_t n) { double *p = d; d += n; return p; };
     s.dpr = take(lev1 + 1);
     s.tref_v = take(lev1 + 1);
     s.tref_i = take(lev1 + 1);
     s.tref_c = take(lev1 + 1);
     s.trayaer = take((lev1 + 1) * D_NV);
-    s.taer_i = take((lev1 + 1) * D_NI);
-    s.tcld_i = take((lev1 + 1) * D_NI);
-    s.cosb_v = take((nl + 1) * D_NV);
-    s.wnum_v = take((nl + 1) * D_NV);
     s.cbs_v = take((nl + 1) * D_NV);
-    s.cosb_i = take((nl + 1) * D_NI);
-    s.wnum_i = take((nl + 1) * D_NI);
-    s.b0_i = take((nl + 1) * D_NI);
-    s.pdif_i = take((nl + 1) * D_NI);
     s.bsurf_i = take(D_NI);
     s.pltop_i = take(D_NI);
     if (!with_red) {
@@ -119,6 +130,7 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
     int *ip = reinterpret_cast<int *>(d);
     s.skip = reinterpret_cast<unsigned char *>(ip);
     s.meta = reinterpret_cast<int *>(((reinterpret_cast<uintptr_t>(s.skip + NSYS) + 15) / 16) * 16);
+    s.odd = s.meta + 2 * SCREEN_GROUPS;
     s.day = 0;
     return s;
 }

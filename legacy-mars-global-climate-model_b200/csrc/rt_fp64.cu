@@ -28,6 +28,7 @@
 // the CPU oracle uses too, so host and device agree bit-for-bit.
 #include "rt_fp64_sys.cuh"
 #include "rt_quad.cuh"
+#include "rt_solve.cuh"
 #include "../../include/mgcm_rt_math.h"
 
 namespace mgcm {
@@ -127,39 +128,38 @@ template __global__ void rt_stage<true>(STAGE_ARGS);
 
 // K1: screen every system (optics sums, TLIMIT test, DETAU, CUMTAUV) and
 // append the kept ones to the family lists.  F32 (mixed precision): visible
-// gas opacities from the FP32 table; the IR family always screens in FP64.  One warp per (column, group);
-// warps never wait on one another.  A group's kept systems take one
+// gas opacities from the FP32 table; the IR family always screens in FP64.
+// One warp per (column, group); warps never wait on one another.  `groups` is
+// SCREEN_GROUPS_V when the solve screens the IR systems itself (rt_ir_dense).  A group's kept systems take one
 // contiguous run of list positions in ascending order; its base and count go
 // to the column's meta words.
 template <bool F32>
 __global__ void __launch_bounds__(128, 8)   // 64 registers: 8 CTAs/SM (measured 6% faster than 80)
 rt_fp64_screen(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ kv,
-               const double *__restrict__ ki, const RtConst K, int *__restrict__ list_v,
+               const double *__restrict__ ki, const __grid_constant__ RtConst K, int *__restrict__ list_v,
                int *__restrict__ list_i, unsigned int *counts, unsigned long long *nsys,
-               const float *__restrict__ kvf) {
-    SysLocal w;
+               const float *__restrict__ kvf, int groups) {
+    SolveLocal w;
     unsigned int nsolved = 0;
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const long long items = (long long)(col_end - col_begin) * SCREEN_GROUPS;
-    for (long long it = (long long)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); it < items; it += nwarps) {
-        const int g = col_begin + (int)(it / SCREEN_GROUPS), grp = (int)(it % SCREEN_GROUPS);
+    const int items = (col_end - col_begin) * groups;
+    for (int it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += nwarps) {
+        const int g = col_begin + it / groups, grp = it % groups;
         const SegDev &sg = st->seg[find_seg(st, g)];
         const int c = g - sg.col0;
-        ColSmem s = carve_smem(blocks + (size_t)(g - col_begin) * stride, max_nl, nullptr, false);
+        unsigned char *block = blocks + (size_t)(g - col_begin) * stride;
+        ColSmem s = carve_smem(block, max_nl, nullptr, false);
         const bool vis = grp < SCREEN_GROUPS_V;
         const int t = group_first(grp) + lane;
         bool act = false;
         if (vis) {
-            if (t < group_end(grp) && sg.acosz[c] >= R4(1.0e-5)) {
-                solve_vis<1, F32>(sg, c, t / D_NG + 1, t % D_NG + 1, t, s, K, kv, w, nsolved, nullptr,
-                                  nullptr, nullptr, nullptr, nullptr, kvf);
-                act = s.skip[t] == 0;
-            }
+            if (t < group_end(grp) && sg.acosz[c] >= R4(1.0e-5))
+                act = fast_vis_screen<F32>(sg, c, t, block, max_nl, s, K, kv, kvf, w, nsolved);
         } else if (t < group_end(grp)) {
             const int j = t - NSYS_V;
-            solve_ir<1>(sg, c, j / D_NG + 1, j % D_NG + 1, t, s, K, ki, w, nsolved, nullptr, nullptr,
+            solve_ir<1>(sg, c, j / D_NG + 1, j % D_NG + 1, t, s, K, ki, w.g, nsolved, nullptr, nullptr,
                         nullptr);
             act = s.skip[t] == 0;
         }
@@ -183,50 +183,57 @@ rt_fp64_screen(const SegTable *__restrict__ st, int col_begin, int col_end, int 
 
 #define SCREEN_ARGS                                                                                    \
     const SegTable *__restrict__, int, int, int, unsigned char *__restrict__, size_t,                \
-        const double *__restrict__, const double *__restrict__, const RtConst, int *__restrict__,    \
-        int *__restrict__, unsigned int *, unsigned long long *, const float *__restrict__
+        const double *__restrict__, const double *__restrict__, const __grid_constant__ RtConst, int *__restrict__,    \
+        int *__restrict__, unsigned int *, unsigned long long *, const float *__restrict__, int
 template __global__ void rt_fp64_screen<false>(SCREEN_ARGS);
 template __global__ void rt_fp64_screen<true>(SCREEN_ARGS);
 #undef SCREEN_ARGS
 
-// K2: solve the listed systems of one family, one thread per system.
-template <bool VIS>
-__global__ void __launch_bounds__(128, VIS ? MGCM_VIS_SOLVE_MINB : MGCM_IR_SOLVE_MINB)
-rt_fp64_solve(const SegTable *__restrict__ st, int col_begin, int max_nl,
-              unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ ktab,
-              const RtConst K, const int *__restrict__ list, const unsigned int *count,
-              double *__restrict__ fl, double *__restrict__ sc) {
-    SysLocal w;
-    unsigned int dummy = 0;
-    const unsigned int n = VIS ? count[0] : count[1];
+// K2: solve the listed visible systems, one thread per system.
+__global__ void __launch_bounds__(128, MGCM_VIS_SOLVE_MINB)
+rt_fp64_solve_vis(const SegTable *__restrict__ st, int col_begin, int max_nl,
+                  unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ ktab,
+                  const __grid_constant__ RtConst K, const int *__restrict__ list, const unsigned int *count,
+                  double *__restrict__ fl, double *__restrict__ sc) {
+    SolveLocal w;
+    const unsigned int n = count[0];
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = list[i];
-        const int g = e >> 8, sidx = e & 255;
-        const int si = find_seg(st, g);
-        const SegDev &sg = st->seg[si];
-        const int c = g - sg.col0;
-        ColSmem s = carve_smem(blocks + (size_t)(g - col_begin) * stride, max_nl, nullptr, false);
-        double *row = fl + row_base(i, max_nl), *scr = sc + sc_base(i);
-        double *rdn = row + (size_t)max_nl * ROW_BLK;   // downward fluxes
-        if (VIS) {
-            solve_vis<2>(sg, c, sidx / D_NG + 1, sidx % D_NG + 1, sidx, s, K, ktab, w, dummy, row,
-                         rdn, scr, scr + ROW_BLK, scr + 2 * ROW_BLK, nullptr, ROW_BLK);
-        } else {
-            const int j = sidx - NSYS_V;
-            solve_ir<2>(sg, c, j / D_NG + 1, j % D_NG + 1, sidx, s, K, ktab, w, dummy, row,
-                        rdn, scr, ROW_BLK);
-        }
+        const int g = e >> 8;
+        const SegDev &sg = st->seg[find_seg(st, g)];
+        double *row = fl + row_base(i, max_nl);
+        fast_vis<false>(sg, g - sg.col0, e & 255, blocks + (size_t)(g - col_begin) * stride, max_nl, K, ktab,
+                        nullptr, w, row, row + (size_t)max_nl * ROW_BLK, sc + sc_base(i));
     }
 }
 
-template __global__ void rt_fp64_solve<true>(const SegTable *__restrict__, int, int, unsigned char *__restrict__,
-                                             size_t, const double *__restrict__, const RtConst,
-                                             const int *__restrict__, const unsigned int *,
-                                             double *__restrict__, double *__restrict__);
-template __global__ void rt_fp64_solve<false>(const SegTable *__restrict__, int, int, unsigned char *__restrict__,
-                                              size_t, const double *__restrict__, const RtConst,
-                                              const int *__restrict__, const unsigned int *,
-                                              double *__restrict__, double *__restrict__);
+// K2: screen and solve the IR systems of a chunk, one thread per system, at
+// list position (column in the chunk) * 85 + system.  Nine tenths of them
+// pass TLIMIT, so a list of the kept ones would fill 8% more lanes but take
+// every gas optical depth twice, in a screen and here; the threads of a
+// screened system wait.  With the fast arithmetic (rt_solve.cuh) the call
+// of 64,800 x 24 columns takes 13.4 -> 11.45 ms (FP64), the screen of 8,192
+// columns 433 -> 365 us, both solves 1,185 -> 1,090 us.
+__global__ void __launch_bounds__(128, MGCM_IR_SOLVE_MINB)
+rt_ir_dense(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
+            unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ ktab,
+            const __grid_constant__ RtConst K, double *__restrict__ fl, double *__restrict__ sc,
+            unsigned long long *nsys) {
+    SolveLocal w;
+    unsigned int nsolved = 0;
+    const int n = (col_end - col_begin) * NSYS_I;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int cc = i / NSYS_I, j = i - cc * NSYS_I, g = col_begin + cc;
+        const SegDev &sg = st->seg[find_seg(st, g)];
+        double *row = fl + row_base(i, max_nl);
+        nsolved += fast_ir(sg, g - sg.col0, j, blocks + (size_t)cc * stride, max_nl, K, ktab, w, row,
+                           row + (size_t)max_nl * ROW_BLK, sc + sc_base(i)) == 0;
+    }
+    if (nsys) {
+        for (int o = 16; o > 0; o >>= 1) nsolved += __shfl_down_sync(0xffffffffu, nsolved, o);
+        if ((threadIdx.x & 31) == 0 && nsolved) atomicAdd(nsys, (unsigned long long)nsolved);
+    }
+}
 
 // K2 (four-lane form, L <= 51): a quad of lanes per kept system, 8 systems
 // per warp, per-layer values in registers (rt_quad.cuh).  A quad past the
@@ -358,7 +365,7 @@ __global__ void __launch_bounds__(32 * RED_WARPS)
 rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                unsigned char *__restrict__ blocks, size_t stride, const RtConst K,
                const double *__restrict__ fl_v, const double *__restrict__ sc_v,
-               const double *__restrict__ fl_i, const double *__restrict__ sc_i) {
+               const double *__restrict__ fl_i, const double *__restrict__ sc_i, int dense_ir) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int LPL = ONE_LEVEL ? 1 : RED_LPL;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -381,7 +388,15 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
             // list positions of the family's kept systems (none at night for
             // the visible family: its outputs are zeros)
             int nrow = 0;
-            if (!vis || day) {
+            if (!vis && dense_ir) {   // rt_ir_dense: every system has its position
+                for (int j0 = 0; j0 < NSYS_I; j0 += 32) {
+                    const int j = j0 + lane;
+                    const bool kept = j < NSYS_I && s.skip[NSYS_V + j] == 0;
+                    const unsigned m = __ballot_sync(0xffffffffu, kept);
+                    if (kept) rpos[nrow + __popc(m & ((1u << lane) - 1u))] = (g - col_begin) * NSYS_I + j;
+                    nrow += __popc(m);
+                }
+            } else if (!vis || day) {
                 const int w0 = vis ? 0 : SCREEN_GROUPS_V, w1 = vis ? SCREEN_GROUPS_V : SCREEN_GROUPS;
                 for (int gw = w0; gw < w1; ++gw) {
                     const int gb = s.meta[2 * gw], gn = s.meta[2 * gw + 1];
@@ -500,7 +515,7 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
 #define REDUCE_ARGS                                                                                    \
     const SegTable *__restrict__, int, int, int, unsigned char *__restrict__, size_t, const RtConst,  \
         const double *__restrict__, const double *__restrict__, const double *__restrict__,          \
-        const double *__restrict__
+        const double *__restrict__, int
 #define REDUCE_INST(RB)                                              \
     template __global__ void rt_fp64_reduce<true, RB>(REDUCE_ARGS);  \
     template __global__ void rt_fp64_reduce<false, RB>(REDUCE_ARGS);

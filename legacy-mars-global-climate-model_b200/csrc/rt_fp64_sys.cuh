@@ -36,9 +36,14 @@ struct Lay {   // per-layer two-stream coefficients
 // pass-A slots instead -- and both write the DSOLVER rows' AS/DS for the
 // back-substitution.
 struct SysLocal {
-    double a0[D_MAXNL + 1], a1[D_MAXNL + 1], a2[D_MAXNL + 1], a3[D_MAXNL + 2], a4[D_MAXNL + 1];
+    alignas(16) double a0[D_MAXNL + 1];
+    double a1[D_MAXNL + 1];
+    alignas(16) double a2[D_MAXNL + 1];
+    double a3[D_MAXNL + 2];
+    alignas(16) double a4[D_MAXNL + 1];
     double c5[D_MAXNL + 1];
-    double as[2 * D_MAXNL + 1], ds[2 * D_MAXNL + 1];
+    alignas(16) double as[2 * D_MAXNL + 1];
+    double ds[2 * D_MAXNL + 1];
 };
 
 // One step of the DTRIDGL upward elimination for row i given row i+1's AS/DS.
@@ -222,8 +227,8 @@ __device__ void solve_vis(const SegDev &sg, int c, int nw, int ng, int sidx, Col
             tcB = tcA;
             dt = da;
         }
-        const double wb = s.wnum_v[l * D_NV + nw - 1] / dt;
-        const double cb = s.cosb_v[l * D_NV + nw - 1];
+        const double wb = s.lay_v[l * D_NV + nw - 1].wnum / dt;
+        const double cb = s.lay_v[l * D_NV + nw - 1].cosb;
         const double f = 1.0 - wb * (cb * cb);
         if (l == 1) {
             tau = 0.0 * f;
@@ -399,7 +404,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
     const double *tb = ki + (size_t)(nw - 1) * D_NT * D_NP * D_NH * D_NGK + (ng - 1);
     double taugsurf = 0.0;
     auto dtauk = [&](int k) -> double {
-        const double ta = s.taer_i[k * D_NI + nw - 1], tcl = s.tcld_i[k * D_NI + nw - 1];
+        const double ta = s.ext_i[k * D_NI + nw - 1].x, tcl = s.ext_i[k * D_NI + nw - 1].y;
         if (ng < D_NG) {
             const double tg = taugas_at(s, k, tb);
             taugsurf += tg;
@@ -450,7 +455,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
         }
         double wb;
         if (dt > tiny) {
-            wb = s.wnum_i[l * D_NI + nw - 1] / dt;
+            wb = s.lay_i[l * D_NI + nw - 1].wnum / dt;
         } else {
             wb = 0.0;
             dt = tiny;
@@ -483,10 +488,10 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
     // 15.8 -> 15.4 ms).  The visible solve keeps its stored coefficients:
     // there the recomputation measured slower.
     auto lay4 = [&](int l, double w0, double dt, double &lam, double &gama, double &b1, double &term) {
-        const double cb = s.cosb_i[l * D_NI + nw - 1];
+        const double cb = s.lay_i[l * D_NI + nw - 1].cosb;
         const double alpha = sqrt((1.0 - w0) / (1.0 - w0 * cb));
         lam = alpha * (1.0 - w0 * cb) / UBARI;
-        b1 = s.pdif_i[l * D_NI + nw - 1] / dt;
+        b1 = s.lay_i[l * D_NI + nw - 1].pdif / dt;
         gama = (1.0 - alpha) / (1.0 + alpha);
         term = UBARI / (1.0 - w0 * cb);
     };
@@ -494,7 +499,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
         Lay y;
         double lam, b1, term;
         lay4(l, w0, dt, lam, y.gama, b1, term);
-        const double b0 = s.b0_i[l * D_NI + nw - 1];
+        const double b0 = s.lay_i[l * D_NI + nw - 1].b0;
         y.cp = b0 + b1 * dt + b1 * term;
         y.cm = b0 + b1 * dt - b1 * term;
         y.cpm1 = b0 + b1 * term;
@@ -546,7 +551,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
         xprev = xb;
         double xk1, xk2;
         unmix(xa, xb, xk1, xk2);
-        const double b0 = s.b0_i[n * D_NI + nw - 1];
+        const double b0 = s.lay_i[n * D_NI + nw - 1].b0;
         const double ep = mgcm_rt_exp(dmin(lam * dtk, TAUMAX));
         const double em = 1.0 / ep;
         const double cpmid = b0 + b1 * dtk + b1 * term;

@@ -18,28 +18,24 @@
 // under the same rounding moves heating by 4e-6 K/sol.  FP32 two-stream
 // coefficients put ~0.2 K/sol of rounding noise into the thin top layers.
 #include "rt_quad.cuh"
+#include "rt_solve.cuh"
 
 namespace mgcm {
 
 __global__ void __launch_bounds__(128, MGCM_VIS_SOLVE_MINB)   // 72 registers, as the FP64 visible solve
 rt_mixed_solve_vis(const SegTable *__restrict__ st, int col_begin, int max_nl,
                unsigned char *__restrict__ blocks, size_t stride, const float *__restrict__ ktabf,
-               const double *__restrict__ ktab, const RtConst K, const int *__restrict__ list,
+               const double *__restrict__ ktab, const __grid_constant__ RtConst K, const int *__restrict__ list,
                const unsigned int *count, double *__restrict__ fl, double *__restrict__ sc) {
     const unsigned int n = count[0];
-    fp64::SysLocal w;
-    unsigned int dummy = 0;
+    fp64::SolveLocal w;
     for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = list[i];
-        const int g = e >> 8, sidx = e & 255;
+        const int g = e >> 8;
         const SegDev &sg = st->seg[find_seg(st, g)];
-        const int c = g - sg.col0;
-        ColSmem s = carve_smem(blocks + (size_t)(g - col_begin) * stride, max_nl, nullptr, false);
-        double *row = fl + row_base(i, max_nl), *scr = sc + sc_base(i);
-        double *rdn = row + (size_t)max_nl * ROW_BLK;   // downward fluxes
-        fp64::solve_vis<2, true>(sg, c, sidx / D_NG + 1, sidx % D_NG + 1, sidx, s, K, ktab, w,
-                                 dummy, row, rdn, scr, scr + ROW_BLK, scr + 2 * ROW_BLK, ktabf,
-                                 ROW_BLK);
+        double *row = fl + row_base(i, max_nl);
+        fp64::fast_vis<true>(sg, g - sg.col0, e & 255, blocks + (size_t)(g - col_begin) * stride, max_nl, K, ktab,
+                             ktabf, w, row, row + (size_t)max_nl * ROW_BLK, sc + sc_base(i));
     }
 }
 

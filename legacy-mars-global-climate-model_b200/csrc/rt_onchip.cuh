@@ -71,7 +71,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
     const int oW = 0, oDT = NL, oTK = 2 * NL, oAS = 3 * NL, oDS = 5 * NL;   // AS(r) at oAS + r-1
     const double *tb = ki + (size_t)(nw - 1) * D_NT * D_NP * D_NH * D_NGK + (ng - 1);
     auto dtauk = [&](int k) -> double {
-        const double ta = s.taer_i[k * D_NI + nw - 1], tcl = s.tcld_i[k * D_NI + nw - 1];
+        const double ta = s.ext_i[k * D_NI + nw - 1].x, tcl = s.ext_i[k * D_NI + nw - 1].y;
         if (ng < D_NG) return taugas_at(s, k, tb) + ta + tcl;
         return ta + tcl;
     };
@@ -93,7 +93,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
         }
         double wb;
         if (dt > tiny) {
-            wb = s.wnum_i[l * D_NI + nw - 1] / dt;
+            wb = s.lay_i[l * D_NI + nw - 1].wnum / dt;
         } else {
             wb = 0.0;
             dt = tiny;
@@ -110,10 +110,10 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
     const double btop = (1.0 - mgcm_rt_exp(-tautop / UBARI)) * s.pltop_i[nw - 1];
     const double bsurf = s.bsurf_i[nw - 1];
     auto lay4 = [&](int l, double w0, double dt, double &lam, double &gama, double &b1, double &term) {
-        const double cb = s.cosb_i[l * D_NI + nw - 1];
+        const double cb = s.lay_i[l * D_NI + nw - 1].cosb;
         const double alpha = sqrt((1.0 - w0) / (1.0 - w0 * cb));
         lam = alpha * (1.0 - w0 * cb) / UBARI;
-        b1 = s.pdif_i[l * D_NI + nw - 1] / dt;
+        b1 = s.lay_i[l * D_NI + nw - 1].pdif / dt;
         gama = (1.0 - alpha) / (1.0 + alpha);
         term = UBARI / (1.0 - w0 * cb);
     };
@@ -121,7 +121,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
         Lay y;
         double lam, b1, term;
         lay4(l, w0, dt, lam, y.gama, b1, term);
-        const double b0 = s.b0_i[l * D_NI + nw - 1];
+        const double b0 = s.lay_i[l * D_NI + nw - 1].b0;
         y.cp = b0 + b1 * dt + b1 * term;
         y.cm = b0 + b1 * dt - b1 * term;
         y.cpm1 = b0 + b1 * term;
@@ -186,7 +186,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
         xprev = xb;
         double xk1, xk2;
         unmix(xa, xb, xk1, xk2);
-        const double b0 = s.b0_i[n * D_NI + nw - 1];
+        const double b0 = s.lay_i[n * D_NI + nw - 1].b0;
         const double ep = mgcm_rt_exp(dmin(lam * dtk, TAUMAX));
         const double em = 1.0 / ep;
         const double cpmid = b0 + b1 * dtk + b1 * term;
@@ -238,8 +238,8 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
             tcB = tcA;
             dt = da;
         }
-        const double wb = s.wnum_v[l * D_NV + nw - 1] / dt;
-        const double cb = s.cosb_v[l * D_NV + nw - 1];
+        const double wb = s.lay_v[l * D_NV + nw - 1].wnum / dt;
+        const double cb = s.lay_v[l * D_NV + nw - 1].cosb;
         const double f = 1.0 - wb * (cb * cb);
         if (l == 1) {
             tau = 0.0 * f;

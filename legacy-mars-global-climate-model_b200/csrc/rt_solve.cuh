@@ -1,0 +1,441 @@
+// Thread-per-system solves of the pipeline in the arithmetic of
+// rt_fastmath.cuh: the passes of rt_fp64_sys.cuh (solve_vis, solve_ir),
+// operation for operation, for systems whose operands stay in range.  A
+// system that leaves it anywhere (`odd`) is redone by the general solve.
+//
+// Range: the stage marks bands with |COSBAR| >= 1 or an unusual scattering
+// numerator (usual_layer); pass A checks that the layer's optical depth is
+// below 2^100 and its albedo in [0, 1), pass C every eliminated denominator
+// (and, visible, the root and the divisor of GAMA).  What else is divided by
+// or rooted then lies in range: 1 - W0 COSB >= 2^-53, and ALPHA within 2^27
+// of 1, EP in [1, exp(35)].
+#pragma once
+#include "rt_fp64_sys.cuh"
+
+namespace mgcm {
+namespace fp64 {
+
+// Per-layer values of a system in local memory, two to a 16-byte access.
+struct SolveLocal {
+    SysLocal g;   // the general solve's arrays; the fast ones lie over them
+    __device__ __forceinline__ double2 *pair() { return reinterpret_cast<double2 *>(g.a0); }        // layer l: W0, DTAU
+    __device__ __forceinline__ double2 *depth() { return reinterpret_cast<double2 *>(g.a2); }       // visible: TAU, mid TAU
+    __device__ __forceinline__ double *mid() { return g.a2; }                                       // IR: TAUCUM step
+    __device__ __forceinline__ double2 *src() { return reinterpret_cast<double2 *>(g.a4); }         // visible: AM, AP
+    __device__ __forceinline__ double2 *row() { return reinterpret_cast<double2 *>(g.as); }         // row i: AS, DS
+};
+
+// The general solves, out of line: systems out of range only.  They carve the
+// column block themselves, so that the callers' ColSmem stays in registers.
+static __device__ __noinline__ void general_ir(const SegDev &sg, int c, int j, unsigned char *block, int max_nl,
+                                        const RtConst &K, const double *__restrict__ ki, SysLocal &w, double *row,
+                                        double *rdn, double *scr) {
+    unsigned int dummy = 0;
+    ColSmem s = carve_smem(block, max_nl, nullptr, false);
+    solve_ir<2>(sg, c, j / D_NG + 1, j % D_NG + 1, NSYS_V + j, s, K, ki, w, dummy, row, rdn, scr, ROW_BLK);
+}
+
+template <int MODE, bool F32>
+static __device__ __noinline__ unsigned int general_vis(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
+                                                 const RtConst &K, const double *__restrict__ kv,
+                                                 const float *__restrict__ kvf, SysLocal &w, double *row,
+                                                 double *rdn, double *scr) {
+    unsigned int nsolved = 0;
+    ColSmem s = carve_smem(block, max_nl, nullptr, false);
+    solve_vis<MODE, F32>(sg, c, t / D_NG + 1, t % D_NG + 1, t, s, K, kv, w, nsolved, row, rdn, scr, scr + ROW_BLK,
+                         scr + 2 * ROW_BLK, kvf, ROW_BLK);
+    return nsolved;
+}
+
+// x / u0 capped at MAXEXP, y = 1 / u0 (GFLUXV's beam exponents).
+__device__ __forceinline__ double beam(double x, double u0, double y) {
+    return exp_r(-dmin(quot(x, u0, y), MAXEXP));
+}
+
+// Lay's exponential terms from GAMA and LAMDA*DTAU (gfluxi.f90:113-123, gfluxv.f90:150-163).
+__device__ __forceinline__ void exp_terms(Lay &y, double x) {
+    const double ep = exp_r(dmin(x, TAUMAX)), em = rcp_n(ep);
+    const double a = y.gama * em, b = y.gama * ep;
+    y.e1 = ep + a;
+    y.e2 = ep - a;
+    y.e3 = b + em;
+    y.e4 = b - em;
+}
+
+// rows_of_pair with the fast reciprocal; odd collects the range tests.
+__device__ __forceinline__ void fast_rows(const Lay &lo, const Lay &hi, double &as, double &ds, double &as_odd,
+                                          double &ds_odd, bool &odd) {
+    const double hp = hi.gama - 1.0, c13 = (lo.e1 + lo.e3) * hp;
+    const double dp = hi.cpm1 - lo.cp, dm = lo.cm - hi.cmm1;
+    {
+        const double af = 2.0 * (1.0 - lo.gama * lo.gama);
+        const double den = (lo.e1 - lo.e3) * (1.0 + hi.gama) - c13 * as;
+        const double df = lo.e3 * dp + lo.e1 * dm;
+        odd |= out_of_range(den);
+        const double x = rcp_s(den);
+        ds = (df - c13 * ds) * x;
+        as = af * x;
+        as_odd = as;
+        ds_odd = ds;
+    }
+    {
+        const double cf = 2.0 * (1.0 - hi.gama * hi.gama);
+        const double den = (lo.e2 + lo.e4) * hp - cf * as;
+        const double df = hp * dp + (1.0 - hi.gama) * dm;
+        odd |= out_of_range(den);
+        const double x = rcp_s(den);
+        ds = (df - cf * ds) * x;
+        as = c13 * x;
+    }
+}
+
+// ---------------------------------------------------------------- infrared
+// System j of column c: pass A with the TLIMIT decision (code/sfluxi.f90:72-75),
+// then the solve.  Returns 0 solved, 1 skipped (TLIMIT), 2 no work, and
+// writes the column's skip entry.
+__device__ __forceinline__ int fast_ir(const SegDev &sg, int c, int j, unsigned char *block, int max_nl,
+                                       const RtConst &K, const double *__restrict__ ki, SolveLocal &w, double *fmp,
+                                       double *fmm, double *sc0) {
+    const ColSmem s = carve_smem(block, max_nl, nullptr, false);
+    const int L = sg.L, NL = L + 1, LEV = 2 * L + 3;
+    const int nb = j / D_NG, ng = j - nb * D_NG;   // 0-based band and Gauss point
+    if (ng < D_NG - 1 && K.fzeroi[nb] >= R4(0.99)) return s.skip[NSYS_V + j] = 2;
+    const bool gas = ng < D_NG - 1;
+    const double *tb = ki + (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
+    const double2 *ext = s.ext_i + nb;
+    const IrLayer *lay = s.lay_i + nb;
+    double taug = 0.0;
+    auto dtauk = [&](int k) -> double {
+        const double2 e = ext[k * D_NI];
+        if (gas) {
+            const double tg = taugas_at(s, k, tb);
+            taug += tg;
+            return tg + e.x + e.y;
+        }
+        return e.x + e.y;
+    };
+    // pass A: pair = (WBARI, DTAUI), mid = TAUCUMI(2l+1) - TAUCUMI(2l)
+    double2 *pair = w.pair(), *row = w.row();
+    double *mid = w.mid();
+    const double tiny = R4(1.0E-9);
+    bool odd = (*s.odd >> (D_NV + nb)) & 1;
+    double tc = 0.0 + dtauk(2);
+    for (int l = 1; l <= NL; ++l) {
+        const int k = 2 * l + 1;
+        const double da = dtauk(k);
+        const double tcA = tc + da;
+        double dt = da, tcB = tcA;
+        if (k + 1 <= LEV) {
+            const double db = dtauk(k + 1);
+            tcB = tcA + db;
+            dt = da + db;
+        }
+        // the reference adds 1.D-50 to DTAUI: without effect above its TINY of 1e-9
+        const bool thick = dt > tiny;
+        dt = thick ? dt : tiny;
+        const double wb = thick ? quot(lay[l * D_NI].wnum, dt, rcp_n(dt)) : 0.0;
+        odd |= hi32(dt) >= 0x46300000u || hi32(wb) >= 0x3ff00000u;   // DTAUI < 2^100, 0 <= WBARI < 1
+        pair[l] = make_double2(wb, dt);
+        mid[l] = l < NL ? tcA - tc : dt;
+        tc = tcB;
+    }
+    if (gas && taug < TLIMITI) return s.skip[NSYS_V + j] = 1;
+    s.skip[NSYS_V + j] = 0;
+    if (!odd) {
+        const double *plev = sg.plev + (size_t)c * LEV;
+        const double rsf = sg.albi[c];
+        const double tautop = pair[1].y * plev[2 - 1] / (plev[4 - 1] - plev[2 - 1]);
+        const double btop = (1.0 - mgcm_rt_exp(-tautop / UBARI)) * s.pltop_i[nb];
+        // LAMDA, GAMA, TERM of a layer (code/gfluxi.f90:69-93), UBARI = 0.5.
+        // Passes C and D both evaluate them, B1 too: cheaper than a round
+        // trip of four more values per layer through local memory.
+        auto lay3 = [&](const IrLayer &r, double w0, double &lam, double &gama, double &term) {
+            const double d = 1.0 - w0 * r.cosb, y = rcp_n(d);
+            const double alpha = sqrt_n(quot(1.0 - w0, d, y));
+            const double ap1 = 1.0 + alpha;
+            lam = alpha * d * 2.0;
+            gama = quot(1.0 - alpha, ap1, rcp_n(ap1));
+            term = 0.5 * y;
+        };
+        // pass C
+        auto coef = [&](const IrLayer &r, double2 p) {
+            Lay y;
+            double lam, term;
+            lay3(r, p.x, lam, y.gama, term);
+            const double b1 = quot(r.pdif, p.y, rcp_n(p.y));
+            const double bt = b1 * term, bb = r.b0 + b1 * p.y;
+            y.cp = bb + bt;
+            y.cm = bb - bt;
+            y.cpm1 = r.b0 + bt;
+            y.cmm1 = r.b0 - bt;
+            exp_terms(y, lam * p.y);
+            return y;
+        };
+        Lay hi = coef(lay[NL * D_NI], pair[NL]);
+        double as, ds;
+        bottom_row_v(hi, s.bsurf_i[nb], rsf, as, ds);
+        row[2 * NL] = make_double2(as, ds);
+        double2 nxt = pair[NL - 1];
+        for (int n = NL - 1; n >= 1; --n) {
+            const double2 cur = nxt;
+            if (n > 1) nxt = pair[n - 1];
+            const Lay lo = coef(lay[n * D_NI], cur);
+            double ao, dd;
+            fast_rows(lo, hi, as, ds, ao, dd, odd);
+            row[2 * n + 1] = make_double2(ao, dd);
+            row[2 * n] = make_double2(as, ds);
+            hi = lo;
+        }
+        {
+            const double cf = hi.gama - 1.0, den = hi.gama + 1.0 - cf * as;
+            odd |= out_of_range(den);
+            const double x = rcp_s(den);
+            row[1] = make_double2(0.0 * x, (btop - hi.cmm1 - cf * ds) * x);
+        }
+        if (!odd) {
+            // pass D
+            double xprev = 0.0;
+            double2 n1 = row[1], n2 = row[2], np = pair[1];
+            double nm = mid[1];
+            for (int n = 1; n <= NL; ++n) {
+                const double2 r1 = n1, r2 = n2, p = np;
+                const double dtk = nm;
+                if (n < NL) {
+                    n1 = row[2 * n + 1];
+                    n2 = row[2 * n + 2];
+                    np = pair[n + 1];
+                    nm = mid[n + 1];
+                }
+                const IrLayer r = lay[n * D_NI];
+                double lam, gama, term;
+                lay3(r, p.x, lam, gama, term);
+                const double b1 = quot(r.pdif, p.y, rcp_n(p.y));
+                const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
+                const double xb = r2.y - r2.x * xa;
+                xprev = xb;
+                double xk1, xk2;
+                unmix(xa, xb, xk1, xk2);
+                const double ep = exp_r(dmin(lam * dtk, TAUMAX)), em = rcp_n(ep);
+                const double bt = b1 * term, bb = r.b0 + b1 * dtk;
+                const double u = xk1 * ep, v = gama * xk2 * em;
+                const double p1 = u + v + (bb + bt);
+                const double m1 = u * gama + xk2 * em + (bb - bt);
+                fmp[(size_t)(n - 1) * ROW_BLK] = p1 * PI_D;
+                fmm[(size_t)(n - 1) * ROW_BLK] = m1 * PI_D;
+                if (n == 1) {
+                    const double fup = xk1 + gama * xk2 + (r.b0 + bt);
+                    const double fdn = xk1 * gama + xk2 + (r.b0 - bt);
+                    *sc0 = (fup - fdn) * PI_D;
+                }
+            }
+            return 0;
+        }
+    }
+    general_ir(sg, c, j, block, max_nl, K, ki, w.g, fmp, fmm, sc0);
+    return 0;
+}
+
+// ---------------------------------------------------------------- visible
+// Pass A of system t: TAUs per layer (kept with KEEP), the surface values,
+// and whether an operand left the range.
+template <bool KEEP, bool F32>
+struct VisPassA {
+    double taugsurf = 0.0, tau = 0.0, tclev = 0.0, tce1 = 0.0;
+    bool odd = false;
+    __device__ __forceinline__ void run(const SegDev &sg, int t, const ColSmem &s, const double *__restrict__ kv,
+                                        const float *__restrict__ kvf, SolveLocal &w) {
+        const int L = sg.L, NL = L + 1;
+        const int nb = t / D_NG, ng = t - nb * D_NG;
+        const bool gas = ng < D_NG - 1;
+        const size_t to = (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
+        const double *tb = kv + to, *ray = s.trayaer + nb;
+        const float *tbf = F32 ? kvf + to : nullptr;
+        const VisLayer *lay = s.lay_v + nb;
+        auto dtauk = [&](int k) -> double {
+            if (gas) {
+                const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
+                taugsurf += tg;
+                return tg + ray[k * D_NV];
+            }
+            return ray[k * D_NV];
+        };
+        double2 *pair = w.pair(), *depth = w.depth();
+        odd = (*s.odd >> nb) & 1;
+        const double tc2 = 0.0 + dtauk(2);
+        double tc = tc2, fprev = 0.0;
+        for (int l = 1; l <= NL; ++l) {
+            const int k = 2 * l + 1;
+            const double da = dtauk(k);
+            const double tcA = tc + da;
+            double dt = da, tcB = tcA;
+            if (l <= L) {
+                const double db = dtauk(k + 1);
+                tcB = tcA + db;
+                dt = da + db;
+            }
+            const VisLayer r = lay[l * D_NV];
+            const double wb = quot(r.wnum, dt, rcp_n(dt));
+            const double f = 1.0 - wb * (r.cosb * r.cosb);
+            odd |= hi32(dt) - 0x2d300000u >= 0x19000000u || hi32(wb) >= 0x3ff00000u;   // [2^-300, 2^100), [0, 1)
+            const double dtl = dt * f;
+            if (KEEP) {
+                double m = 0.0;
+                if (l == 1) {
+                    tce1 = tc2 * f;
+                    m = tce1 + (tcA - tc2) * f;
+                } else if (l < NL) {
+                    m = tau + (tcA - tc) * fprev;
+                }
+                pair[l] = make_double2(quot(wb * (1.0 - r.cosb * r.cosb), f, rcp_n(f)), dtl);
+                depth[l] = make_double2(tau, m);
+            }
+            tau = tau + dtl;
+            fprev = f;
+            tc = tcB;
+        }
+        tclev = tc;
+    }
+};
+
+// Screen of system t of a day column: DETAU, CUMTAUV and the TLIMIT decision
+// (code/sfluxv.f90:60-75); true when the system is to be solved.
+template <bool F32>
+__device__ __forceinline__ bool fast_vis_screen(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
+                                                const ColSmem &s, const RtConst &K, const double *__restrict__ kv,
+                                                const float *__restrict__ kvf, SolveLocal &w,
+                                                unsigned int &nsolved) {
+    VisPassA<false, F32> a;
+    a.run(sg, t, s, kv, kvf, w);
+    const int nb = t / D_NG, ng = t - nb * D_NG;
+    if (a.odd) {
+        nsolved += general_vis<1, F32>(sg, c, t, block, max_nl, K, kv, kvf, w.g, nullptr, nullptr, nullptr);
+        return s.skip[t] == 0;
+    }
+    const size_t o = (size_t)c * NSYS_V + nb + D_NV * ng;
+    sg.cumtauv[o] = a.tclev;
+    if (ng < D_NG - 1 && K.fzerov[nb] >= R4(0.99)) {
+        s.skip[t] = 2;
+        return false;
+    }
+    sg.detau[o] = a.tau;
+    const bool skip = ng < D_NG - 1 && a.taugsurf < TLIMITS;
+    s.skip[t] = skip ? 1 : 0;
+    nsolved += skip ? 0 : 1;
+    return !skip;
+}
+
+// Solve of a kept visible system.
+template <bool F32>
+__device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
+                                         const RtConst &K, const double *__restrict__ kv,
+                                         const float *__restrict__ kvf, SolveLocal &w, double *fmp, double *fmm,
+                                         double *sc) {
+    const ColSmem s = carve_smem(block, max_nl, nullptr, false);
+    const int NL = sg.L + 1, nb = t / D_NG;
+    const double u0 = sg.acosz[c], rsf = sg.als[c], f0pi = sg.sol[nb];
+    VisPassA<true, F32> a;
+    a.run(sg, t, s, kv, kvf, w);
+    // u0 in [2^-30, 2^30), the band's sun 0 or in [2^-60, 2^60)
+    bool odd = a.odd || hi32(u0) - 0x3e100000u >= 0x03c00000u || (f0pi != 0.0 && hi32(f0pi) - 0x3c300000u >= 0x07800000u);
+    if (!odd) {
+        double2 *pair = w.pair(), *depth = w.depth(), *src = w.src(), *row = w.row();
+        const double *cbs = s.cbs_v + nb;
+        const double rcp_u0 = rcp_n(u0), rcp_u02 = 1.0 / (u0 * u0);
+        const double s3 = (double)sqrtf(3.0f), s3h = (double)(sqrtf(3.0f) * 0.5f);
+        const double bsurf = rsf * u0 * f0pi * beam(a.tau, u0, rcp_u0);
+        // pass C; pair becomes (LAMDA, GAMA), src = (AM, AP)
+        auto coef = [&](int l, double2 p, double cb, double et_top, double et_bot) {
+            Lay y;
+            const double w0 = p.x;
+            const double g1 = s3h * (2.0 - w0 * (1.0 + cb));
+            const double g2 = (s3 * w0 * 0.5) * (1.0 - cb);
+            const double g3 = 0.5 * (1.0 - s3 * cb * u0);
+            const double l2 = g1 * g1 - g2 * g2;
+            odd |= hi32(l2) - 0x2d300000u >= 0x25800000u || out_of_range(g2);
+            const double lam = sqrt_n(l2);
+            y.gama = quot(g1 - lam, g2, rcp_s(g2));
+            const double g4 = 1.0 - g3;
+            double denom = lam * lam - rcp_u02;
+            if (denom == 0.0) denom = R4(1.E-10);
+            const double rd = rcp_s(denom);
+            const double am = quot(f0pi * w0 * (g4 * (g1 + rcp_u0) + g2 * g3), denom, rd);
+            const double ap = quot(f0pi * w0 * (g3 * (g1 - rcp_u0) + g2 * g4), denom, rd);
+            pair[l] = make_double2(lam, y.gama);
+            src[l] = make_double2(am, ap);
+            y.cpm1 = ap * et_top;
+            y.cmm1 = am * et_top;
+            y.cp = ap * et_bot;
+            y.cm = am * et_bot;
+            exp_terms(y, lam * p.y);
+            return y;
+        };
+        double et_bot = beam(a.tau, u0, rcp_u0), et_top = beam(depth[NL].x, u0, rcp_u0);
+        Lay hi = coef(NL, pair[NL], cbs[NL * D_NV], et_top, et_bot);
+        double as, ds;
+        bottom_row_v(hi, bsurf, rsf, as, ds);
+        row[2 * NL] = make_double2(as, ds);
+        double2 nxt = pair[NL - 1];
+        double nd = depth[NL - 1].x;
+        for (int n = NL - 1; n >= 1; --n) {
+            const double2 cur = nxt;
+            const double d = nd;
+            if (n > 1) {
+                nxt = pair[n - 1];
+                nd = depth[n - 1].x;
+            }
+            et_bot = et_top;
+            et_top = beam(d, u0, rcp_u0);
+            const Lay lo = coef(n, cur, cbs[n * D_NV], et_top, et_bot);
+            double ao, dd;
+            fast_rows(lo, hi, as, ds, ao, dd, odd);
+            row[2 * n + 1] = make_double2(ao, dd);
+            row[2 * n] = make_double2(as, ds);
+            hi = lo;
+        }
+        {
+            const double cf = hi.gama - 1.0, den = hi.gama + 1.0 - cf * as;
+            odd |= out_of_range(den);
+            const double x = rcp_s(den);
+            row[1] = make_double2(0.0 * x, (0.0 - hi.cmm1 - cf * ds) * x);
+        }
+        if (!odd) {
+            // pass D
+            double xprev = 0.0;
+            double2 n1 = row[1], n2 = row[2], nl = pair[1], ns = src[1], nt = depth[1];
+            for (int n = 1; n <= NL; ++n) {
+                const double2 r1 = n1, r2 = n2, t2 = nt;
+                const double lam = nl.x, gama = nl.y, am = ns.x, ap = ns.y;
+                if (n < NL) {
+                    n1 = row[2 * n + 1];
+                    n2 = row[2 * n + 2];
+                    nl = pair[n + 1];
+                    ns = src[n + 1];
+                    nt = depth[n + 1];
+                }
+                const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
+                const double xb = r2.y - r2.x * xa;
+                xprev = xb;
+                double xk1, xk2;
+                unmix(xa, xb, xk1, xk2);
+                if (n == 1) {
+                    sc[0] = xk1 + gama * xk2 + ap;
+                    sc[ROW_BLK] = xk1 * gama + xk2 + am + u0 * f0pi;
+                }
+                // the middle of the layer; its bottom in the last one
+                const double top = n == 1 && n < NL ? a.tce1 : t2.x;
+                const double at = n < NL ? t2.y : a.tau;
+                const double ep = exp_r(dmin(TAUMAX, lam * (at - top))), em = rcp_n(ep);
+                const double et = beam(n < NL ? at : dmin(at, TAUMAX), u0, rcp_u0);
+                fmp[(size_t)(n - 1) * ROW_BLK] = xk1 * ep + gama * xk2 * em + ap * et;
+                const double m = xk1 * ep * gama + xk2 * em + am * et;
+                if (n == NL) sc[2 * ROW_BLK] = m;
+                fmm[(size_t)(n - 1) * ROW_BLK] = m + u0 * f0pi * et;
+            }
+            return;
+        }
+    }
+    general_vis<2, F32>(sg, c, t, block, max_nl, K, kv, kvf, w.g, fmp, fmm, sc);
+}
+
+}  // namespace fp64
+}  // namespace mgcm

@@ -4,6 +4,7 @@
 // code/sfluxi.f90:51-62 and code/gfluxi.f90:69-87.
 #pragma once
 #include "rt_column.cuh"
+#include "rt_fastmath.cuh"
 
 namespace mgcm {
 
@@ -40,6 +41,13 @@ struct Check {
         }
     }
 };
+
+// A layer the solves' fast arithmetic may take: |COSBAR| < 1, a numerator of
+// the single-scattering albedo that is 0 or in [2^-300, 2^300).  Any physical
+// layer is; a column with another one goes through the general solve.
+__device__ __forceinline__ bool usual_layer(double cosb, double wnum) {
+    return fabs(cosb) < 1.0 && (wnum == 0.0 || (wnum > 0.0 && !out_of_range(wnum)));
+}
 
 // Level item k (2..LEV+1) of column c: bins, U, DPR and the TAUREF ratios.
 // With V the item checks the level's inputs; item 2 also level 1 and the
@@ -81,6 +89,7 @@ __device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, Co
             s.tref_v[k] = tauref[k - 1] / (db ? db[NREFV_IDX] : qxv[(size_t)(NREFV_IDX)*LEV1 + k - 1]);
             s.tref_i[k] = tauref[k - 1] / (db ? db[NREFV_IDX] : qxref[k - 1]);
             s.tref_c[k] = cld ? taucld[k - 1] / qxcld[k - 1] : 0.0 / 1.0;
+            if (k == 2) *s.odd = 0;   // the band items come after a barrier
         } else {
             s.tref_i[k] = db ? 0.0 : tauref[k - 1];
             s.tref_c[k] = cld ? taucld[k - 1] : 0.0;
@@ -170,6 +179,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 g2 = cld ? gc[k - 1] : 0.0;
                 check(k - 1);
             };
+            bool usual = true;
             double tra, tla, tca, ga, gca;
             if (l == 0) {
                 lvl(2, tra, tla, tca, ga, gca);
@@ -180,18 +190,23 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 lvl(k, tra, tla, tca, ga, gca);
                 lvl(k + 1, trb, tlb, tcb, gb, gcb);
                 const double cb = (ga * tla + gb * tlb + gca * tca + gcb * tcb) / (tra + trb + tla + tlb + tca + tcb);
-                s.cosb_v[l * D_NV + nw - 1] = cb;
+                s.lay_v[l * D_NV + nw - 1].cosb = cb;
                 s.cbs_v[l * D_NV + nw - 1] = cb / (1.0 + cb);   // code/getdetau.f90:29-56
-                s.wnum_v[l * D_NV + nw - 1] = tla + tlb + tca + tcb + (tra + trb) * R4(0.9999);
+                const double wn = tla + tlb + tca + tcb + (tra + trb) * R4(0.9999);
+                s.lay_v[l * D_NV + nw - 1].wnum = wn;
+                usual = usual_layer(cb, wn);
             } else {
                 const int k = LEV;
                 lvl(k, tra, tla, tca, ga, gca);
                 const double cb = (ga * tla + gca * tca) / (tra + tla + tca);
-                s.cosb_v[l * D_NV + nw - 1] = cb;
+                s.lay_v[l * D_NV + nw - 1].cosb = cb;
                 s.cbs_v[l * D_NV + nw - 1] = cb / (1.0 + cb);
-                s.wnum_v[l * D_NV + nw - 1] = tla + tca + tra * R4(0.9999);
+                const double wn = tla + tca + tra * R4(0.9999);
+                s.lay_v[l * D_NV + nw - 1].wnum = wn;
+                usual = usual_layer(cb, wn);
                 check(LEV);
             }
+            if (!usual) atomicOr(s.odd, 1 << (nw - 1));
         } else if (it < nitem_v + nitem_i) {
             const int j = it - nitem_v;
             const int l = j / D_NI, nw = j % D_NI + 1;
@@ -206,8 +221,8 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
             const double *qsc = cld ? sg.qsicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
             const double *gc = cld ? sg.gicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
             auto ext = [&](int k) {   // TAEROS, TCLOUD at level k <= LEV
-                s.taer_i[k * D_NI + nw - 1] = s.tref_i[k] * qx[(k - 1) * ks];
-                s.tcld_i[k * D_NI + nw - 1] = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
+                s.ext_i[k * D_NI + nw - 1].x = s.tref_i[k] * qx[(k - 1) * ks];
+                s.ext_i[k * D_NI + nw - 1].y = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
             };
             auto check = [&](int i) {
                 if (V) {
@@ -237,26 +252,22 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 const double tca = s.tref_c[k] * (cld ? qsc[k - 1] : 0.0);
                 const double tcb = s.tref_c[k + 1] * (cld ? qsc[k] : 0.0);
                 const double tauac = tla + tlb + tca + tcb;
-                s.wnum_i[l * D_NI + nw - 1] = tauac;
+                s.lay_i[l * D_NI + nw - 1].wnum = tauac;
                 double cb = 0.0;
                 if (tauac > 0.0)
                     cb = (gi[(k - 1) * ks] * tla + gi[k * ks] * tlb + (cld ? gc[k - 1] : 0.0) * tca +
                           (cld ? gc[k] : 0.0) * tcb) /
                          (tla + tlb + tca + tcb);
-                s.cosb_i[l * D_NI + nw - 1] = cb;
+                s.lay_i[l * D_NI + nw - 1].cosb = cb;
                 // Planck source terms (gfluxi.f90:219-239)
-                int nta, ntb;
-                if (l < NL) {
-                    ntb = planck_index(tlev[2 * l + 2 - 1], status);
-                    nta = planck_index(tlev[2 * l - 1], status);
-                    s.pdif_i[l * D_NI + nw - 1] = planck[(ntb - 1) * D_NI + nw - 1] - planck[(nta - 1) * D_NI + nw - 1];
-                    s.b0_i[l * D_NI + nw - 1] = planck[(nta - 1) * D_NI + nw - 1];
-                } else {
-                    nta = planck_index(tlev[2 * l + 1 - 1], status);
-                    ntb = planck_index(tlev[2 * l - 1], status);
-                    s.pdif_i[l * D_NI + nw - 1] = planck[(nta - 1) * D_NI + nw - 1] - planck[(ntb - 1) * D_NI + nw - 1];
-                    s.b0_i[l * D_NI + nw - 1] = planck[(ntb - 1) * D_NI + nw - 1];
-                }
+                const int na = planck_index(l < NL ? tlev[2 * l - 1] : tlev[2 * l + 1 - 1], status);
+                const int nb = planck_index(l < NL ? tlev[2 * l + 2 - 1] : tlev[2 * l - 1], status);
+                const double pa = planck[(na - 1) * D_NI + nw - 1], pb = planck[(nb - 1) * D_NI + nw - 1];
+                const double pd = l < NL ? pb - pa : pa - pb;
+                s.lay_i[l * D_NI + nw - 1].pdif = pd;
+                s.lay_i[l * D_NI + nw - 1].b0 = l < NL ? pa : pb;
+                if (!usual_layer(cb, tauac) || (pd != 0.0 && out_of_range(pd)))
+                    atomicOr(s.odd, 1 << (D_NV + nw - 1));
             }
         } else {
             // IR boundary terms (sfluxi.f90:51-62)
