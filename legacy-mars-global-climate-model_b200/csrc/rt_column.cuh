@@ -21,12 +21,17 @@ __device__ __forceinline__ int find_seg(const SegTable *__restrict__ st, int g) 
 // one 64-byte record so a thread fetches it with four 16-byte loads: the
 // bilinear weights LCOEF(1..4), WRATIO, U = Cmk*DPR, the element offset of
 // the (MT, MP, NH2O) corner within a band's table and the step to the
-// NH2O+1 row (0 where NH2O = 10, whose WRATIO is 0).
+// NH2O+1 row (0 where NH2O = 10, whose WRATIO is 0).  `same` compares the
+// second level of a layer (K = 2l+2) with the first, whose PMID and TMID
+// FILLPT makes equal (code/fillpt.f90:60-66): SAME_VALUE when the water is
+// equal too (the interpolated k is the first level's), SAME_CORNERS when only
+// WRATIO differs (the 8 table values are), 0 otherwise.
+constexpr int SAME_CORNERS = 1, SAME_VALUE = 2;
 struct alignas(16) KLevel {
     double lk[4];
     double wr, u;
     int kofs, kdh;
-    int pad[2];
+    int same, pad;
 };
 static_assert(sizeof(KLevel) == 64, "KLevel is one 64-byte record");
 
@@ -147,6 +152,15 @@ __device__ __forceinline__ int planck_index(double t, uint32_t *status) {
     return it;
 }
 
+// NH2O of tpindex (code/tpindex.f90:116-134).
+__device__ __forceinline__ int water_bin(const RtConst &c, double qh2o) {
+    if (qh2o <= c.wrefh2o[0]) return 1;
+    if (qh2o >= c.wrefh2o[D_NH - 1]) return D_NH;
+    for (int n = 2; n <= D_NH; ++n)
+        if (qh2o >= c.wrefh2o[n - 2] && qh2o < c.wrefh2o[n - 1]) return n - 1;
+    return 1;
+}
+
 // tpindex (code/tpindex.f90:72-134).  The log10 bin search is done on the
 // pressure against host-computed limits so bins agree bit-for-bit with the
 // host libm; the weight T uses mgcm_rt_log10, bit-identical to the oracle's.
@@ -172,20 +186,10 @@ __device__ __forceinline__ void tpindex_dev(const RtConst &c, double pw, double 
     lk[1] = tt * (1.0 - uu);
     lk[2] = tt * uu;
     lk[3] = (1.0 - tt) * uu;
+    nh = water_bin(c, qh2o);
     wratio = 0.0;
-    nh = 1;
-    if (qh2o <= c.wrefh2o[0]) {
-        nh = 1;
-    } else if (qh2o >= c.wrefh2o[D_NH - 1]) {
-        nh = D_NH;
-    } else {
-        for (int n = 2; n <= D_NH; ++n)
-            if (qh2o >= c.wrefh2o[n - 2] && qh2o < c.wrefh2o[n - 1]) {
-                nh = n - 1;
-                wratio = (qh2o - c.wrefh2o[n - 2]) / (c.wrefh2o[n - 1] - c.wrefh2o[n - 2]);
-                break;
-            }
-    }
+    if (qh2o > c.wrefh2o[0] && nh < D_NH)
+        wratio = (qh2o - c.wrefh2o[nh - 1]) / (c.wrefh2o[nh] - c.wrefh2o[nh - 1]);
 }
 
 }  // namespace mgcm

@@ -134,7 +134,7 @@ template __global__ void rt_stage<true>(STAGE_ARGS);
 // contiguous run of list positions in ascending order; its base and count go
 // to the column's meta words.
 template <bool F32>
-__global__ void __launch_bounds__(128, 8)   // 64 registers: 8 CTAs/SM (measured 6% faster than 80)
+__global__ void __launch_bounds__(128, 8)   // 64 registers (5 / 6 / 8 CTAs per SM: 10.60 / 10.45 / 10.34 ms)
 rt_fp64_screen(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ kv,
                const double *__restrict__ ki, const __grid_constant__ RtConst K, int *__restrict__ list_v,

@@ -9,6 +9,9 @@
 // (and, visible, the root and the divisor of GAMA).  What else is divided by
 // or rooted then lies in range: 1 - W0 COSB >= 2^-53, and ALPHA within 2^27
 // of 1, EP in [1, exp(35)].
+//
+// IR solve of 8,192 x 24 columns: 896 instructions issued per layer and warp
+// in the general arithmetic, 617 in this one.
 #pragma once
 #include "rt_fp64_sys.cuh"
 
@@ -18,9 +21,9 @@ namespace fp64 {
 // Per-layer values of a system in local memory, two to a 16-byte access.
 struct SolveLocal {
     SysLocal g;   // the general solve's arrays; the fast ones lie over them
-    __device__ __forceinline__ double2 *pair() { return reinterpret_cast<double2 *>(g.a0); }        // layer l: W0, DTAU
+    __device__ __forceinline__ double2 *pair() { return reinterpret_cast<double2 *>(g.a0); }        // layer l: W0, DTAU (IR: DTAUK of its levels)
     __device__ __forceinline__ double2 *depth() { return reinterpret_cast<double2 *>(g.a2); }       // visible: TAU, mid TAU
-    __device__ __forceinline__ double *mid() { return g.a2; }                                       // IR: TAUCUM step
+    __device__ __forceinline__ double *mid() { return g.a2; }                                       // IR: WBARI
     __device__ __forceinline__ double2 *src() { return reinterpret_cast<double2 *>(g.a4); }         // visible: AM, AP
     __device__ __forceinline__ double2 *row() { return reinterpret_cast<double2 *>(g.as); }         // row i: AS, DS
 };
@@ -45,6 +48,42 @@ static __device__ __noinline__ unsigned int general_vis(const SegDev &sg, int c,
     solve_vis<MODE, F32>(sg, c, t / D_NG + 1, t % D_NG + 1, t, s, K, kv, w, nsolved, row, rdn, scr, scr + ROW_BLK,
                          scr + 2 * ROW_BLK, kvf, ROW_BLK);
     return nsolved;
+}
+
+// TAUGAS of the two levels K = k, k+1 of a layer (taugas_at, taugas_f).  The
+// second level's table values are mostly the first one's (KLevel::same): a
+// layer's 16 gathered values become 8, its two interpolations one.  With the
+// one-pass IR solve below: 64,800 x 24 FP64 11.45 -> 10.3 ms, 16,200 x 48
+// 7.80 -> 7.03 ms, 60 x 24 235 -> 215 us.
+template <bool F32, class T>
+__device__ __forceinline__ void taugas_layer(const ColSmem &s, int k, const T *__restrict__ tb, T &t1, T &t2) {
+    const KLv kl = klev_load(s, k);
+    const T *p = tb + kl.kd.x;
+    const int dh = kl.kd.y;
+    T c[4], d[4];
+    c[0] = __ldg(p);
+    c[1] = __ldg(p + KT_DP);
+    c[2] = __ldg(p + KT_DT + KT_DP);
+    c[3] = __ldg(p + KT_DT);
+    p += dh;
+    d[0] = __ldg(p) - c[0];
+    d[1] = __ldg(p + KT_DP) - c[1];
+    d[2] = __ldg(p + KT_DT + KT_DP) - c[2];
+    d[3] = __ldg(p + KT_DT) - c[3];
+    auto value = [&](T wr) {
+        const T k1 = c[0] + wr * d[0], k2 = c[1] + wr * d[1], k3 = c[2] + wr * d[2], k4 = c[3] + wr * d[3];
+        return (T)kl.lk01.x * k1 + (T)kl.lk01.y * k2 + (T)kl.lk23.x * k3 + (T)kl.lk23.y * k4;
+    };
+    const double2 *q2 = reinterpret_cast<const double2 *>(s.klev + k + 1);
+    const double2 wu = q2[2];
+    const int same = reinterpret_cast<const int4 *>(q2 + 3)->z;
+    const T v = value((T)kl.wu.x);
+    t1 = (F32 ? (T)s.dpr[k] : (T)kl.wu.y) * v;
+    const T u2 = F32 ? (T)s.dpr[k + 1] : (T)wu.y;
+    if (same == SAME_VALUE) t2 = u2 * v;
+    else if (same == SAME_CORNERS) t2 = u2 * value((T)wu.x);
+    else if constexpr (F32) t2 = taugas_f(s, k + 1, tb);
+    else t2 = taugas_at(s, k + 1, tb);
 }
 
 // x / u0 capped at MAXEXP, y = 1 / u0 (GFLUXV's beam exponents).
@@ -90,148 +129,188 @@ __device__ __forceinline__ void fast_rows(const Lay &lo, const Lay &hi, double &
 }
 
 // ---------------------------------------------------------------- infrared
-// System j of column c: pass A with the TLIMIT decision (code/sfluxi.f90:72-75),
-// then the solve.  Returns 0 solved, 1 skipped (TLIMIT), 2 no work, and
-// writes the column's skip entry.
+// TAUGSURF of an IR system in the reference order (code/optci.f90:143-167).
+static __device__ __noinline__ double ir_taugsurf(unsigned char *block, int max_nl, int lev,
+                                                  const double *__restrict__ tb) {
+    const ColSmem s = carve_smem(block, max_nl, nullptr, false);
+    double taug = 0.0;
+    for (int k = 2; k <= lev; ++k) taug += taugas_at(s, k, tb);
+    return taug;
+}
+
+// System j of column c: the TLIMIT decision (code/sfluxi.f90:72-75), then the
+// solve.  Returns 0 solved, 1 skipped (TLIMIT), 2 no work, and writes the
+// column's skip entry.
+//
+// Optical depths, coefficients and elimination run in one bottom-up pass, so
+// a layer's table gathers overlap the arithmetic of the ones before it; a
+// pass of its own for the gathers (top-down, as the reference's) was bound
+// by their latency and sent 24 more bytes per layer through local memory.
+// What needs the top-down order is formed in pass D (TAUCUMI, for the middle
+// of the layers) or decided apart: the gas optical depths are summed bottom-up
+// here, and where that sum, at most 1e-13 off the reference's, does not
+// decide the TLIMIT test -- or a depth is negative -- they are summed again.
 __device__ __forceinline__ int fast_ir(const SegDev &sg, int c, int j, unsigned char *block, int max_nl,
                                        const RtConst &K, const double *__restrict__ ki, SolveLocal &w, double *fmp,
                                        double *fmm, double *sc0) {
     const ColSmem s = carve_smem(block, max_nl, nullptr, false);
     const int L = sg.L, NL = L + 1, LEV = 2 * L + 3;
     const int nb = j / D_NG, ng = j - nb * D_NG;   // 0-based band and Gauss point
-    if (ng < D_NG - 1 && K.fzeroi[nb] >= R4(0.99)) return s.skip[NSYS_V + j] = 2;
     const bool gas = ng < D_NG - 1;
+    if (gas && K.fzeroi[nb] >= R4(0.99)) return s.skip[NSYS_V + j] = 2;
     const double *tb = ki + (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
     const double2 *ext = s.ext_i + nb;
     const IrLayer *lay = s.lay_i + nb;
-    double taug = 0.0;
-    auto dtauk = [&](int k) -> double {
-        const double2 e = ext[k * D_NI];
-        if (gas) {
-            const double tg = taugas_at(s, k, tb);
-            taug += tg;
-            return tg + e.x + e.y;
-        }
-        return e.x + e.y;
-    };
-    // pass A: pair = (WBARI, DTAUI), mid = TAUCUMI(2l+1) - TAUCUMI(2l)
-    double2 *pair = w.pair(), *row = w.row();
-    double *mid = w.mid();
+    double2 *pair = w.pair(), *row = w.row();   // pair: DTAUKI of the layer's two levels
+    double *w0s = w.mid();                      // WBARI
     const double tiny = R4(1.0E-9);
+    const double rsf = sg.albi[c];
+    double taug = 0.0;
+    unsigned neg = 0;
     bool odd = (*s.odd >> (D_NV + nb)) & 1;
-    double tc = 0.0 + dtauk(2);
-    for (int l = 1; l <= NL; ++l) {
-        const int k = 2 * l + 1;
-        const double da = dtauk(k);
-        const double tcA = tc + da;
-        double dt = da, tcB = tcA;
-        if (k + 1 <= LEV) {
-            const double db = dtauk(k + 1);
-            tcB = tcA + db;
-            dt = da + db;
-        }
-        // the reference adds 1.D-50 to DTAUI: without effect above its TINY of 1e-9
-        const bool thick = dt > tiny;
+    auto one_level = [&](int k) {   // DTAUKI(k)
+        const double2 e = ext[k * D_NI];
+        if (!gas) return e.x + e.y;
+        const double tg = taugas_at(s, k, tb);
+        taug += tg;
+        neg |= hi32(tg);
+        return tg + e.x + e.y;
+    };
+    // LAMDA, GAMA, TERM of a layer (code/gfluxi.f90:69-93), UBARI = 0.5.
+    // Passes C and D both evaluate them, B1 too: cheaper than a round trip
+    // of four more values per layer through local memory.
+    auto lay3 = [&](const IrLayer &r, double w0, double &lam, double &gama, double &term) {
+        const double d = 1.0 - w0 * r.cosb, y = rcp_n(d);
+        const double alpha = sqrt_n(quot(1.0 - w0, d, y));
+        const double ap1 = 1.0 + alpha;
+        lam = alpha * d * 2.0;
+        gama = quot(1.0 - alpha, ap1, rcp_n(ap1));
+        term = 0.5 * y;
+    };
+    // DTAUI and 1/DTAUI; the reference's added 1.D-50 has no effect above its TINY of 1e-9
+    auto depth = [&](double dt, bool &thick, double &y) {
+        thick = dt > tiny;
         dt = thick ? dt : tiny;
-        const double wb = thick ? quot(lay[l * D_NI].wnum, dt, rcp_n(dt)) : 0.0;
-        odd |= hi32(dt) >= 0x46300000u || hi32(wb) >= 0x3ff00000u;   // DTAUI < 2^100, 0 <= WBARI < 1
-        pair[l] = make_double2(wb, dt);
-        mid[l] = l < NL ? tcA - tc : dt;
-        tc = tcB;
+        y = rcp_n(dt);
+        return dt;
+    };
+    // pass C of one layer, its two optical depths summed in dt
+    double dt1 = 0.0;
+    auto coef = [&](int l, double dtsum) {
+        const IrLayer r = lay[l * D_NI];
+        bool thick;
+        double ydt;
+        const double dt = depth(dtsum, thick, ydt);
+        const double w0 = thick ? quot(r.wnum, dt, ydt) : 0.0;
+        odd |= hi32(dt) >= 0x46300000u || hi32(w0) >= 0x3ff00000u;   // DTAUI < 2^100, 0 <= WBARI < 1
+        w0s[l] = w0;
+        dt1 = dt;
+        Lay y;
+        double lam, term;
+        lay3(r, w0, lam, y.gama, term);
+        const double b1 = quot(r.pdif, dt, ydt);
+        const double bt = b1 * term, bb = r.b0 + b1 * dt;
+        y.cp = bb + bt;
+        y.cm = bb - bt;
+        y.cpm1 = r.b0 + bt;
+        y.cmm1 = r.b0 - bt;
+        exp_terms(y, lam * dt);
+        return y;
+    };
+    const double dlast = one_level(LEV);
+    pair[NL] = make_double2(dlast, 0.0);
+    Lay hi = coef(NL, dlast);
+    double as, ds;
+    bottom_row_v(hi, s.bsurf_i[nb], rsf, as, ds);
+    row[2 * NL] = make_double2(as, ds);
+    for (int n = NL - 1; n >= 1; --n) {
+        const int k = 2 * n + 1;
+        const double2 e1 = ext[k * D_NI], e2 = ext[(k + 1) * D_NI];
+        double da, db;
+        if (gas) {
+            double t1, t2;
+            taugas_layer<false>(s, k, tb, t1, t2);
+            taug += t2;
+            taug += t1;
+            neg |= hi32(t1) | hi32(t2);
+            da = t1 + e1.x + e1.y;
+            db = t2 + e2.x + e2.y;
+        } else {
+            da = e1.x + e1.y;
+            db = e2.x + e2.y;
+        }
+        pair[n] = make_double2(da, db);
+        const Lay lo = coef(n, da + db);
+        double ao, dd;
+        fast_rows(lo, hi, as, ds, ao, dd, odd);
+        row[2 * n + 1] = make_double2(ao, dd);
+        row[2 * n] = make_double2(as, ds);
+        hi = lo;
     }
-    if (gas && taug < TLIMITI) return s.skip[NSYS_V + j] = 1;
+    double tc = 0.0 + one_level(2);
+    if (gas) {
+        bool skip = taug < TLIMITI;
+        if ((neg >> 31) || !(fabs(taug - TLIMITI) > 1e-12 * TLIMITI))
+            skip = ir_taugsurf(block, max_nl, LEV, tb) < TLIMITI;
+        if (skip) return s.skip[NSYS_V + j] = 1;
+    }
     s.skip[NSYS_V + j] = 0;
-    if (!odd) {
+    double as1, ds1;
+    {
         const double *plev = sg.plev + (size_t)c * LEV;
-        const double rsf = sg.albi[c];
-        const double tautop = pair[1].y * plev[2 - 1] / (plev[4 - 1] - plev[2 - 1]);
+        const double tautop = dt1 * plev[2 - 1] / (plev[4 - 1] - plev[2 - 1]);
         const double btop = (1.0 - mgcm_rt_exp(-tautop / UBARI)) * s.pltop_i[nb];
-        // LAMDA, GAMA, TERM of a layer (code/gfluxi.f90:69-93), UBARI = 0.5.
-        // Passes C and D both evaluate them, B1 too: cheaper than a round
-        // trip of four more values per layer through local memory.
-        auto lay3 = [&](const IrLayer &r, double w0, double &lam, double &gama, double &term) {
-            const double d = 1.0 - w0 * r.cosb, y = rcp_n(d);
-            const double alpha = sqrt_n(quot(1.0 - w0, d, y));
-            const double ap1 = 1.0 + alpha;
-            lam = alpha * d * 2.0;
-            gama = quot(1.0 - alpha, ap1, rcp_n(ap1));
-            term = 0.5 * y;
-        };
-        // pass C
-        auto coef = [&](const IrLayer &r, double2 p) {
-            Lay y;
-            double lam, term;
-            lay3(r, p.x, lam, y.gama, term);
-            const double b1 = quot(r.pdif, p.y, rcp_n(p.y));
-            const double bt = b1 * term, bb = r.b0 + b1 * p.y;
-            y.cp = bb + bt;
-            y.cm = bb - bt;
-            y.cpm1 = r.b0 + bt;
-            y.cmm1 = r.b0 - bt;
-            exp_terms(y, lam * p.y);
-            return y;
-        };
-        Lay hi = coef(lay[NL * D_NI], pair[NL]);
-        double as, ds;
-        bottom_row_v(hi, s.bsurf_i[nb], rsf, as, ds);
-        row[2 * NL] = make_double2(as, ds);
-        double2 nxt = pair[NL - 1];
-        for (int n = NL - 1; n >= 1; --n) {
-            const double2 cur = nxt;
-            if (n > 1) nxt = pair[n - 1];
-            const Lay lo = coef(lay[n * D_NI], cur);
-            double ao, dd;
-            fast_rows(lo, hi, as, ds, ao, dd, odd);
-            row[2 * n + 1] = make_double2(ao, dd);
-            row[2 * n] = make_double2(as, ds);
-            hi = lo;
+        const double cf = hi.gama - 1.0, den = hi.gama + 1.0 - cf * as;
+        odd |= out_of_range(den);
+        const double x = rcp_s(den);
+        as1 = 0.0 * x;
+        ds1 = (btop - hi.cmm1 - cf * ds) * x;
+    }
+    if (odd) {
+        general_ir(sg, c, j, block, max_nl, K, ki, w.g, fmp, fmm, sc0);
+        return 0;
+    }
+    // pass D
+    double xprev = 0.0;
+    double2 n1 = make_double2(as1, ds1), n2 = row[2], np = pair[1];
+    double nw = w0s[1];
+    for (int n = 1; n <= NL; ++n) {
+        const double2 r1 = n1, r2 = n2, p = np;
+        const double w0 = nw;
+        if (n < NL) {
+            n1 = row[2 * n + 1];
+            n2 = row[2 * n + 2];
+            np = pair[n + 1];
+            nw = w0s[n + 1];
         }
-        {
-            const double cf = hi.gama - 1.0, den = hi.gama + 1.0 - cf * as;
-            odd |= out_of_range(den);
-            const double x = rcp_s(den);
-            row[1] = make_double2(0.0 * x, (btop - hi.cmm1 - cf * ds) * x);
-        }
-        if (!odd) {
-            // pass D
-            double xprev = 0.0;
-            double2 n1 = row[1], n2 = row[2], np = pair[1];
-            double nm = mid[1];
-            for (int n = 1; n <= NL; ++n) {
-                const double2 r1 = n1, r2 = n2, p = np;
-                const double dtk = nm;
-                if (n < NL) {
-                    n1 = row[2 * n + 1];
-                    n2 = row[2 * n + 2];
-                    np = pair[n + 1];
-                    nm = mid[n + 1];
-                }
-                const IrLayer r = lay[n * D_NI];
-                double lam, gama, term;
-                lay3(r, p.x, lam, gama, term);
-                const double b1 = quot(r.pdif, p.y, rcp_n(p.y));
-                const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
-                const double xb = r2.y - r2.x * xa;
-                xprev = xb;
-                double xk1, xk2;
-                unmix(xa, xb, xk1, xk2);
-                const double ep = exp_r(dmin(lam * dtk, TAUMAX)), em = rcp_n(ep);
-                const double bt = b1 * term, bb = r.b0 + b1 * dtk;
-                const double u = xk1 * ep, v = gama * xk2 * em;
-                const double p1 = u + v + (bb + bt);
-                const double m1 = u * gama + xk2 * em + (bb - bt);
-                fmp[(size_t)(n - 1) * ROW_BLK] = p1 * PI_D;
-                fmm[(size_t)(n - 1) * ROW_BLK] = m1 * PI_D;
-                if (n == 1) {
-                    const double fup = xk1 + gama * xk2 + (r.b0 + bt);
-                    const double fdn = xk1 * gama + xk2 + (r.b0 - bt);
-                    *sc0 = (fup - fdn) * PI_D;
-                }
-            }
-            return 0;
+        const IrLayer r = lay[n * D_NI];
+        const double tcA = tc + p.x;
+        bool thick;
+        double ydt;
+        const double dt = depth(n < NL ? p.x + p.y : p.x, thick, ydt);
+        const double dtk = n < NL ? tcA - tc : dt;
+        tc = tcA + p.y;
+        double lam, gama, term;
+        lay3(r, w0, lam, gama, term);
+        const double b1 = quot(r.pdif, dt, ydt);
+        const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
+        const double xb = r2.y - r2.x * xa;
+        xprev = xb;
+        double xk1, xk2;
+        unmix(xa, xb, xk1, xk2);
+        const double ep = exp_r(dmin(lam * dtk, TAUMAX)), em = rcp_n(ep);
+        const double bt = b1 * term, bb = r.b0 + b1 * dtk;
+        const double u = xk1 * ep, v = gama * xk2 * em;
+        const double p1 = u + v + (bb + bt);
+        const double m1 = u * gama + xk2 * em + (bb - bt);
+        fmp[(size_t)(n - 1) * ROW_BLK] = p1 * PI_D;
+        fmm[(size_t)(n - 1) * ROW_BLK] = m1 * PI_D;
+        if (n == 1) {
+            const double fup = xk1 + gama * xk2 + (r.b0 + bt);
+            const double fdn = xk1 * gama + xk2 + (r.b0 - bt);
+            *sc0 = (fup - fdn) * PI_D;
         }
     }
-    general_ir(sg, c, j, block, max_nl, K, ki, w.g, fmp, fmm, sc0);
     return 0;
 }
 
@@ -265,13 +344,32 @@ struct VisPassA {
         double tc = tc2, fprev = 0.0;
         for (int l = 1; l <= NL; ++l) {
             const int k = 2 * l + 1;
-            const double da = dtauk(k);
-            const double tcA = tc + da;
-            double dt = da, tcB = tcA;
+            double da, dt, tcA, tcB;
             if (l <= L) {
-                const double db = dtauk(k + 1);
+                double db;
+                if (gas) {
+                    if constexpr (F32) {
+                        float t1, t2;
+                        taugas_layer<true>(s, k, tbf, t1, t2);
+                        da = t1;
+                        db = t2;
+                    } else {
+                        taugas_layer<false>(s, k, tb, da, db);
+                    }
+                    taugsurf += da;
+                    taugsurf += db;
+                    da = da + ray[k * D_NV];
+                    db = db + ray[(k + 1) * D_NV];
+                } else {
+                    da = ray[k * D_NV];
+                    db = ray[(k + 1) * D_NV];
+                }
+                tcA = tc + da;
                 tcB = tcA + db;
                 dt = da + db;
+            } else {
+                dt = da = dtauk(k);
+                tcA = tcB = tc + da;
             }
             const VisLayer r = lay[l * D_NV];
             const double wb = quot(r.wnum, dt, rcp_n(dt));

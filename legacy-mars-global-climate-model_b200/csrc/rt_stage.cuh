@@ -83,6 +83,13 @@ __device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, Co
             kl.lk[1] = lk[1];
             kl.lk[2] = lk[2];
             kl.lk[3] = lk[3];
+            kl.same = 0;
+            if ((k & 1) == 0 && k >= 4 && pmid[k - 1] == pmid[k - 2] && tmid[k - 1] == tmid[k - 2]) {
+                if (qh2o[k - 1] == qh2o[k - 2])
+                    kl.same = SAME_VALUE;
+                else if (water_bin(K, qh2o[k - 2]) == nh)
+                    kl.same = SAME_CORNERS;
+            }
             const double dpr = plev[k - 1] - plev[k - 2];
             s.dpr[k] = dpr;
             kl.u = 3.51e22 * dpr;
