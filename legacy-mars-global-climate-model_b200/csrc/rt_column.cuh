@@ -36,14 +36,19 @@ struct alignas(16) KLevel {
 static_assert(sizeof(KLevel) == 64, "KLevel is one 64-byte record");
 
 // What the IR systems of a band read per layer: COSBI, the numerator of
-// WBARI, Planck B0 and the numerator of B1 (B1*DTAU), two 16-byte loads.
+// WBARI, Planck B0 and the numerator of B1 (B1*DTAU), and TAEROS, TCLOUD of
+// the layer's levels K = 2l+1, 2l+2 (l = 0: level 2; l = NL: level LEV only).
+// One record, so a solver thread walks one pointer with 16-byte loads.
 struct alignas(16) IrLayer {
     double cosb, wnum, b0, pdif;
+    double2 ext[2];
 };
 
-// What the visible systems of a band read per layer in pass A.
+// What the visible systems of a band read per layer: COSBV, the numerator of
+// WBARV, TRAY+TAEROS+TCLOUD of its two levels, and COSBV/(1+COSBV), the
+// delta-Eddington COSBAR.
 struct alignas(16) VisLayer {
-    double cosb, wnum;
+    double cosb, wnum, ray[2], cbs, pad;
 };
 
 // Shared-memory layout of one column; sized by the launch's largest NL.
@@ -52,13 +57,9 @@ struct ColSmem {
     KLevel *klev;
     double *dpr;
     double *tref_v, *tref_i, *tref_c;   // TAUREF/QEXTREF (vis, IR), TAUREFCLD/QEXTREFCLD
-    // per level and band
-    double *trayaer;                    // [k][7] visible TRAY+TAEROS+TCLOUD
-    double2 *ext_i;                     // [k][5] IR TAEROS, TCLOUD
-    // per layer and band
-    VisLayer *lay_v;                    // [l][7]
-    double *cbs_v;                      // [l][7] COSBV/(1+COSBV), the delta-Eddington COSBAR
+    // per layer (0..NL) and band
     IrLayer *lay_i;                     // [l][5]
+    VisLayer *lay_v;                    // [l][7]
     double *bsurf_i, *pltop_i;          // [5]
     // reduction staging
     double *fmp, *fmm;                  // [sys][l]
@@ -70,6 +71,13 @@ struct ColSmem {
     double *fmnet_v, *fmnet_i;          // [l] reduced net fluxes for the divergences
     double *misc;                       // [4] NFLUXTOPV, NFLUXTOPI
     int day;
+    // TAEROS, TCLOUD of level k, IR band nw; TRAY+TAEROS+TCLOUD, visible band nw (1-based)
+    __device__ __forceinline__ double2 &ext(int k, int nw) const {
+        return lay_i[((k - 1) >> 1) * D_NI + nw - 1].ext[(k - 1) & 1];
+    }
+    __device__ __forceinline__ double &ray(int k, int nw) const {
+        return lay_v[((k - 1) >> 1) * D_NV + nw - 1].ray[(k - 1) & 1];
+    }
 };
 
 // Largest dynamic shared memory a CTA may use (227 KB opt-in on sm_100).
@@ -85,8 +93,7 @@ __host__ __device__ inline size_t col_smem_bytes(int nl, bool red_in_smem = true
     size_t b = 0;
     b += (lev1 + 1) * sizeof(KLevel);
     b += (lev1 + 1) * (1 + 3) * sizeof(double);
-    b += (lev1 + 1) * (D_NV + 2 * D_NI) * sizeof(double);
-    b += (nl + 1) * (3 * D_NV + 4 * D_NI) * sizeof(double);
+    b += (nl + 1) * (D_NV * sizeof(VisLayer) + D_NI * sizeof(IrLayer));
     b += 2 * D_NI * sizeof(double);
     if (red_in_smem) b += red_bytes(nl);
     b += 3 * NSYS * sizeof(double);
@@ -102,8 +109,6 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
     s.klev = reinterpret_cast<KLevel *>(base);   // base is 16-byte aligned
     // records first: 16-byte aligned
     unsigned char *q = base + (size_t)(lev1 + 1) * sizeof(KLevel);
-    s.ext_i = reinterpret_cast<double2 *>(q);
-    q += (size_t)(lev1 + 1) * D_NI * sizeof(double2);
     s.lay_i = reinterpret_cast<IrLayer *>(q);
     q += (size_t)(nl + 1) * D_NI * sizeof(IrLayer);
     s.lay_v = reinterpret_cast<VisLayer *>(q);
@@ -113,8 +118,6 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
     s.tref_v = take(lev1 + 1);
     s.tref_i = take(lev1 + 1);
     s.tref_c = take(lev1 + 1);
-    s.trayaer = take((lev1 + 1) * D_NV);
-    s.cbs_v = take((nl + 1) * D_NV);
     s.bsurf_i = take(D_NI);
     s.pltop_i = take(D_NI);
     if (!with_red) {

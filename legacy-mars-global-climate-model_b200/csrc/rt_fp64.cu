@@ -223,11 +223,7 @@ rt_ir_dense(const SegTable *__restrict__ st, int col_begin, int col_end, int max
     unsigned int nsolved = 0;
     const int n = (col_end - col_begin) * NSYS_I;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int cc = i / NSYS_I, j = i - cc * NSYS_I, g = col_begin + cc;
-        const SegDev &sg = st->seg[find_seg(st, g)];
-        double *row = fl + row_base(i, max_nl);
-        nsolved += fast_ir(sg, g - sg.col0, j, blocks + (size_t)cc * stride, max_nl, K, ktab, w, row,
-                           row + (size_t)max_nl * ROW_BLK, sc + sc_base(i)) == 0;
+        nsolved += fast_ir(st, col_begin, i, max_nl, blocks, stride, K, ktab, w, fl, sc) == 0;
     }
     if (nsys) {
         for (int o = 16; o > 0; o >>= 1) nsolved += __shfl_down_sync(0xffffffffu, nsolved, o);

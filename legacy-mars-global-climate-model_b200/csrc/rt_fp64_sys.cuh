@@ -203,13 +203,13 @@ __device__ void solve_vis(const SegDev &sg, int c, int nw, int ng, int sidx, Col
         if (ng < D_NG) {
             const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
             taugsurf += tg;
-            return tg + s.trayaer[k * D_NV + nw - 1];
+            return tg + s.ray(k, nw);
         }
-        return s.trayaer[k * D_NV + nw - 1];
+        return s.ray(k, nw);
     };
     // pass A: levels 2..LEV, TCIN prefix sums, delta-Eddington stream.
     // a0 = W0, a2 = scaled DTAU, a3 = TAU (1..NL+1), a4 = TAUCUM(2l+1); the
-    // scaled COSBAR of a layer is staged in the column block (cbs_v)
+    // scaled COSBAR of a layer is staged in the column block (VisLayer::cbs)
     const double tc2 = 0.0 + dtauk(2);
     double tc = tc2, tau = 0.0, fprev = 0.0, tcE1 = 0.0, tcLev = 0.0;
     for (int l = 1; l <= NL; ++l) {
@@ -304,16 +304,16 @@ __device__ void solve_vis(const SegDev &sg, int c, int nw, int ng, int sidx, Col
     double et_bot = mgcm_rt_exp(-dmin(w.a3[NL + 1] / u0, MAXEXP));
     double et_top = mgcm_rt_exp(-dmin(w.a3[NL] / u0, MAXEXP));
     // layer NL-1's inputs are fetched one step ahead
-    const double *cbs = s.cbs_v + nw - 1;   // layer l at cbs[l * D_NV]
-    double pw0 = w.a0[NL - 1], pcb = cbs[(NL - 1) * D_NV], pdt = w.a2[NL - 1], pa3 = w.a3[NL - 1];
-    Lay hi = coef(NL, w.a0[NL], cbs[NL * D_NV], w.a2[NL], et_top, et_bot);
+    const VisLayer *lv = s.lay_v + nw - 1;   // layer l at lv[l * D_NV]
+    double pw0 = w.a0[NL - 1], pcb = lv[(NL - 1) * D_NV].cbs, pdt = w.a2[NL - 1], pa3 = w.a3[NL - 1];
+    Lay hi = coef(NL, w.a0[NL], lv[NL * D_NV].cbs, w.a2[NL], et_top, et_bot);
     double as, ds;
     bottom_row(hi, NL, bsurf, rsf, w, as, ds);
     for (int n = NL - 1; n >= 1; --n) {
         const double w0 = pw0, cb = pcb, dtl = pdt, a3n = pa3;
         if (n > 1) {
             pw0 = w.a0[n - 1];
-            pcb = cbs[(n - 1) * D_NV];
+            pcb = lv[(n - 1) * D_NV].cbs;
             pdt = w.a2[n - 1];
             pa3 = w.a3[n - 1];
         }
@@ -402,7 +402,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
     const double *tb = ki + (size_t)(nw - 1) * D_NT * D_NP * D_NH * D_NGK + (ng - 1);
     double taugsurf = 0.0;
     auto dtauk = [&](int k) -> double {
-        const double ta = s.ext_i[k * D_NI + nw - 1].x, tcl = s.ext_i[k * D_NI + nw - 1].y;
+        const double ta = s.ext(k, nw).x, tcl = s.ext(k, nw).y;
         if (ng < D_NG) {
             const double tg = taugas_at(s, k, tb);
             taugsurf += tg;

@@ -71,7 +71,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
     const int oW = 0, oDT = NL, oTK = 2 * NL, oAS = 3 * NL, oDS = 5 * NL;   // AS(r) at oAS + r-1
     const double *tb = ki + (size_t)(nw - 1) * D_NT * D_NP * D_NH * D_NGK + (ng - 1);
     auto dtauk = [&](int k) -> double {
-        const double ta = s.ext_i[k * D_NI + nw - 1].x, tcl = s.ext_i[k * D_NI + nw - 1].y;
+        const double ta = s.ext(k, nw).x, tcl = s.ext(k, nw).y;
         if (ng < D_NG) return taugas_at(s, k, tb) + ta + tcl;
         return ta + tcl;
     };
@@ -218,9 +218,9 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     auto dtauk = [&](int k) -> double {
         if (ng < D_NG) {
             const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
-            return tg + s.trayaer[k * D_NV + nw - 1];
+            return tg + s.ray(k, nw);
         }
-        return s.trayaer[k * D_NV + nw - 1];
+        return s.ray(k, nw);
     };
     // pass A (code/optcv.f90:128-274, code/gfluxv.f90:76-103)
     const double tc2 = 0.0 + dtauk(2);
@@ -267,7 +267,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     // LAMDA, GAMA, AM, AP of a layer from W0, the scaled COSBAR (staged per
     // layer and band) and U0; pass C and pass D both evaluate them
     struct Co { double lam, gama, am, ap; };
-    const double *cbs = s.cbs_v + nw - 1;   // layer l at cbs[l * D_NV]
+    const VisLayer *lv = s.lay_v + nw - 1;   // layer l at lv[l * D_NV]
     auto co4 = [&](double w0, double cb) {
         Co r;
         const double g1 = s3h * (2.0 - w0 * (1.0 + cb));
@@ -300,8 +300,8 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     double et_bot = mgcm_rt_exp(-dmin(st.get(oTAU + NL) / u0, MAXEXP));
     double et_top = mgcm_rt_exp(-dmin(st.get(oTAU + NL - 1) / u0, MAXEXP));
     const int nm = NL >= 2 ? NL - 2 : 0;
-    double pw0 = st.get(oW + nm), pcb = cbs[(NL - 1) * D_NV], pdt = st.get(oDL + nm), pa3 = st.get(oTAU + nm);
-    Lay hi = coef(co4(st.get(oW + NL - 1), cbs[NL * D_NV]), st.get(oDL + NL - 1), et_top, et_bot);
+    double pw0 = st.get(oW + nm), pcb = lv[(NL - 1) * D_NV].cbs, pdt = st.get(oDL + nm), pa3 = st.get(oTAU + nm);
+    Lay hi = coef(co4(st.get(oW + NL - 1), lv[NL * D_NV].cbs), st.get(oDL + NL - 1), et_top, et_bot);
     double as, ds;
     bottom_row_v(hi, bsurf, rsf, as, ds);
     st.put(oAS + 2 * NL - 1, as);
@@ -310,7 +310,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
         const double w0 = pw0, cb = pcb, dtl = pdt, a3n = pa3;
         if (n > 1) {
             pw0 = st.get(oW + n - 2);
-            pcb = cbs[(n - 1) * D_NV];
+            pcb = lv[(n - 1) * D_NV].cbs;
             pdt = st.get(oDL + n - 2);
             pa3 = st.get(oTAU + n - 2);
         }
@@ -335,7 +335,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     double xprev = 0.0;
     double nas1 = st.get(oAS), nds1 = st.get(oDS), nas2 = st.get(oAS + 1), nds2 = st.get(oDS + 1);
     double nw0 = st.get(oW), na3 = st.get(oTAU), na4 = st.get(oTCM);
-    double ncb = cbs[1 * D_NV];
+    double ncb = lv[1 * D_NV].cbs;
     const double tbot = st.get(oTAU + NL);
     for (int n = 1; n <= NL; ++n) {
         const double as1 = nas1, ds1 = nds1, as2 = nas2, ds2 = nds2;
@@ -346,7 +346,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
             nas2 = st.get(oAS + 2 * n + 1);
             nds2 = st.get(oDS + 2 * n + 1);
             nw0 = st.get(oW + n);
-            ncb = cbs[(n + 1) * D_NV];
+            ncb = lv[(n + 1) * D_NV].cbs;
             na3 = st.get(oTAU + n);
             na4 = n + 1 < NL ? st.get(oTCM + n) : 0.0;
         }

@@ -41,7 +41,7 @@ __device__ __forceinline__ void quad_vis(const SegDev &sg, int c, int nw, int ng
     const float *tbf = F32 ? kvf + (size_t)(nw - 1) * D_NT * D_NP * D_NH * D_NGK + (ng - 1) : nullptr;
     const bool gas = ng < D_NG;
     auto dtauk = [&](int k) -> double {
-        const double tr = s.trayaer[k * D_NV + nw - 1];
+        const double tr = s.ray(k, nw);
         if (gas) {
             const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
             return tg + tr;
@@ -70,7 +70,7 @@ __device__ __forceinline__ void quad_vis(const SegDev &sg, int c, int nw, int ng
             const double f = 1.0 - wb * (cb * cb);
             fv[j] = f;
             w0v[j] = wb * (1.0 - cb * cb) / f;
-            cbv[j] = s.cbs_v[l * D_NV + nw - 1];
+            cbv[j] = s.lay_v[l * D_NV + nw - 1].cbs;
             dtl[j] = dt * f;
         }
     }
@@ -266,7 +266,7 @@ __device__ __forceinline__ void quad_ir(const SegDev &sg, int c, int nw, int ng,
     const double *tb = ki + (size_t)(nw - 1) * D_NT * D_NP * D_NH * D_NGK + (ng - 1);
     const bool gas = ng < D_NG;
     auto dtauk = [&](int k) -> double {
-        const double ta = s.ext_i[k * D_NI + nw - 1].x, tcl = s.ext_i[k * D_NI + nw - 1].y;
+        const double ta = s.ext(k, nw).x, tcl = s.ext(k, nw).y;
         if (gas) {
             const double tg = taugas_at(s, k, tb);
             return tg + ta + tcl;

@@ -18,14 +18,22 @@
 namespace mgcm {
 namespace fp64 {
 
-// Per-layer values of a system in local memory, two to a 16-byte access.
-struct SolveLocal {
-    SysLocal g;   // the general solve's arrays; the fast ones lie over them
-    __device__ __forceinline__ double2 *pair() { return reinterpret_cast<double2 *>(g.a0); }        // layer l: W0, DTAU (IR: DTAUK of its levels)
-    __device__ __forceinline__ double2 *depth() { return reinterpret_cast<double2 *>(g.a2); }       // visible: TAU, mid TAU
-    __device__ __forceinline__ double *mid() { return g.a2; }                                       // IR: WBARI
-    __device__ __forceinline__ double2 *src() { return reinterpret_cast<double2 *>(g.a4); }         // visible: AM, AP
-    __device__ __forceinline__ double2 *row() { return reinterpret_cast<double2 *>(g.as); }         // row i: AS, DS
+// Per-layer values of a system in local memory, a record per layer so that
+// a thread indexes them with one register, in 16-byte accesses: the rows 2l-1
+// and 2l of DSOLVER (AS, DS) and
+//   IR       DTAUKI of the layer's two levels;
+//   visible  (W0, DTAU), then (LAMDA, GAMA); TAU at the top and the middle; (AM, AP).
+struct alignas(16) IrSlot {
+    double2 odd, even, pair;
+};
+struct alignas(16) VisSlot {
+    double2 odd, even, pair, depth, src;
+};
+union SolveLocal {
+    SysLocal g;   // the general solve's
+    IrSlot ir[D_MAXNL + 1];
+    VisSlot vis[D_MAXNL + 1];
+    __device__ SolveLocal() {}
 };
 
 // The general solves, out of line: systems out of range only.  They carve the
@@ -86,6 +94,14 @@ __device__ __forceinline__ void taugas_layer(const ColSmem &s, int k, const T *_
     else t2 = taugas_at(s, k + 1, tb);
 }
 
+// Fetches the line of a global address into L1: the solves ask for the next
+// layer's records a layer ahead (64,800 x 24: 9.86 -> 9.62 ms FP64, 9.72 -> 9.37
+// ms MIXED).  Asking for the next layer's table values too was slower (11.2 ms):
+// with the per-layer values streaming through it, L1 has no room.
+__device__ __forceinline__ void prefetch_l1(const void *p) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
 // x / u0 capped at MAXEXP, y = 1 / u0 (GFLUXV's beam exponents).
 __device__ __forceinline__ double beam(double x, double u0, double y) {
     return exp_r(-dmin(quot(x, u0, y), MAXEXP));
@@ -138,8 +154,8 @@ static __device__ __noinline__ double ir_taugsurf(unsigned char *block, int max_
     return taug;
 }
 
-// System j of column c: the TLIMIT decision (code/sfluxi.f90:72-75), then the
-// solve.  Returns 0 solved, 1 skipped (TLIMIT), 2 no work, and writes the
+// System i % 85 of column i / 85 of the chunk: the TLIMIT decision
+// (code/sfluxi.f90:72-75) and the solve.  Returns 0 solved, 1 skipped (TLIMIT), 2 no work, and writes the
 // column's skip entry.
 //
 // Optical depths, coefficients and elimination run in one bottom-up pass, so
@@ -150,164 +166,172 @@ static __device__ __noinline__ double ir_taugsurf(unsigned char *block, int max_
 // of the layers) or decided apart: the gas optical depths are summed bottom-up
 // here, and where that sum, at most 1e-13 off the reference's, does not
 // decide the TLIMIT test -- or a depth is negative -- they are summed again.
-__device__ __forceinline__ int fast_ir(const SegDev &sg, int c, int j, unsigned char *block, int max_nl,
-                                       const RtConst &K, const double *__restrict__ ki, SolveLocal &w, double *fmp,
-                                       double *fmm, double *sc0) {
-    const ColSmem s = carve_smem(block, max_nl, nullptr, false);
-    const int L = sg.L, NL = L + 1, LEV = 2 * L + 3;
-    const int nb = j / D_NG, ng = j - nb * D_NG;   // 0-based band and Gauss point
-    const bool gas = ng < D_NG - 1;
-    if (gas && K.fzeroi[nb] >= R4(0.99)) return s.skip[NSYS_V + j] = 2;
-    const double *tb = ki + (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
-    const double2 *ext = s.ext_i + nb;
-    const IrLayer *lay = s.lay_i + nb;
-    double2 *pair = w.pair(), *row = w.row();   // pair: DTAUKI of the layer's two levels
-    double *w0s = w.mid();                      // WBARI
-    const double tiny = R4(1.0E-9);
-    const double rsf = sg.albi[c];
-    double taug = 0.0;
-    unsigned neg = 0;
-    bool odd = (*s.odd >> (D_NV + nb)) & 1;
-    auto one_level = [&](int k) {   // DTAUKI(k)
-        const double2 e = ext[k * D_NI];
-        if (!gas) return e.x + e.y;
-        const double tg = taugas_at(s, k, tb);
-        taug += tg;
-        neg |= hi32(tg);
-        return tg + e.x + e.y;
-    };
+__device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_begin, int i, int max_nl,
+                                       unsigned char *__restrict__ blocks, size_t stride, const RtConst &K,
+                                       const double *__restrict__ ki, SolveLocal &w, double *__restrict__ fl,
+                                       double *__restrict__ sc) {
+    double tc, as1, ds1;
+    unsigned flags;   // bit 0: out of range; bit 31: a negative gas optical depth
     // LAMDA, GAMA, TERM of a layer (code/gfluxi.f90:69-93), UBARI = 0.5.
     // Passes C and D both evaluate them, B1 too: cheaper than a round trip
     // of four more values per layer through local memory.
-    auto lay3 = [&](const IrLayer &r, double w0, double &lam, double &gama, double &term) {
-        const double d = 1.0 - w0 * r.cosb, y = rcp_n(d);
+    auto lay3 = [&](double cosb, double w0, double &lam, double &gama, double &term) {
+        const double d = 1.0 - w0 * cosb, y = rcp_n(d);
         const double alpha = sqrt_n(quot(1.0 - w0, d, y));
         const double ap1 = 1.0 + alpha;
         lam = alpha * d * 2.0;
         gama = quot(1.0 - alpha, ap1, rcp_n(ap1));
         term = 0.5 * y;
     };
-    // DTAUI and 1/DTAUI; the reference's added 1.D-50 has no effect above its TINY of 1e-9
-    auto depth = [&](double dt, bool &thick, double &y) {
-        thick = dt > tiny;
-        dt = thick ? dt : tiny;
-        y = rcp_n(dt);
-        return dt;
-    };
-    // pass C of one layer, its two optical depths summed in dt
-    double dt1 = 0.0;
-    auto coef = [&](int l, double dtsum) {
-        const IrLayer r = lay[l * D_NI];
-        bool thick;
-        double ydt;
-        const double dt = depth(dtsum, thick, ydt);
-        const double w0 = thick ? quot(r.wnum, dt, ydt) : 0.0;
-        odd |= hi32(dt) >= 0x46300000u || hi32(w0) >= 0x3ff00000u;   // DTAUI < 2^100, 0 <= WBARI < 1
-        w0s[l] = w0;
-        dt1 = dt;
-        Lay y;
-        double lam, term;
-        lay3(r, w0, lam, y.gama, term);
-        const double b1 = quot(r.pdif, dt, ydt);
-        const double bt = b1 * term, bb = r.b0 + b1 * dt;
-        y.cp = bb + bt;
-        y.cm = bb - bt;
-        y.cpm1 = r.b0 + bt;
-        y.cmm1 = r.b0 - bt;
-        exp_terms(y, lam * dt);
-        return y;
-    };
-    const double dlast = one_level(LEV);
-    pair[NL] = make_double2(dlast, 0.0);
-    Lay hi = coef(NL, dlast);
-    double as, ds;
-    bottom_row_v(hi, s.bsurf_i[nb], rsf, as, ds);
-    row[2 * NL] = make_double2(as, ds);
-    for (int n = NL - 1; n >= 1; --n) {
-        const int k = 2 * n + 1;
-        const double2 e1 = ext[k * D_NI], e2 = ext[(k + 1) * D_NI];
-        double da, db;
-        if (gas) {
-            double t1, t2;
-            taugas_layer<false>(s, k, tb, t1, t2);
-            taug += t2;
-            taug += t1;
-            neg |= hi32(t1) | hi32(t2);
-            da = t1 + e1.x + e1.y;
-            db = t2 + e2.x + e2.y;
-        } else {
-            da = e1.x + e1.y;
-            db = e2.x + e2.y;
-        }
-        pair[n] = make_double2(da, db);
-        const Lay lo = coef(n, da + db);
-        double ao, dd;
-        fast_rows(lo, hi, as, ds, ao, dd, odd);
-        row[2 * n + 1] = make_double2(ao, dd);
-        row[2 * n] = make_double2(as, ds);
-        hi = lo;
-    }
-    double tc = 0.0 + one_level(2);
-    if (gas) {
-        bool skip = taug < TLIMITI;
-        if ((neg >> 31) || !(fabs(taug - TLIMITI) > 1e-12 * TLIMITI))
-            skip = ir_taugsurf(block, max_nl, LEV, tb) < TLIMITI;
-        if (skip) return s.skip[NSYS_V + j] = 1;
-    }
-    s.skip[NSYS_V + j] = 0;
-    double as1, ds1;
+    // The reference's added 1.D-50 has no effect on a DTAUI above its TINY.
+    const double tiny = R4(1.0E-9);
     {
-        const double *plev = sg.plev + (size_t)c * LEV;
+        const int cc = i / NSYS_I, j = i - cc * NSYS_I, g = col_begin + cc;
+        const SegDev &sg = st->seg[find_seg(st, g)];
+        const ColSmem s = carve_smem(blocks + (size_t)cc * stride, max_nl, nullptr, false);
+        const int nb = j / D_NG;   // 0-based band
+        const int NL = sg.L + 1, LEV = 2 * NL + 1, ng = j - nb * D_NG;
+        const bool gas = ng < D_NG - 1;
+        if (gas && K.fzeroi[nb] >= R4(0.99)) return s.skip[NSYS_V + j] = 2;
+        const double *tb = ki + (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
+        flags = (*s.odd >> (D_NV + nb)) & 1;
+        double taug;
+        double dt1 = 0.0;
+        // pass C of one layer
+        auto coef = [&](const IrLayer &r, double dtsum) {
+            const bool thick = dtsum > tiny;
+            const double dt = thick ? dtsum : tiny, ydt = rcp_n(dt);
+            const double w0 = thick ? quot(r.wnum, dt, ydt) : 0.0;
+            if (hi32(dt) >= 0x46300000u || hi32(w0) >= 0x3ff00000u) flags |= 1;   // DTAUI < 2^100, 0 <= WBARI < 1
+            dt1 = dt;
+            Lay y;
+            double lam, term;
+            lay3(r.cosb, w0, lam, y.gama, term);
+            const double b1 = quot(r.pdif, dt, ydt), b0 = r.b0;
+            const double bt = b1 * term, bb = b0 + b1 * dt;
+            y.cp = bb + bt;
+            y.cm = bb - bt;
+            y.cpm1 = b0 + bt;
+            y.cmm1 = b0 - bt;
+            exp_terms(y, lam * dt);
+            return y;
+        };
+        const IrLayer *r = s.lay_i + NL * D_NI + nb;
+        double2 e = r->ext[0];
+        double tg = gas ? taugas_at(s, LEV, tb) : 0.0;
+        taug = tg;
+        flags |= hi32(tg) & 0x80000000u;
+        double da = gas ? tg + e.x + e.y : e.x + e.y;
+        w.ir[NL].pair = make_double2(da, 0.0);
+        Lay hi = coef(*r, da);
+        double as, ds;
+        bottom_row_v(hi, s.bsurf_i[nb], sg.albi[cc + col_begin - sg.col0], as, ds);
+        w.ir[NL].even = make_double2(as, ds);
+#pragma unroll 1
+        for (int n = NL - 1; n >= 1; --n) {
+            r -= D_NI;
+            const double2 e1 = r->ext[0], e2 = r->ext[1];
+            double db;
+            if (gas) {
+                double t1, t2;
+                taugas_layer<false>(s, 2 * n + 1, tb, t1, t2);
+                taug += t2;
+                taug += t1;
+                flags |= (hi32(t1) | hi32(t2)) & 0x80000000u;
+                da = t1 + e1.x + e1.y;
+                db = t2 + e2.x + e2.y;
+            } else {
+                da = e1.x + e1.y;
+                db = e2.x + e2.y;
+            }
+            w.ir[n].pair = make_double2(da, db);
+            if (n > 1) {
+                prefetch_l1(r - D_NI);
+                prefetch_l1(s.klev + 2 * n - 1);
+            }
+            const Lay lo = coef(*r, da + db);
+            double ao, dd;
+            bool odd = false;
+            fast_rows(lo, hi, as, ds, ao, dd, odd);
+            if (odd) flags |= 1;
+            w.ir[n + 1].odd = make_double2(ao, dd);
+            w.ir[n].even = make_double2(as, ds);
+            hi = lo;
+        }
+        r -= D_NI;
+        e = r->ext[1];
+        tg = gas ? taugas_at(s, 2, tb) : 0.0;
+        taug += tg;
+        flags |= hi32(tg) & 0x80000000u;
+        tc = 0.0 + (gas ? tg + e.x + e.y : e.x + e.y);
+        if (gas) {
+            bool skip = taug < TLIMITI;
+            if ((flags >> 31) || !(fabs(taug - TLIMITI) > 1e-12 * TLIMITI))
+                skip = ir_taugsurf(blocks + (size_t)cc * stride, max_nl, LEV, tb) < TLIMITI;
+            if (skip) return s.skip[NSYS_V + j] = 1;
+        }
+        s.skip[NSYS_V + j] = 0;
+        const double *plev = sg.plev + (size_t)(cc + col_begin - sg.col0) * LEV;
         const double tautop = dt1 * plev[2 - 1] / (plev[4 - 1] - plev[2 - 1]);
         const double btop = (1.0 - mgcm_rt_exp(-tautop / UBARI)) * s.pltop_i[nb];
         const double cf = hi.gama - 1.0, den = hi.gama + 1.0 - cf * as;
-        odd |= out_of_range(den);
+        if (out_of_range(den)) flags |= 1;
         const double x = rcp_s(den);
         as1 = 0.0 * x;
         ds1 = (btop - hi.cmm1 - cf * ds) * x;
     }
-    if (odd) {
-        general_ir(sg, c, j, block, max_nl, K, ki, w.g, fmp, fmm, sc0);
+    // pass D; what it needs of the column is found again rather than held in
+    // registers through pass C
+    asm volatile("" : "+r"(i));
+    const int cc = i / NSYS_I, nb = (i - cc * NSYS_I) / D_NG;
+    const SegDev &sg = st->seg[find_seg(st, col_begin + cc)];
+    const int NL = sg.L + 1;
+    unsigned char *block = blocks + (size_t)cc * stride;
+    double *fmp = fl + row_base(i, max_nl), *fmm = fmp + (size_t)max_nl * ROW_BLK, *sc0 = sc + sc_base(i);
+    if (flags & 1) {
+        general_ir(sg, col_begin + cc - sg.col0, i - cc * NSYS_I, block, max_nl, K, ki, w.g, fmp, fmm, sc0);
         return 0;
     }
-    // pass D
+    const IrLayer *r = carve_smem(block, max_nl, nullptr, false).lay_i + nb;
     double xprev = 0.0;
-    double2 n1 = make_double2(as1, ds1), n2 = row[2], np = pair[1];
-    double nw = w0s[1];
+    double2 n1 = make_double2(as1, ds1), n2 = w.ir[1].even, np = w.ir[1].pair;
+#pragma unroll 1
     for (int n = 1; n <= NL; ++n) {
         const double2 r1 = n1, r2 = n2, p = np;
-        const double w0 = nw;
         if (n < NL) {
-            n1 = row[2 * n + 1];
-            n2 = row[2 * n + 2];
-            np = pair[n + 1];
-            nw = w0s[n + 1];
+            n1 = w.ir[n + 1].odd;
+            n2 = w.ir[n + 1].even;
+            np = w.ir[n + 1].pair;
         }
-        const IrLayer r = lay[n * D_NI];
+        r += D_NI;
+        if (n < NL) prefetch_l1(r + D_NI);
         const double tcA = tc + p.x;
-        bool thick;
-        double ydt;
-        const double dt = depth(n < NL ? p.x + p.y : p.x, thick, ydt);
+        const double dtsum = n < NL ? p.x + p.y : p.x;
+        const bool thick = dtsum > tiny;
+        const double dt = thick ? dtsum : tiny, ydt = rcp_n(dt);
+        const double w0 = thick ? quot(r->wnum, dt, ydt) : 0.0;
         const double dtk = n < NL ? tcA - tc : dt;
         tc = tcA + p.y;
         double lam, gama, term;
-        lay3(r, w0, lam, gama, term);
-        const double b1 = quot(r.pdif, dt, ydt);
+        lay3(r->cosb, w0, lam, gama, term);
+        const double b1 = quot(r->pdif, dt, ydt), b0 = r->b0;
         const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
         const double xb = r2.y - r2.x * xa;
         xprev = xb;
         double xk1, xk2;
         unmix(xa, xb, xk1, xk2);
         const double ep = exp_r(dmin(lam * dtk, TAUMAX)), em = rcp_n(ep);
-        const double bt = b1 * term, bb = r.b0 + b1 * dtk;
+        const double bt = b1 * term, bb = b0 + b1 * dtk;
         const double u = xk1 * ep, v = gama * xk2 * em;
         const double p1 = u + v + (bb + bt);
         const double m1 = u * gama + xk2 * em + (bb - bt);
-        fmp[(size_t)(n - 1) * ROW_BLK] = p1 * PI_D;
-        fmm[(size_t)(n - 1) * ROW_BLK] = m1 * PI_D;
+        *fmp = p1 * PI_D;
+        *fmm = m1 * PI_D;
+        fmp += ROW_BLK;
+        fmm += ROW_BLK;
         if (n == 1) {
-            const double fup = xk1 + gama * xk2 + (r.b0 + bt);
-            const double fdn = xk1 * gama + xk2 + (r.b0 - bt);
+            const double fup = xk1 + gama * xk2 + (b0 + bt);
+            const double fdn = xk1 * gama + xk2 + (b0 - bt);
             *sc0 = (fup - fdn) * PI_D;
         }
     }
@@ -327,23 +351,26 @@ struct VisPassA {
         const int nb = t / D_NG, ng = t - nb * D_NG;
         const bool gas = ng < D_NG - 1;
         const size_t to = (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
-        const double *tb = kv + to, *ray = s.trayaer + nb;
+        const double *tb = kv + to;
         const float *tbf = F32 ? kvf + to : nullptr;
         const VisLayer *lay = s.lay_v + nb;
-        auto dtauk = [&](int k) -> double {
-            if (gas) {
-                const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
-                taugsurf += tg;
-                return tg + ray[k * D_NV];
-            }
-            return ray[k * D_NV];
+        auto level = [&](int k, double ray) -> double {
+            if (!gas) return ray;
+            const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
+            taugsurf += tg;
+            return tg + ray;
         };
-        double2 *pair = w.pair(), *depth = w.depth();
         odd = (*s.odd >> nb) & 1;
-        const double tc2 = 0.0 + dtauk(2);
+        const double tc2 = 0.0 + level(2, lay->ray[1]);
         double tc = tc2, fprev = 0.0;
+#pragma unroll 1
         for (int l = 1; l <= NL; ++l) {
             const int k = 2 * l + 1;
+            lay += D_NV;
+            if (true && l < NL) {
+                prefetch_l1(lay + D_NV);
+                prefetch_l1(s.klev + k + 2);
+            }
             double da, dt, tcA, tcB;
             if (l <= L) {
                 double db;
@@ -358,22 +385,22 @@ struct VisPassA {
                     }
                     taugsurf += da;
                     taugsurf += db;
-                    da = da + ray[k * D_NV];
-                    db = db + ray[(k + 1) * D_NV];
+                    da = da + lay->ray[0];
+                    db = db + lay->ray[1];
                 } else {
-                    da = ray[k * D_NV];
-                    db = ray[(k + 1) * D_NV];
+                    da = lay->ray[0];
+                    db = lay->ray[1];
                 }
                 tcA = tc + da;
                 tcB = tcA + db;
                 dt = da + db;
             } else {
-                dt = da = dtauk(k);
+                dt = da = level(k, lay->ray[0]);
                 tcA = tcB = tc + da;
             }
-            const VisLayer r = lay[l * D_NV];
-            const double wb = quot(r.wnum, dt, rcp_n(dt));
-            const double f = 1.0 - wb * (r.cosb * r.cosb);
+            const double cosb = lay->cosb;
+            const double wb = quot(lay->wnum, dt, rcp_n(dt));
+            const double f = 1.0 - wb * (cosb * cosb);
             odd |= hi32(dt) - 0x2d300000u >= 0x19000000u || hi32(wb) >= 0x3ff00000u;   // [2^-300, 2^100), [0, 1)
             const double dtl = dt * f;
             if (KEEP) {
@@ -384,8 +411,8 @@ struct VisPassA {
                 } else if (l < NL) {
                     m = tau + (tcA - tc) * fprev;
                 }
-                pair[l] = make_double2(quot(wb * (1.0 - r.cosb * r.cosb), f, rcp_n(f)), dtl);
-                depth[l] = make_double2(tau, m);
+                w.vis[l].pair = make_double2(quot(wb * (1.0 - cosb * cosb), f, rcp_n(f)), dtl);
+                w.vis[l].depth = make_double2(tau, m);
             }
             tau = tau + dtl;
             fprev = f;
@@ -436,8 +463,7 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
     // u0 in [2^-30, 2^30), the band's sun 0 or in [2^-60, 2^60)
     bool odd = a.odd || hi32(u0) - 0x3e100000u >= 0x03c00000u || (f0pi != 0.0 && hi32(f0pi) - 0x3c300000u >= 0x07800000u);
     if (!odd) {
-        double2 *pair = w.pair(), *depth = w.depth(), *src = w.src(), *row = w.row();
-        const double *cbs = s.cbs_v + nb;
+        const VisLayer *lay = s.lay_v + NL * D_NV + nb;
         const double rcp_u0 = rcp_n(u0), rcp_u02 = 1.0 / (u0 * u0);
         const double s3 = (double)sqrtf(3.0f), s3h = (double)(sqrtf(3.0f) * 0.5f);
         const double bsurf = rsf * u0 * f0pi * beam(a.tau, u0, rcp_u0);
@@ -458,8 +484,8 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
             const double rd = rcp_s(denom);
             const double am = quot(f0pi * w0 * (g4 * (g1 + rcp_u0) + g2 * g3), denom, rd);
             const double ap = quot(f0pi * w0 * (g3 * (g1 - rcp_u0) + g2 * g4), denom, rd);
-            pair[l] = make_double2(lam, y.gama);
-            src[l] = make_double2(am, ap);
+            w.vis[l].pair = make_double2(lam, y.gama);
+            w.vis[l].src = make_double2(am, ap);
             y.cpm1 = ap * et_top;
             y.cmm1 = am * et_top;
             y.cp = ap * et_bot;
@@ -467,48 +493,52 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
             exp_terms(y, lam * p.y);
             return y;
         };
-        double et_bot = beam(a.tau, u0, rcp_u0), et_top = beam(depth[NL].x, u0, rcp_u0);
-        Lay hi = coef(NL, pair[NL], cbs[NL * D_NV], et_top, et_bot);
+        double et_bot = beam(a.tau, u0, rcp_u0), et_top = beam(w.vis[NL].depth.x, u0, rcp_u0);
+        Lay hi = coef(NL, w.vis[NL].pair, lay->cbs, et_top, et_bot);
         double as, ds;
         bottom_row_v(hi, bsurf, rsf, as, ds);
-        row[2 * NL] = make_double2(as, ds);
-        double2 nxt = pair[NL - 1];
-        double nd = depth[NL - 1].x;
+        w.vis[NL].even = make_double2(as, ds);
+        double2 nxt = w.vis[NL - 1].pair;
+        double nd = w.vis[NL - 1].depth.x;
+#pragma unroll 1
         for (int n = NL - 1; n >= 1; --n) {
             const double2 cur = nxt;
             const double d = nd;
             if (n > 1) {
-                nxt = pair[n - 1];
-                nd = depth[n - 1].x;
+                nxt = w.vis[n - 1].pair;
+                nd = w.vis[n - 1].depth.x;
             }
             et_bot = et_top;
             et_top = beam(d, u0, rcp_u0);
-            const Lay lo = coef(n, cur, cbs[n * D_NV], et_top, et_bot);
+            lay -= D_NV;
+            if (n > 1) prefetch_l1(&lay[-D_NV].cbs);
+            const Lay lo = coef(n, cur, lay->cbs, et_top, et_bot);
             double ao, dd;
             fast_rows(lo, hi, as, ds, ao, dd, odd);
-            row[2 * n + 1] = make_double2(ao, dd);
-            row[2 * n] = make_double2(as, ds);
+            w.vis[n + 1].odd = make_double2(ao, dd);
+            w.vis[n].even = make_double2(as, ds);
             hi = lo;
         }
         {
             const double cf = hi.gama - 1.0, den = hi.gama + 1.0 - cf * as;
             odd |= out_of_range(den);
             const double x = rcp_s(den);
-            row[1] = make_double2(0.0 * x, (0.0 - hi.cmm1 - cf * ds) * x);
+            w.vis[1].odd = make_double2(0.0 * x, (0.0 - hi.cmm1 - cf * ds) * x);
         }
         if (!odd) {
             // pass D
             double xprev = 0.0;
-            double2 n1 = row[1], n2 = row[2], nl = pair[1], ns = src[1], nt = depth[1];
+            double2 n1 = w.vis[1].odd, n2 = w.vis[1].even, nl = w.vis[1].pair, ns = w.vis[1].src, nt = w.vis[1].depth;
+#pragma unroll 1
             for (int n = 1; n <= NL; ++n) {
                 const double2 r1 = n1, r2 = n2, t2 = nt;
                 const double lam = nl.x, gama = nl.y, am = ns.x, ap = ns.y;
                 if (n < NL) {
-                    n1 = row[2 * n + 1];
-                    n2 = row[2 * n + 2];
-                    nl = pair[n + 1];
-                    ns = src[n + 1];
-                    nt = depth[n + 1];
+                    n1 = w.vis[n + 1].odd;
+                    n2 = w.vis[n + 1].even;
+                    nl = w.vis[n + 1].pair;
+                    ns = w.vis[n + 1].src;
+                    nt = w.vis[n + 1].depth;
                 }
                 const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
                 const double xb = r2.y - r2.x * xa;

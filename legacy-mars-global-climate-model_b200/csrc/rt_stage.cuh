@@ -179,7 +179,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 tr = tr0 * s.dpr[k];
                 const double taeros = s.tref_v[k] * qx[(k - 1) * ks];
                 const double tcloud = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
-                s.trayaer[k * D_NV + nw - 1] = tr + taeros + tcloud;
+                s.ray(k, nw) = tr + taeros + tcloud;
                 tl = s.tref_v[k] * qs[(k - 1) * ks];
                 tc = s.tref_c[k] * (cld ? qsc[k - 1] : 0.0);
                 g1 = gv[(k - 1) * ks];
@@ -198,7 +198,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 lvl(k + 1, trb, tlb, tcb, gb, gcb);
                 const double cb = (ga * tla + gb * tlb + gca * tca + gcb * tcb) / (tra + trb + tla + tlb + tca + tcb);
                 s.lay_v[l * D_NV + nw - 1].cosb = cb;
-                s.cbs_v[l * D_NV + nw - 1] = cb / (1.0 + cb);   // code/getdetau.f90:29-56
+                s.lay_v[l * D_NV + nw - 1].cbs = cb / (1.0 + cb);   // code/getdetau.f90:29-56
                 const double wn = tla + tlb + tca + tcb + (tra + trb) * R4(0.9999);
                 s.lay_v[l * D_NV + nw - 1].wnum = wn;
                 usual = usual_layer(cb, wn);
@@ -207,7 +207,7 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
                 lvl(k, tra, tla, tca, ga, gca);
                 const double cb = (ga * tla + gca * tca) / (tra + tla + tca);
                 s.lay_v[l * D_NV + nw - 1].cosb = cb;
-                s.cbs_v[l * D_NV + nw - 1] = cb / (1.0 + cb);
+                s.lay_v[l * D_NV + nw - 1].cbs = cb / (1.0 + cb);
                 const double wn = tla + tca + tra * R4(0.9999);
                 s.lay_v[l * D_NV + nw - 1].wnum = wn;
                 usual = usual_layer(cb, wn);
@@ -228,8 +228,8 @@ __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
             const double *qsc = cld ? sg.qsicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
             const double *gc = cld ? sg.gicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
             auto ext = [&](int k) {   // TAEROS, TCLOUD at level k <= LEV
-                s.ext_i[k * D_NI + nw - 1].x = s.tref_i[k] * qx[(k - 1) * ks];
-                s.ext_i[k * D_NI + nw - 1].y = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
+                s.ext(k, nw).x = s.tref_i[k] * qx[(k - 1) * ks];
+                s.ext(k, nw).y = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
             };
             auto check = [&](int i) {
                 if (V) {
