@@ -75,17 +75,11 @@ __global__ void rt_mixed_solve_vis(const SegTable *__restrict__ st, int col_begi
                                    const __grid_constant__ RtConst K, const int *__restrict__ list,
                                    const unsigned int *count, double *__restrict__ fl,
                                    double *__restrict__ sc);
-template <bool ONE_LEVEL, int RB>
-__global__ void rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end,
-                               int max_nl, unsigned char *__restrict__ blocks, size_t stride,
-                               const RtConst K, const double *__restrict__ fl_v,
-                               const double *__restrict__ sc_v, const double *__restrict__ fl_i,
-                               const double *__restrict__ sc_i, int dense_ir);
-size_t reduce_smem_bytes(int max_nl, int rb);
-const void *reduce_kernel(int max_nl, int rb);
-constexpr int REDUCE_WARPS = 4, REDUCE_THREADS = 32 * REDUCE_WARPS;   // rt_fp64_reduce: warp per column
+size_t reduce_smem_bytes(int max_nl);
+const void *reduce_kernel(int rb);
+constexpr int REDUCE_THREADS = 32;   // rt_fp64_reduce: a warp, and CTA, per column
 constexpr int STAGE_THREADS = 256, SCREEN_THREADS = 128;
-int reduce_rows_per_chunk(int max_nl);
+int reduce_rows_per_chunk();
 __global__ void rt_dsolflux_kernel(int ncol, const double *__restrict__ sol,
                                    const double *__restrict__ acosz,
                                    const double *__restrict__ detau,
@@ -282,7 +276,7 @@ struct Job {
 struct Tune {
     int chunk = 0;        // columns per pipeline pass
     int solve_ctas = 0;   // solver CTAs per SM
-    int rb = 0;           // reduce: kept-system rows per TMA chunk
+    int rb = 0;           // reduce: systems read before they are summed
     int fused = -1;       // fused kernel: index into FUSED_SHAPES (-1: the default shape)
 };
 
@@ -565,10 +559,8 @@ int configure_kernels(int device) {
     std::lock_guard<std::mutex> lk(mu);
     if (device < 0 || device >= 256) return MGCM_RT_EINVAL;
     if (done[device]) return MGCM_RT_OK;
-    for (int nl : {32, 33})
-        for (int rb : {1, 2, 4, 8})
-            CK(cudaFuncSetAttribute(reduce_kernel(nl, rb), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SMEM_CAP));
+    for (int rb : {1, 2, 4, 8})
+        CK(cudaFuncSetAttribute(reduce_kernel(rb), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP));
     CK(cudaFuncSetAttribute(rt_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP));
     for (int f = 0; f < 3; ++f)
         for (int q = 0; q < OC_NT; ++q)
@@ -627,8 +619,8 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
     double *sc_v = reinterpret_cast<double *>(take(r_v * 32));
     double *sc_i = reinterpret_cast<double *>(take(r_i * 32));
     unsigned int *counts = reinterpret_cast<unsigned int *>(take(256));
-    const int rb = sl.tune.rb > 0 ? sl.tune.rb : reduce_rows_per_chunk(max_nl);
-    const size_t rsm = reduce_smem_bytes(max_nl, rb);
+    const int rb = sl.tune.rb > 0 ? sl.tune.rb : reduce_rows_per_chunk();
+    const size_t rsm = reduce_smem_bytes(max_nl);
     const bool mixed = h->cfg.precision == MGCM_RT_MIXED;
     if (sl.occ_nl != max_nl || sl.occ_rb != rb) {
         sl.occ_nl = max_nl;
@@ -647,7 +639,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         else if (qr == 10) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qo, rt_quad_solve<false, 10>, 128, 0);
         else if (qr == 13) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qo, rt_quad_solve<false, 13>, 128, 0);
         sl.occ_quad = std::max(qo, 1);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, reduce_kernel(max_nl, rb), REDUCE_THREADS, rsm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, reduce_kernel(rb), REDUCE_THREADS, rsm);
         sl.occ_screen = std::max(a, 1);
         sl.occ_solve = std::max(b, 1);
         sl.occ_reduce = std::max(c, 1);
@@ -738,14 +730,14 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         CK(cudaGetLastError());
         CK(cudaEventRecord(sl.join_ev, sl.aux));
         CK(cudaStreamWaitEvent(st, sl.join_ev, 0));
-        const int g3 = std::min((c1 - c0 + REDUCE_WARPS - 1) / REDUCE_WARPS, h->num_sms * sl.occ_reduce);
+        const int g3 = std::min(c1 - c0, h->num_sms * sl.occ_reduce);
         {
             const SegTable *segs = sl.d_segs;
             const RtConst &K = h->K;
             void *args[] = {(void *)&segs, (void *)&c0, (void *)&c1, (void *)&max_nl, (void *)&blocks,
                             (void *)&stride, (void *)&K, (void *)&fl_v, (void *)&sc_v, (void *)&fl_i,
                             (void *)&sc_i, (void *)&dense_ir};
-            CK(cudaLaunchKernel(reduce_kernel(max_nl, rb), dim3(g3), dim3(REDUCE_THREADS), args, rsm, st));
+            CK(cudaLaunchKernel(reduce_kernel(rb), dim3(g3), dim3(REDUCE_THREADS), args, rsm, st));
         }
         nk += 5;
         CK(cudaGetLastError());
@@ -2157,8 +2149,7 @@ int mgcm_rt_graph_create(mgcm_rt_handle *h, int nbatch, const mgcm_rt_batch_in *
             if ((rc = consider(t))) return fail(rc);
         }
         for (int r : {1, 2, 4, 8}) {
-            if (reduce_smem_bytes(max_nl, r) > SMEM_CAP) continue;
-            if (r == reduce_rows_per_chunk(max_nl)) continue;
+            if (r == reduce_rows_per_chunk()) continue;
             Tune t = best;
             t.rb = r;
             if ((rc = consider(t))) return fail(rc);
@@ -2208,7 +2199,7 @@ int mgcm_rt_graph_create(mgcm_rt_handle *h, int nbatch, const mgcm_rt_batch_in *
     mgcm_rt_tune &inf = g->info;
     inf.chunk_cols = best.chunk > 0 ? std::min(best.chunk, g->max_chunk) : std::min(total, g->max_chunk);
     inf.solve_ctas_per_sm = best.solve_ctas;
-    inf.reduce_rows = best.rb > 0 ? best.rb : reduce_rows_per_chunk(max_nl);
+    inf.reduce_rows = best.rb > 0 ? best.rb : reduce_rows_per_chunk();
     inf.candidates = ncand;
     inf.tuning_cols = sample;
     inf.default_ms = t_def;

@@ -282,180 +282,213 @@ template __global__ void rt_quad_solve<false, 13>(QUAD_ARGS);
 // flux rows in blocks of 32 list positions (row_base, sc_base): value k of
 // the system at position p is fl[row_base(p) + 32 k] (k < max_nl: upward
 // midpoint flux of layer k+1; max_nl + k: downward), scalar q
-// sc[sc_base(p) + 32 q].  A column's kept systems sit in one run of
-// positions per screening group, in ascending (band, Gauss) order.  Lane j
-// owns levels j+1, j+33, ... and sums its outputs over the systems in the
-// reference order, each scaled by the multipliers of family_multipliers; the
-// loads of RB systems are issued before they are summed.
-constexpr int RED_WARPS = 4;
-constexpr int RED_LPL = (D_MAXNL + 1 + 31) / 32;   // levels per lane
+// sc[sc_base(p) + 32 q].  A column's kept systems sit in ascending (band,
+// Gauss) order, in one run of positions per screening group (visible) or at
+// 85 positions a column (rt_ir_dense).
+//
+// The rows of up to 16 systems at a time come into shared memory with
+// asynchronous copies, half a warp along the systems for the upward and half
+// for the downward fluxes (a value of 16 consecutive positions is one
+// 128-byte segment), at a pitch of 17; then a lane per
+// level sums its outputs over the systems in the reference order, reading
+// the buffer without bank conflicts.  8,192 x 24 columns: 255 -> 191 us against
+// loading the rows lane by level straight from global memory, 32 cache lines
+// a value, which ran at 76% of the L1's tag rate; what bounds it now is the
+// latency of its short phases at 17 warps per SM (issue 30%, DRAM 29%).  32
+// systems at a time: the same at 24 layers, 1.5% slower calls at 48.
+constexpr int RED_LPL = (D_MAXNL + 2 + 31) / 32;   // items (levels and two scalar sums) per lane
+constexpr int RED_SYS = 16, RED_PITCH = RED_SYS + 1;   // systems staged at a time
 
-// Shared memory of one warp: the multipliers of both families, FMNET per
-// level of both families, the top-of-atmosphere values, and one family's
-// kept list positions in order.
-__host__ __device__ inline size_t red_warp_bytes() {
-    size_t b = (size_t)3 * NSYS * 8;                  // multipliers
-    b += (size_t)2 * (D_MAXNL + 2) * 8 + 4 * 8;       // FMNET per level, top values
-    b += (size_t)NSYS * 4;                            // list positions
-    return (b + 127) / 128 * 128;
+// A kept system: its multipliers m1, m2, m3 as family_multipliers gives them,
+// its list position, and which factors are not exactly 1.0 (bit 0: m2, bit 1: m3).
+struct alignas(16) RedSys {
+    double a, b, e;
+    int pos, fac;
+};
+
+// Shared memory of one warp (= CTA): one family's kept systems, FMNET per
+// level of both families and the two factors of the heating rate, the top
+// values, and the staged rows: NL + 2 items, upward and downward.
+__host__ __device__ inline size_t red_fixed_bytes(int max_nl) {
+    const size_t b = (size_t)NSYS_V * sizeof(RedSys) + (size_t)(4 * (max_nl + 1) + 2) * 8;
+    return (b + 15) / 16 * 16;
+}
+__host__ __device__ inline size_t red_warp_bytes(int max_nl) {
+    return red_fixed_bytes(max_nl) + (size_t)2 * (max_nl + 2) * RED_PITCH * 8;
 }
 
-// Multipliers of both families for one column, one lane per band (visible
-// bands on lanes 0-6, IR bands on lanes 8-12); each lane walks its band as
-// family_multipliers does, at the band's offset among the kept rows.
-__device__ inline void warp_multipliers(const unsigned char *skip, bool day, const RtConst &K,
-                                        double *m1, double *m2, double *m3) {
+// Multipliers of one family of a column, one lane per band: `mine` holds, on
+// lane w, the kept flags of systems 32w .. 32w+31 of the family.  Each lane
+// walks its band as family_multipliers does, at the band's offset among the
+// kept rows.
+__device__ inline void warp_multipliers(unsigned mine, bool vis, const RtConst &K, RedSys *sys) {
     const int lane = threadIdx.x & 31;
-    const bool isv = lane < D_NV && day, isi = lane >= 8 && lane < 8 + D_NI;
-    const int nw = isv ? lane + 1 : (isi ? lane - 7 : 0);
-    const int base = isv ? 0 : NSYS_V;
-    const double fz = isv ? K.fzerov[nw - 1] : (isi ? K.fzeroi[nw - 1] : 0.0);
-    const unsigned char *sk = skip + base + (nw > 0 ? nw - 1 : 0) * D_NG;
-    int cnt = 0;
-    if (isv || isi) {
-        if (!(fz >= R4(0.99)))
-            for (int ng = 1; ng <= D_NG - 1; ++ng) cnt += sk[ng - 1] == 0;
-        cnt += 1;
+    const bool on = lane < (vis ? D_NV : D_NI);
+    const double fz = on ? (vis ? K.fzerov[lane] : K.fzeroi[lane]) : 0.0;
+    const int first = (on ? lane : 0) * D_NG, w = first >> 5;
+    const unsigned lo = __shfl_sync(0xffffffffu, mine, w), hi = __shfl_sync(0xffffffffu, mine, w + 1);
+    const unsigned bits = __funnelshift_r(lo, hi, first & 31) & 0xffffu;   // points 1..16
+    const bool gas = !(fz >= R4(0.99));
+    const int cnt = on ? (gas ? __popc(bits) : 0) + 1 : 0;
+    int pos = cnt;   // exclusive prefix over the bands
+    for (int o = 1; o < 8; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, pos, o);
+        if (lane >= o) pos += v;
     }
-    // exclusive prefix over the lanes of the same family
-    const int first = isv ? 0 : 8;
-    int pos = 0;
-    for (int k = 1; k < 8; ++k) {
-        const int v = __shfl_up_sync(0xffffffffu, cnt, k);
-        if (lane - k >= first) pos += v;
-    }
-    if (!(isv || isi)) return;
-    double *p1 = m1 + base, *p2 = m2 + base, *p3 = m3 + base;
+    pos -= cnt;
+    if (!on) return;
     double fzero = fz;
-    const double dw = isv ? 1.0 : K.dwni[nw - 1];
-    if (!(fz >= R4(0.99))) {
-        for (int ng = 1; ng <= D_NG - 1; ++ng) {
-            if (sk[ng - 1] != 0) {
-                fzero = fzero + (1.0 - fz) * K.gweight[ng - 1];
-                continue;
-            }
-            if (isv) {
-                p1[pos] = K.gweight[ng - 1];
-                p2[pos] = 1.0 - fz;
-                p3[pos] = 1.0;
-            } else {
-                p1[pos] = dw;
-                p2[pos] = K.gweight[ng - 1];
-                p3[pos] = 1.0 - fz;
-            }
-            ++pos;
+    const double dw = vis ? 1.0 : K.dwni[lane], one = 1.0 - fz;
+    auto put = [&](double a, double b, double e) {
+        RedSys &r = sys[pos++];
+        r.a = a;
+        r.b = b;
+        r.e = e;
+        r.fac = (b != 1.0 ? 1 : 0) | (e != 1.0 ? 2 : 0);
+    };
+    if (gas) {
+        for (int ng = 0; ng < D_NG - 1; ++ng) {
+            if (!((bits >> ng) & 1u)) fzero = fzero + one * K.gweight[ng];
+            else if (vis) put(K.gweight[ng], one, 1.0);
+            else put(dw, K.gweight[ng], one);
         }
     }
-    if (isv) {
-        p1[pos] = fzero;
-        p2[pos] = 1.0;
-    } else {
-        p1[pos] = dw;
-        p2[pos] = fzero;
-    }
-    p3[pos] = 1.0;
+    if (vis) put(fzero, 1.0, 1.0);
+    else put(dw, fzero, 1.0);
 }
 
-template <bool ONE_LEVEL, int RB>   // ONE_LEVEL: max NL <= 32, one level per lane
-__global__ void __launch_bounds__(32 * RED_WARPS)
+// 8 bytes from global to shared memory, asynchronously.
+__device__ __forceinline__ void copy8_async(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+template <int RB>   // systems whose staged values are read before they are summed
+__global__ void __launch_bounds__(32)
 rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
-               unsigned char *__restrict__ blocks, size_t stride, const RtConst K,
+               unsigned char *__restrict__ blocks, size_t stride, const __grid_constant__ RtConst K,
                const double *__restrict__ fl_v, const double *__restrict__ sc_v,
                const double *__restrict__ fl_i, const double *__restrict__ sc_i, int dense_ir) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    constexpr int LPL = ONE_LEVEL ? 1 : RED_LPL;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned char *ws = smem_raw + (size_t)wid * red_warp_bytes();
-    double *m1 = reinterpret_cast<double *>(ws);
-    double *m2 = m1 + NSYS, *m3 = m2 + NSYS;
-    double *fmv = m3 + NSYS, *fmi = fmv + (D_MAXNL + 2), *misc = fmi + (D_MAXNL + 2);
-    int *rpos = reinterpret_cast<int *>(misc + 4);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x;
+    RedSys *sys = reinterpret_cast<RedSys *>(smem_raw);
+    double *fmv = reinterpret_cast<double *>(sys + NSYS_V), *fmi = fmv + max_nl + 1;   // [1..NL]
+    double *pnl = fmi + max_nl + 1, *den = pnl + max_nl + 1, *misc = den + max_nl + 1;
+    double *buf = reinterpret_cast<double *>(smem_raw + red_fixed_bytes(max_nl));
 
-    for (int g = col_begin + blockIdx.x * RED_WARPS + wid; g < col_end; g += gridDim.x * RED_WARPS) {
-        const int si = find_seg(st, g);
-        const SegDev &sg = st->seg[si];
+    for (int g = col_begin + blockIdx.x; g < col_end; g += gridDim.x) {
+        const SegDev &sg = st->seg[find_seg(st, g)];
         const int c = g - sg.col0;
-        const int NL = sg.L + 1;
+        const int NL = sg.L + 1, LEV = 2 * NL + 1, R = NL + 2;   // staged items: the levels, FLUXUP/FLUXDN at the top, DIFFV
         const ColSmem s = carve_smem(blocks + (size_t)(g - col_begin) * stride, max_nl, nullptr, false);
         const bool day = sg.acosz[c] >= R4(1.0e-5);
-        warp_multipliers(s.skip, day, K, m1, m2, m3);
+        // kept flags of both families: lane w holds those of systems 32w .. 32w+31
+        unsigned mine_v = 0, mine_i = 0;
+        {
+            unsigned char f[7];
+#pragma unroll
+            for (int w = 0; w < 7; ++w) {
+                const int t = w < 4 ? 32 * w + lane : NSYS_V + 32 * (w - 4) + lane;
+                f[w] = t < (w < 4 ? NSYS_V : NSYS) ? s.skip[t] : 1;
+            }
+#pragma unroll
+            for (int w = 0; w < 7; ++w) {
+                const unsigned m = __ballot_sync(0xffffffffu, f[w] == 0);
+                if (w < 4 && lane == w) mine_v = m;
+                if (w >= 4 && lane == w - 4) mine_i = m;
+            }
+        }
+        if (!day) mine_v = 0;
+        const int gbase = lane < SCREEN_GROUPS ? s.meta[2 * lane] : 0;   // list positions of the groups
+        // what the heating rates need besides the fluxes (code/comp3.f:765-771)
+        const double *plev = sg.plev + (size_t)c * LEV;
+        for (int l = 1 + lane; l <= NL; l += 32) {
+            const int k = 2 * l;
+            const double ptrop = sg.ptrop;
+            const double ym = k == 2 ? ptrop * 100.0 / 3.72 : (plev[k + 1 - 1] - plev[k - 1 - 1]) * 100.0 / 3.72;
+            const double om = pow(plev[k - 1] / plev[LEV - 1], 0.25684);
+            pnl[l] = sg.sigma[k - 1] * (sg.pcol[c] - ptrop) + ptrop;
+            den[l] = 735.94 * ym * om;
+        }
         for (int fam = 0; fam < 2; ++fam) {
             const bool vis = fam == 0;
-            // list positions of the family's kept systems (none at night for
-            // the visible family: its outputs are zeros)
+            const unsigned mine = vis ? mine_v : mine_i;
+            // the family's kept systems in order (none at night for the
+            // visible family: its outputs are zeros)
             int nrow = 0;
-            if (!vis && dense_ir) {   // rt_ir_dense: every system has its position
-                for (int j0 = 0; j0 < NSYS_I; j0 += 32) {
-                    const int j = j0 + lane;
-                    const bool kept = j < NSYS_I && s.skip[NSYS_V + j] == 0;
-                    const unsigned m = __ballot_sync(0xffffffffu, kept);
-                    if (kept) rpos[nrow + __popc(m & ((1u << lane) - 1u))] = (g - col_begin) * NSYS_I + j;
+            if (!vis || day) {
+                for (int w = 0; w < (vis ? 4 : 3); ++w) {
+                    const unsigned m = __shfl_sync(0xffffffffu, mine, w);
+                    const int base = __shfl_sync(0xffffffffu, gbase, vis ? w : 4 + w);
+                    const int before = __popc(m & ((1u << lane) - 1u));
+                    if ((m >> lane) & 1u)
+                        sys[nrow + before].pos = !vis && dense_ir ? (g - col_begin) * NSYS_I + 32 * w + lane : base + before;
                     nrow += __popc(m);
                 }
-            } else if (!vis || day) {
-                const int w0 = vis ? 0 : SCREEN_GROUPS_V, w1 = vis ? SCREEN_GROUPS_V : SCREEN_GROUPS;
-                for (int gw = w0; gw < w1; ++gw) {
-                    const int gb = s.meta[2 * gw], gn = s.meta[2 * gw + 1];
-                    for (int q = lane; q < gn; q += 32) rpos[nrow + q] = gb + q;
-                    nrow += gn;
-                }
+                warp_multipliers(mine, vis, K, sys);
             }
             __syncwarp();
             const double *fl = vis ? fl_v : fl_i, *sc = vis ? sc_v : sc_i;
-            const double *f1 = vis ? m1 : m1 + NSYS_V, *f2 = vis ? m2 : m2 + NSYS_V, *f3 = vis ? m3 : m3 + NSYS_V;
-            double top = 0.0, dif = 0.0;
+            double acc[RED_LPL][3];
+#pragma unroll
+            for (int r = 0; r < RED_LPL; ++r) acc[r][0] = acc[r][1] = acc[r][2] = 0.0;
+            for (int f0 = 0; f0 < nrow; f0 += RED_SYS) {
+                const int n = min(RED_SYS, nrow - f0), q = lane % RED_SYS;
+                const bool down = lane >= RED_SYS;
+                if (q < n) {
+                    const int p = sys[f0 + q].pos;
+                    const double *pr = fl + row_base(p, max_nl) + (down ? (size_t)max_nl * ROW_BLK : 0);
+                    const double *ps = sc + sc_base(p);
+                    double *bw = buf + q + (down ? R * RED_PITCH : 0);
+                    for (int k = 0; k < NL; ++k) copy8_async(bw + k * RED_PITCH, pr + k * ROW_BLK);
+                    // FLUXUP and, visible, FLUXDN at the top; DIFFV
+                    if (!down || vis) copy8_async(bw + NL * RED_PITCH, down ? ps + ROW_BLK : ps);
+                    else bw[NL * RED_PITCH] = 0.0;
+                    if (!down && vis) copy8_async(bw + (NL + 1) * RED_PITCH, ps + 2 * ROW_BLK);
+                    else bw[(NL + 1) * RED_PITCH] = 0.0;
+                }
+                asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < RED_LPL; ++r) {
+                    if (32 * r >= R) break;
+                    const int it = min(lane + 32 * r, R - 1);
+                    const double *bu = buf + it * RED_PITCH, *bd = bu + R * RED_PITCH;
 #pragma unroll 1
-            for (int r = 0; r < LPL; ++r) {
-                if (32 * r >= NL) break;
-                const int l = lane + 1 + 32 * r;
-                const bool lv = l <= NL;
-                const size_t ou = (size_t)(lv ? l - 1 : 0) * ROW_BLK, od = ou + (size_t)max_nl * ROW_BLK;
-                double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-                for (int f0 = 0; f0 < nrow; f0 += RB) {
-                    double up[RB], dn[RB], t0[RB], t1[RB];
+                    for (int q0 = 0; q0 < n; q0 += RB) {
+                        double up[RB], dn[RB];
 #pragma unroll
-                    for (int q = 0; q < RB; ++q) {
-                        up[q] = dn[q] = t0[q] = t1[q] = 0.0;
-                        if (f0 + q < nrow) {
-                            const int p = rpos[f0 + q];
-                            const double *pr = fl + row_base(p, max_nl);
-                            if (lv) {
-                                up[q] = __ldg(pr + ou);
-                                dn[q] = __ldg(pr + od);
-                            }
-                            if (r == 0) {
-                                const double *ps = sc + sc_base(p);
-                                t0[q] = vis ? __ldg(ps) - __ldg(ps + ROW_BLK) : __ldg(ps);
-                                if (vis) t1[q] = __ldg(ps + 2 * ROW_BLK);
-                            }
+                        for (int q = 0; q < RB; ++q) {   // past n: within the buffer's pitch, not summed
+                            up[q] = bu[q0 + q];
+                            dn[q] = bd[q0 + q];
                         }
-                    }
 #pragma unroll
-                    for (int q = 0; q < RB; ++q) {
-                        if (f0 + q < nrow) {
-                            const double a = f1[f0 + q], b = f2[f0 + q], e = f3[f0 + q];
-                            // ((v*a)*b)*e in the reference order; a factor that is
-                            // exactly 1.0 leaves the product unchanged and is
-                            // skipped (warp-uniform)
-                            const bool b1 = b == 1.0, e1 = e == 1.0;
-                            auto wt = [&](double v) {
-                                double x = v * a;
-                                if (!b1) x = x * b;
-                                if (!e1) x = x * e;
-                                return x;
-                            };
-                            a0 = a0 + wt(up[q] - dn[q]);
-                            a1 = a1 + wt(up[q]);
-                            a2 = a2 + wt(dn[q]);
-                            if (r == 0) {
-                                top = top + wt(t0[q]);
-                                if (vis) dif = dif + wt(t1[q]);
+                        for (int q = 0; q < RB; ++q) {
+                            if (q0 + q < n) {
+                                const RedSys y = sys[f0 + q0 + q];
+                                // ((v*a)*b)*e in the reference order; a factor that is
+                                // exactly 1.0 leaves the product unchanged and is
+                                // skipped (warp-uniform)
+                                auto wt = [&](double v) {
+                                    double x = v * y.a;
+                                    if (y.fac & 1) x = x * y.b;
+                                    if (y.fac & 2) x = x * y.e;
+                                    return x;
+                                };
+                                acc[r][0] = acc[r][0] + wt(up[q] - dn[q]);
+                                acc[r][1] = acc[r][1] + wt(up[q]);
+                                acc[r][2] = acc[r][2] + wt(dn[q]);
                             }
                         }
                     }
                 }
-                if (lv) {
-                    const size_t o = (size_t)c * NL + l - 1;
+                __syncwarp();   // the buffer is refilled
+            }
+#pragma unroll
+            for (int r = 0; r < RED_LPL; ++r) {
+                const int it = lane + 32 * r, l = it + 1;
+                const double a0 = acc[r][0], a1 = acc[r][1], a2 = acc[r][2];
+                const size_t o = (size_t)c * NL + it;
+                if (it < NL) {
                     if (vis) {
                         sg.fmnetv[o] = a0;
                         sg.fluxupv[o] = a1;
@@ -472,77 +505,50 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
                         fmi[l] = a0;
                         if (l == NL) sg.dnirflux[c] = a2;
                     }
+                } else if (it == NL) {
+                    (vis ? sg.nfluxtopv : sg.nfluxtopi)[c] = a0;
+                    misc[vis ? 0 : 1] = a0;
+                } else if (it == NL + 1 && vis) {
+                    sg.diffvt[c] = a1;
+                    sg.dndiffv[c] = a1;
                 }
             }
-            if (lane == 0) {
-                if (vis) {
-                    sg.nfluxtopv[c] = top;
-                    sg.diffvt[c] = dif;
-                    sg.dndiffv[c] = dif;
-                    misc[0] = top;
-                } else {
-                    sg.nfluxtopi[c] = top;
-                    misc[1] = top;
-                }
-            }
-            __syncwarp();   // rpos is rewritten by the next family
+            __syncwarp();   // sys is rewritten by the next family
         }
         // divergences and heating rates (code/comp3.f:677-681,735-738,765-771)
-        const double *plev = sg.plev + (size_t)c * (2 * sg.L + 3);
-        const int LEV = 2 * sg.L + 3;
         for (int l = 1 + lane; l <= NL; l += 32) {
             const double sun = day ? (l == 1 ? fmv[1] - misc[0] : fmv[l] - fmv[l - 1]) : 0.0;
             const double irt = l == 1 ? fmi[1] - misc[1] : fmi[l] - fmi[l - 1];
-            const int k = 2 * l;
-            const double ptrop = sg.ptrop, p = sg.pcol[c];
-            const double ym = k == 2 ? ptrop * 100.0 / 3.72 : (plev[k + 1 - 1] - plev[k - 1 - 1]) * 100.0 / 3.72;
-            const double om = pow(plev[k - 1] / plev[LEV - 1], 0.25684);
-            const double pnlte = sg.sigma[k - 1] * (p - ptrop) + ptrop;
-            const double sunlte = sun * 2.2e4 * pnlte / (1.0 + 2.2e4 * pnlte);
+            const double sunlte = sun * 2.2e4 * pnl[l] / (1.0 + 2.2e4 * pnl[l]);
             const size_t o = (size_t)c * NL + l - 1;
             sg.suntot[o] = sun;
             sg.irtotal[o] = irt;
-            sg.qrad[o] = (sunlte + irt) / (735.94 * ym * om);
+            sg.qrad[o] = (sunlte + irt) / den[l];
         }
-        __syncwarp();   // fmv, fmi, misc and the multipliers are rewritten by the next column
+        __syncwarp();   // the shared arrays are rewritten by the next column
     }
 }
 
 #define REDUCE_ARGS                                                                                    \
-    const SegTable *__restrict__, int, int, int, unsigned char *__restrict__, size_t, const RtConst,  \
-        const double *__restrict__, const double *__restrict__, const double *__restrict__,          \
-        const double *__restrict__, int
-#define REDUCE_INST(RB)                                              \
-    template __global__ void rt_fp64_reduce<true, RB>(REDUCE_ARGS);  \
-    template __global__ void rt_fp64_reduce<false, RB>(REDUCE_ARGS);
-REDUCE_INST(1)
-REDUCE_INST(2)
-REDUCE_INST(4)
-REDUCE_INST(8)
-#undef REDUCE_INST
+    const SegTable *__restrict__, int, int, int, unsigned char *__restrict__, size_t,                 \
+        const __grid_constant__ RtConst, const double *__restrict__, const double *__restrict__,      \
+        const double *__restrict__, const double *__restrict__, int
+template __global__ void rt_fp64_reduce<1>(REDUCE_ARGS);
+template __global__ void rt_fp64_reduce<2>(REDUCE_ARGS);
+template __global__ void rt_fp64_reduce<4>(REDUCE_ARGS);
+template __global__ void rt_fp64_reduce<8>(REDUCE_ARGS);
 #undef REDUCE_ARGS
 
-// Shared memory of rt_fp64_reduce (the same for every batch size).
-size_t reduce_smem_bytes(int max_nl, int rb) {
-    (void)max_nl;
-    (void)rb;
-    return (size_t)RED_WARPS * red_warp_bytes();
-}
-// Systems whose loads the reduce issues before it sums them, by default
-// (measured on the 64,800-column call: 4 -> 8 saves 0.07 ms; 16 needs 182
-// registers and is slower).
-int reduce_rows_per_chunk(int max_nl) {
-    (void)max_nl;
-    return 8;
-}
-// The reduce kernel of a launch: one level per lane up to NL = 32, and RB
-// in {1, 2, 4, 8} (other values round down).
-const void *reduce_kernel(int max_nl, int rb) {
-    const bool one = max_nl <= 32;
-    if (rb >= 8) return one ? (const void *)rt_fp64_reduce<true, 8> : (const void *)rt_fp64_reduce<false, 8>;
-    if (rb >= 4) return one ? (const void *)rt_fp64_reduce<true, 4> : (const void *)rt_fp64_reduce<false, 4>;
-    if (rb >= 2) return one ? (const void *)rt_fp64_reduce<true, 2> : (const void *)rt_fp64_reduce<false, 2>;
-    return one ? (const void *)rt_fp64_reduce<true, 1> : (const void *)rt_fp64_reduce<false, 1>;
+// Shared memory of a reduce CTA (one warp).
+size_t reduce_smem_bytes(int max_nl) { return red_warp_bytes(max_nl); }
+// Systems whose staged values a lane reads before it sums them, by default.
+int reduce_rows_per_chunk() { return 4; }
+// The reduce kernel of a launch, rb in {1, 2, 4, 8} (other values round down).
+const void *reduce_kernel(int rb) {
+    if (rb >= 8) return (const void *)rt_fp64_reduce<8>;
+    if (rb >= 4) return (const void *)rt_fp64_reduce<4>;
+    if (rb >= 2) return (const void *)rt_fp64_reduce<2>;
+    return (const void *)rt_fp64_reduce<1>;
 }
 
 // Partial radiation: DIRECTSOL from DETAU (code/dsolflux.f:28-45) and
