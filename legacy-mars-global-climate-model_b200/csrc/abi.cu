@@ -41,7 +41,9 @@ __global__ void rt_fp64_kernel(const SegTable *__restrict__ st, const double *__
 template <bool V>
 __global__ void rt_stage(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                          unsigned char *__restrict__ blocks, size_t stride,
-                         const double *__restrict__ planck, const RtConst K, uint32_t *status);
+                         const double *__restrict__ planck, const __grid_constant__ RtConst K, uint32_t *status,
+                         int cols);
+size_t stage_smem_bytes(int max_nl);
 template <bool F32>
 __global__ void rt_fp64_screen(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                                unsigned char *__restrict__ blocks, size_t stride,
@@ -629,7 +631,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, mixed ? rt_fp64_screen<true> : rt_fp64_screen<false>,
                                                       SCREEN_THREADS, 0);
         int e = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, rt_stage<true>, STAGE_THREADS, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e, rt_stage<true>, STAGE_THREADS, stage_smem_bytes(max_nl));
         sl.occ_stage = std::max(e, 1);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, mixed ? (const void *)rt_mixed_solve_vis : (const void *)rt_fp64_solve_vis,
                                                       128, 0);
@@ -647,9 +649,11 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
     for (int c0 = 0; c0 < total; c0 += chunk) {
         const int c1 = std::min(total, c0 + chunk);
         CK(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned int), st));
-        const int g0 = std::min((c1 - c0 + 3) / 4, h->num_sms * sl.occ_stage);   // 4 columns per CTA
-        (check ? rt_stage<true> : rt_stage<false>)<<<g0, STAGE_THREADS, 0, st>>>(
-            sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_planck, h->K, sl.d_status);
+        // 4 columns per CTA, one where that leaves SMs idle
+        const int sc = (c1 - c0) > 2 * h->num_sms ? 4 : 1;
+        const int g0 = std::min((c1 - c0 + sc - 1) / sc, h->num_sms * sl.occ_stage);
+        (check ? rt_stage<true> : rt_stage<false>)<<<g0, STAGE_THREADS, stage_smem_bytes(max_nl), st>>>(
+            sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_planck, h->K, sl.d_status, sc);
         const int g2 = h->num_sms * (sl.tune.solve_ctas > 0 ? sl.tune.solve_ctas : sl.occ_solve);
         const int qr = h->quad ? quad_r_for(max_nl) : 0;
         const bool oc = h->onchip || h->tmem;
@@ -1859,8 +1863,8 @@ int mgcm_rt_debug_bins(mgcm_rt_handle *h, const mgcm_rt_batch_in *in, int *mt, i
                             cudaMemcpyHostToDevice, st) ||
             cudaMemsetAsync(sl.d_status, 0, 256, st)) { rc = MGCM_RT_ECUDA; break; }
         const int g0 = std::min<int>(((int)z.ncol + 3) / 4, h->num_sms * 4);
-        rt_stage<false><<<g0, STAGE_THREADS, 0, st>>>(sl.d_segs, 0, (int)z.ncol, z.nl, blocks, stride, h->d_planck,
-                                               h->K, sl.d_status);
+        rt_stage<false><<<g0, STAGE_THREADS, stage_smem_bytes(z.nl), st>>>(
+            sl.d_segs, 0, (int)z.ncol, z.nl, blocks, stride, h->d_planck, h->K, sl.d_status, 4);
         const long long items = (long long)z.ncol * z.lev;
         const int g1 = (int)std::min<long long>((items + 255) / 256, (long long)h->num_sms * 8);
         rt_bins_decode<<<g1, 256, 0, st>>>(sl.d_segs, (int)z.ncol, z.nl, blocks, stride, sl.d_status, mt, mp,

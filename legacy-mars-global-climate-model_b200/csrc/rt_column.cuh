@@ -57,9 +57,11 @@ struct ColSmem {
     KLevel *klev;
     double *dpr;
     double *tref_v, *tref_i, *tref_c;   // TAUREF/QEXTREF (vis, IR), TAUREFCLD/QEXTREFCLD
-    // per layer (0..NL) and band
-    IrLayer *lay_i;                     // [l][5]
-    VisLayer *lay_v;                    // [l][7]
+    // per band and layer (0..NL), band-major: a solver thread walks one band's
+    // records, and the stage's lanes, a layer each, write them contiguously
+    IrLayer *lay_i;                     // [5][pitch]
+    VisLayer *lay_v;                    // [7][pitch]
+    int pitch;                          // the launch's largest NL + 1
     double *bsurf_i, *pltop_i;          // [5]
     // reduction staging
     double *fmp, *fmm;                  // [sys][l]
@@ -71,13 +73,12 @@ struct ColSmem {
     double *fmnet_v, *fmnet_i;          // [l] reduced net fluxes for the divergences
     double *misc;                       // [4] NFLUXTOPV, NFLUXTOPI
     int day;
-    // TAEROS, TCLOUD of level k, IR band nw; TRAY+TAEROS+TCLOUD, visible band nw (1-based)
-    __device__ __forceinline__ double2 &ext(int k, int nw) const {
-        return lay_i[((k - 1) >> 1) * D_NI + nw - 1].ext[(k - 1) & 1];
-    }
-    __device__ __forceinline__ double &ray(int k, int nw) const {
-        return lay_v[((k - 1) >> 1) * D_NV + nw - 1].ray[(k - 1) & 1];
-    }
+    // the records of layer l, IR / visible band nw (1-based)
+    __device__ __forceinline__ IrLayer &ir(int l, int nw) const { return lay_i[(nw - 1) * pitch + l]; }
+    __device__ __forceinline__ VisLayer &vis(int l, int nw) const { return lay_v[(nw - 1) * pitch + l]; }
+    // TAEROS, TCLOUD of level k, IR band nw; TRAY+TAEROS+TCLOUD, visible band nw
+    __device__ __forceinline__ double2 &ext(int k, int nw) const { return ir((k - 1) >> 1, nw).ext[(k - 1) & 1]; }
+    __device__ __forceinline__ double &ray(int k, int nw) const { return vis((k - 1) >> 1, nw).ray[(k - 1) & 1]; }
 };
 
 // Largest dynamic shared memory a CTA may use (227 KB opt-in on sm_100).
@@ -139,6 +140,7 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
     s.skip = reinterpret_cast<unsigned char *>(ip);
     s.meta = reinterpret_cast<int *>(((reinterpret_cast<uintptr_t>(s.skip + NSYS) + 15) / 16) * 16);
     s.odd = s.meta + 2 * SCREEN_GROUPS;
+    s.pitch = nl + 1;
     s.day = 0;
     return s;
 }

@@ -225,8 +225,8 @@ __device__ void solve_vis(const SegDev &sg, int c, int nw, int ng, int sidx, Col
             tcB = tcA;
             dt = da;
         }
-        const double wb = s.lay_v[l * D_NV + nw - 1].wnum / dt;
-        const double cb = s.lay_v[l * D_NV + nw - 1].cosb;
+        const double wb = s.vis(l, nw).wnum / dt;
+        const double cb = s.vis(l, nw).cosb;
         const double f = 1.0 - wb * (cb * cb);
         if (l == 1) {
             tau = 0.0 * f;
@@ -304,16 +304,16 @@ __device__ void solve_vis(const SegDev &sg, int c, int nw, int ng, int sidx, Col
     double et_bot = mgcm_rt_exp(-dmin(w.a3[NL + 1] / u0, MAXEXP));
     double et_top = mgcm_rt_exp(-dmin(w.a3[NL] / u0, MAXEXP));
     // layer NL-1's inputs are fetched one step ahead
-    const VisLayer *lv = s.lay_v + nw - 1;   // layer l at lv[l * D_NV]
-    double pw0 = w.a0[NL - 1], pcb = lv[(NL - 1) * D_NV].cbs, pdt = w.a2[NL - 1], pa3 = w.a3[NL - 1];
-    Lay hi = coef(NL, w.a0[NL], lv[NL * D_NV].cbs, w.a2[NL], et_top, et_bot);
+    const VisLayer *lv = &s.vis(0, nw);   // layer l at lv[l]
+    double pw0 = w.a0[NL - 1], pcb = lv[NL - 1].cbs, pdt = w.a2[NL - 1], pa3 = w.a3[NL - 1];
+    Lay hi = coef(NL, w.a0[NL], lv[NL].cbs, w.a2[NL], et_top, et_bot);
     double as, ds;
     bottom_row(hi, NL, bsurf, rsf, w, as, ds);
     for (int n = NL - 1; n >= 1; --n) {
         const double w0 = pw0, cb = pcb, dtl = pdt, a3n = pa3;
         if (n > 1) {
             pw0 = w.a0[n - 1];
-            pcb = lv[(n - 1) * D_NV].cbs;
+            pcb = lv[n - 1].cbs;
             pdt = w.a2[n - 1];
             pa3 = w.a3[n - 1];
         }
@@ -453,7 +453,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
         }
         double wb;
         if (dt > tiny) {
-            wb = s.lay_i[l * D_NI + nw - 1].wnum / dt;
+            wb = s.ir(l, nw).wnum / dt;
         } else {
             wb = 0.0;
             dt = tiny;
@@ -486,10 +486,10 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
     // 15.8 -> 15.4 ms).  The visible solve keeps its stored coefficients:
     // there the recomputation measured slower.
     auto lay4 = [&](int l, double w0, double dt, double &lam, double &gama, double &b1, double &term) {
-        const double cb = s.lay_i[l * D_NI + nw - 1].cosb;
+        const double cb = s.ir(l, nw).cosb;
         const double alpha = sqrt((1.0 - w0) / (1.0 - w0 * cb));
         lam = alpha * (1.0 - w0 * cb) / UBARI;
-        b1 = s.lay_i[l * D_NI + nw - 1].pdif / dt;
+        b1 = s.ir(l, nw).pdif / dt;
         gama = (1.0 - alpha) / (1.0 + alpha);
         term = UBARI / (1.0 - w0 * cb);
     };
@@ -497,7 +497,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
         Lay y;
         double lam, b1, term;
         lay4(l, w0, dt, lam, y.gama, b1, term);
-        const double b0 = s.lay_i[l * D_NI + nw - 1].b0;
+        const double b0 = s.ir(l, nw).b0;
         y.cp = b0 + b1 * dt + b1 * term;
         y.cm = b0 + b1 * dt - b1 * term;
         y.cpm1 = b0 + b1 * term;
@@ -549,7 +549,7 @@ __device__ void solve_ir(const SegDev &sg, int c, int nw, int ng, int sidx, ColS
         xprev = xb;
         double xk1, xk2;
         unmix(xa, xb, xk1, xk2);
-        const double b0 = s.lay_i[n * D_NI + nw - 1].b0;
+        const double b0 = s.ir(n, nw).b0;
         const double ep = mgcm_rt_exp(dmin(lam * dtk, TAUMAX));
         const double em = 1.0 / ep;
         const double cpmid = b0 + b1 * dtk + b1 * term;

@@ -79,8 +79,8 @@ __device__ __forceinline__ void fz_stage_column(const SegTable *__restrict__ st,
     const int lev1 = 2 * sg.L + 4;
     for (int k = 2 + lane; k <= lev1; k += 32) stage_level<false>(sg, c, K, s, k, status);
     __syncwarp();
-    const int nb = stage_band_items(sg.L);
-    for (int it = lane; it < nb; it += 32) stage_band<false>(sg, c, K, planck, s, it, status);
+    for (int b = 0; b < D_NV + D_NI; ++b)
+        for (int l = lane; l <= sg.L + 1; l += 32) stage_band<false>(sg, c, K, planck, s, b, l, status);
 }
 
 // Screen one (column, group) item of a tile, one warp; kept systems go to

@@ -93,7 +93,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
         }
         double wb;
         if (dt > tiny) {
-            wb = s.lay_i[l * D_NI + nw - 1].wnum / dt;
+            wb = s.ir(l, nw).wnum / dt;
         } else {
             wb = 0.0;
             dt = tiny;
@@ -110,10 +110,10 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
     const double btop = (1.0 - mgcm_rt_exp(-tautop / UBARI)) * s.pltop_i[nw - 1];
     const double bsurf = s.bsurf_i[nw - 1];
     auto lay4 = [&](int l, double w0, double dt, double &lam, double &gama, double &b1, double &term) {
-        const double cb = s.lay_i[l * D_NI + nw - 1].cosb;
+        const double cb = s.ir(l, nw).cosb;
         const double alpha = sqrt((1.0 - w0) / (1.0 - w0 * cb));
         lam = alpha * (1.0 - w0 * cb) / UBARI;
-        b1 = s.lay_i[l * D_NI + nw - 1].pdif / dt;
+        b1 = s.ir(l, nw).pdif / dt;
         gama = (1.0 - alpha) / (1.0 + alpha);
         term = UBARI / (1.0 - w0 * cb);
     };
@@ -121,7 +121,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
         Lay y;
         double lam, b1, term;
         lay4(l, w0, dt, lam, y.gama, b1, term);
-        const double b0 = s.lay_i[l * D_NI + nw - 1].b0;
+        const double b0 = s.ir(l, nw).b0;
         y.cp = b0 + b1 * dt + b1 * term;
         y.cm = b0 + b1 * dt - b1 * term;
         y.cpm1 = b0 + b1 * term;
@@ -186,7 +186,7 @@ __device__ void solve_ir_oc(const SegDev &sg, int c, int nw, int ng, const ColSm
         xprev = xb;
         double xk1, xk2;
         unmix(xa, xb, xk1, xk2);
-        const double b0 = s.lay_i[n * D_NI + nw - 1].b0;
+        const double b0 = s.ir(n, nw).b0;
         const double ep = mgcm_rt_exp(dmin(lam * dtk, TAUMAX));
         const double em = 1.0 / ep;
         const double cpmid = b0 + b1 * dtk + b1 * term;
@@ -238,8 +238,8 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
             tcB = tcA;
             dt = da;
         }
-        const double wb = s.lay_v[l * D_NV + nw - 1].wnum / dt;
-        const double cb = s.lay_v[l * D_NV + nw - 1].cosb;
+        const double wb = s.vis(l, nw).wnum / dt;
+        const double cb = s.vis(l, nw).cosb;
         const double f = 1.0 - wb * (cb * cb);
         if (l == 1) {
             tau = 0.0 * f;
@@ -267,7 +267,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     // LAMDA, GAMA, AM, AP of a layer from W0, the scaled COSBAR (staged per
     // layer and band) and U0; pass C and pass D both evaluate them
     struct Co { double lam, gama, am, ap; };
-    const VisLayer *lv = s.lay_v + nw - 1;   // layer l at lv[l * D_NV]
+    const VisLayer *lv = &s.vis(0, nw);   // layer l at lv[l]
     auto co4 = [&](double w0, double cb) {
         Co r;
         const double g1 = s3h * (2.0 - w0 * (1.0 + cb));
@@ -300,8 +300,8 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     double et_bot = mgcm_rt_exp(-dmin(st.get(oTAU + NL) / u0, MAXEXP));
     double et_top = mgcm_rt_exp(-dmin(st.get(oTAU + NL - 1) / u0, MAXEXP));
     const int nm = NL >= 2 ? NL - 2 : 0;
-    double pw0 = st.get(oW + nm), pcb = lv[(NL - 1) * D_NV].cbs, pdt = st.get(oDL + nm), pa3 = st.get(oTAU + nm);
-    Lay hi = coef(co4(st.get(oW + NL - 1), lv[NL * D_NV].cbs), st.get(oDL + NL - 1), et_top, et_bot);
+    double pw0 = st.get(oW + nm), pcb = lv[NL - 1].cbs, pdt = st.get(oDL + nm), pa3 = st.get(oTAU + nm);
+    Lay hi = coef(co4(st.get(oW + NL - 1), lv[NL].cbs), st.get(oDL + NL - 1), et_top, et_bot);
     double as, ds;
     bottom_row_v(hi, bsurf, rsf, as, ds);
     st.put(oAS + 2 * NL - 1, as);
@@ -310,7 +310,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
         const double w0 = pw0, cb = pcb, dtl = pdt, a3n = pa3;
         if (n > 1) {
             pw0 = st.get(oW + n - 2);
-            pcb = lv[(n - 1) * D_NV].cbs;
+            pcb = lv[n - 1].cbs;
             pdt = st.get(oDL + n - 2);
             pa3 = st.get(oTAU + n - 2);
         }
@@ -335,7 +335,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
     double xprev = 0.0;
     double nas1 = st.get(oAS), nds1 = st.get(oDS), nas2 = st.get(oAS + 1), nds2 = st.get(oDS + 1);
     double nw0 = st.get(oW), na3 = st.get(oTAU), na4 = st.get(oTCM);
-    double ncb = lv[1 * D_NV].cbs;
+    double ncb = lv[1].cbs;
     const double tbot = st.get(oTAU + NL);
     for (int n = 1; n <= NL; ++n) {
         const double as1 = nas1, ds1 = nds1, as2 = nas2, ds2 = nds2;
@@ -346,7 +346,7 @@ __device__ void solve_vis_oc(const SegDev &sg, int c, int nw, int ng, const ColS
             nas2 = st.get(oAS + 2 * n + 1);
             nds2 = st.get(oDS + 2 * n + 1);
             nw0 = st.get(oW + n);
-            ncb = lv[(n + 1) * D_NV].cbs;
+            ncb = lv[n + 1].cbs;
             na3 = st.get(oTAU + n);
             na4 = n + 1 < NL ? st.get(oTCM + n) : 0.0;
         }

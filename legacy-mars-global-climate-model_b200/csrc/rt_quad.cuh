@@ -65,12 +65,12 @@ __device__ __forceinline__ void quad_vis(const SegDev &sg, int c, int nw, int ng
             } else {
                 dt = da[j];
             }
-            const double wb = s.lay_v[l * D_NV + nw - 1].wnum / dt;
-            const double cb = s.lay_v[l * D_NV + nw - 1].cosb;
+            const double wb = s.vis(l, nw).wnum / dt;
+            const double cb = s.vis(l, nw).cosb;
             const double f = 1.0 - wb * (cb * cb);
             fv[j] = f;
             w0v[j] = wb * (1.0 - cb * cb) / f;
-            cbv[j] = s.lay_v[l * D_NV + nw - 1].cbs;
+            cbv[j] = s.vis(l, nw).cbs;
             dtl[j] = dt * f;
         }
     }
@@ -293,7 +293,7 @@ __device__ __forceinline__ void quad_ir(const SegDev &sg, int c, int nw, int ng,
         }
         double wb;
         if (dt > tiny) {
-            wb = s.lay_i[l * D_NI + nw - 1].wnum / dt;
+            wb = s.ir(l, nw).wnum / dt;
         } else {
             wb = 0.0;
             dt = tiny;
@@ -335,10 +335,10 @@ __device__ __forceinline__ void quad_ir(const SegDev &sg, int c, int nw, int ng,
         ep[j] = em[j] = 1.0;
         if (!own(j)) continue;
         const int l = lfirst + j;
-        const double w0 = w0v[j], cb = s.lay_i[l * D_NI + nw - 1].cosb, dt = dtv[j];
+        const double w0 = w0v[j], cb = s.ir(l, nw).cosb, dt = dtv[j];
         const double alpha = sqrt((1.0 - w0) / (1.0 - w0 * cb));
         lam[j] = alpha * (1.0 - w0 * cb) / UBARI;
-        b1v[j] = s.lay_i[l * D_NI + nw - 1].pdif / dt;
+        b1v[j] = s.ir(l, nw).pdif / dt;
         gam[j] = (1.0 - alpha) / (1.0 + alpha);
         term[j] = UBARI / (1.0 - w0 * cb);
         ep[j] = mgcm_rt_exp(dmin(lam[j] * dt, TAUMAX));
@@ -347,7 +347,7 @@ __device__ __forceinline__ void quad_ir(const SegDev &sg, int c, int nw, int ng,
     auto lay = [&](int j) {
         Lay y;
         const int l = lfirst + j;
-        const double b0 = s.lay_i[l * D_NI + nw - 1].b0, b1 = b1v[j], dt = dtv[j], tm = term[j];
+        const double b0 = s.ir(l, nw).b0, b1 = b1v[j], dt = dtv[j], tm = term[j];
         y.gama = gam[j];
         y.cp = b0 + b1 * dt + b1 * tm;
         y.cm = b0 + b1 * dt - b1 * tm;
@@ -414,7 +414,7 @@ __device__ __forceinline__ void quad_ir(const SegDev &sg, int c, int nw, int ng,
         const double dtk = l < NL ? a4[j] : dtv[j];
         ep[j] = mgcm_rt_exp(dmin(lam[j] * dtk, TAUMAX));
         em[j] = 1.0 / ep[j];
-        const double b0 = s.lay_i[l * D_NI + nw - 1].b0, b1 = b1v[j];
+        const double b0 = s.ir(l, nw).b0, b1 = b1v[j];
         lam[j] = b0 + b1 * dtk + b1 * term[j];   // CPMID
         a4[j] = b0 + b1 * dtk - b1 * term[j];    // CMMID
     }
@@ -437,7 +437,7 @@ __device__ __forceinline__ void quad_ir(const SegDev &sg, int c, int nw, int ng,
                     fmp[(size_t)(l - 1) * rs] = p * PI_D;
                     fmm[(size_t)(l - 1) * rs] = m * PI_D;
                     if (l == 1) {
-                        const double b0 = s.lay_i[l * D_NI + nw - 1].b0, b1 = b1v[j];
+                        const double b0 = s.ir(l, nw).b0, b1 = b1v[j];
                         const double e1 = 1.0, e2 = 1.0;
                         const double cpm = b0 + b1 * term[j], cmm = b0 - b1 * term[j];
                         const double fup = xk1 * e1 + gama * xk2 * e2 + cpm;

@@ -216,7 +216,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
             exp_terms(y, lam * dt);
             return y;
         };
-        const IrLayer *r = s.lay_i + NL * D_NI + nb;
+        const IrLayer *r = &s.ir(NL, nb + 1);
         double2 e = r->ext[0];
         double tg = gas ? taugas_at(s, LEV, tb) : 0.0;
         taug = tg;
@@ -229,7 +229,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
         w.ir[NL].even = make_double2(as, ds);
 #pragma unroll 1
         for (int n = NL - 1; n >= 1; --n) {
-            r -= D_NI;
+            --r;
             const double2 e1 = r->ext[0], e2 = r->ext[1];
             double db;
             if (gas) {
@@ -246,7 +246,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
             }
             w.ir[n].pair = make_double2(da, db);
             if (n > 1) {
-                prefetch_l1(r - D_NI);
+                prefetch_l1(r - 1);
                 prefetch_l1(s.klev + 2 * n - 1);
             }
             const Lay lo = coef(*r, da + db);
@@ -258,7 +258,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
             w.ir[n].even = make_double2(as, ds);
             hi = lo;
         }
-        r -= D_NI;
+        --r;
         e = r->ext[1];
         tg = gas ? taugas_at(s, 2, tb) : 0.0;
         taug += tg;
@@ -292,7 +292,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
         general_ir(sg, col_begin + cc - sg.col0, i - cc * NSYS_I, block, max_nl, K, ki, w.g, fmp, fmm, sc0);
         return 0;
     }
-    const IrLayer *r = carve_smem(block, max_nl, nullptr, false).lay_i + nb;
+    const IrLayer *r = &carve_smem(block, max_nl, nullptr, false).ir(0, nb + 1);
     double xprev = 0.0;
     double2 n1 = make_double2(as1, ds1), n2 = w.ir[1].even, np = w.ir[1].pair;
 #pragma unroll 1
@@ -303,8 +303,8 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
             n2 = w.ir[n + 1].even;
             np = w.ir[n + 1].pair;
         }
-        r += D_NI;
-        if (n < NL) prefetch_l1(r + D_NI);
+        ++r;
+        if (n < NL) prefetch_l1(r + 1);
         const double tcA = tc + p.x;
         const double dtsum = n < NL ? p.x + p.y : p.x;
         const bool thick = dtsum > tiny;
@@ -353,7 +353,7 @@ struct VisPassA {
         const size_t to = (size_t)nb * D_NT * D_NP * D_NH * D_NGK + ng;
         const double *tb = kv + to;
         const float *tbf = F32 ? kvf + to : nullptr;
-        const VisLayer *lay = s.lay_v + nb;
+        const VisLayer *lay = &s.vis(0, nb + 1);
         auto level = [&](int k, double ray) -> double {
             if (!gas) return ray;
             const double tg = F32 ? (double)taugas_f(s, k, tbf) : taugas_at(s, k, tb);
@@ -366,9 +366,9 @@ struct VisPassA {
 #pragma unroll 1
         for (int l = 1; l <= NL; ++l) {
             const int k = 2 * l + 1;
-            lay += D_NV;
+            ++lay;
             if (true && l < NL) {
-                prefetch_l1(lay + D_NV);
+                prefetch_l1(lay + 1);
                 prefetch_l1(s.klev + k + 2);
             }
             double da, dt, tcA, tcB;
@@ -463,7 +463,7 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
     // u0 in [2^-30, 2^30), the band's sun 0 or in [2^-60, 2^60)
     bool odd = a.odd || hi32(u0) - 0x3e100000u >= 0x03c00000u || (f0pi != 0.0 && hi32(f0pi) - 0x3c300000u >= 0x07800000u);
     if (!odd) {
-        const VisLayer *lay = s.lay_v + NL * D_NV + nb;
+        const VisLayer *lay = &s.vis(NL, nb + 1);
         const double rcp_u0 = rcp_n(u0), rcp_u02 = 1.0 / (u0 * u0);
         const double s3 = (double)sqrtf(3.0f), s3h = (double)(sqrtf(3.0f) * 0.5f);
         const double bsurf = rsf * u0 * f0pi * beam(a.tau, u0, rcp_u0);
@@ -510,8 +510,8 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
             }
             et_bot = et_top;
             et_top = beam(d, u0, rcp_u0);
-            lay -= D_NV;
-            if (n > 1) prefetch_l1(&lay[-D_NV].cbs);
+            --lay;
+            if (n > 1) prefetch_l1(&lay[-1].cbs);
             const Lay lo = coef(n, cur, lay->cbs, et_top, et_bot);
             double ao, dd;
             fast_rows(lo, hi, as, ds, ao, dd, odd);

@@ -132,159 +132,120 @@ __device__ inline void stage_level(const SegDev &sg, int c, const RtConst &K, Co
     }
 }
 
-// Band items of a column: nitem_v = (NL+1)*7 visible (layer l = 0..NL: level 2
-// for l = 0), nitem_i = (NL+1)*5 IR with the Planck terms, then 5 IR boundary
-// items.  Needs every level item of the column staged first.
-__device__ __forceinline__ int stage_band_items(int L) { return (L + 2) * (D_NV + D_NI) + D_NI; }
-
-// With V the items check every value of the band arrays: layer item l its
-// levels, item 0 also level 1 and item NL level LEV+1.
+// Record of layer l (0..NL; 0: level 2 only) of a band b of a column: 0..6
+// visible, 7..11 IR with the Planck terms, layer 0 of the IR bands also the
+// boundary terms.  Needs every level item of the column staged first.  Lanes
+// along the layers read each input array contiguously and write whole records.
+// With V the items check every value of the band arrays: a layer item its
+// levels, layer 0 also level 1 and layer NL level LEV+1.
 template <bool V>
 __device__ inline void stage_band(const SegDev &sg, int c, const RtConst &K,
-                                  const double *__restrict__ planck, ColSmem &s, int it,
+                                  const double *__restrict__ planck, ColSmem &s, int b, int l,
                                   uint32_t *status) {
     const int L = sg.L, NL = L + 1, LEV = 2 * L + 3, LEV1 = LEV + 1;
-    const double *tlev = sg.tlev + (size_t)c * LEV;
     const bool cld = sg.taurefcld != nullptr;
-    const int nitem_v = (NL + 1) * D_NV, nitem_i = (NL + 1) * D_NI;
     Check<V> chk;
-    {
-        if (it < nitem_v) {
-            const int l = it / D_NV, nw = it % D_NV + 1;
-            // dust properties of level k at qx[(k - 1) * ks] (ks = 0: band constants)
-            const double *db = sg.dust_band;
-            const int ks = db ? 0 : 1;
-            const double *qx = db ? db + nw - 1 : sg.qxvdst + ((size_t)c * D_NV + nw - 1) * LEV1;
-            const double *qs = db ? db + D_NV + nw - 1 : sg.qsvdst + ((size_t)c * D_NV + nw - 1) * LEV1;
-            const double *gv = db ? db + 2 * D_NV + nw - 1 : sg.gvdst + ((size_t)c * D_NV + nw - 1) * LEV1;
-            const double *qxc = cld ? sg.qxvcld + ((size_t)c * D_NV + nw - 1) * LEV1 : nullptr;
-            const double *qsc = cld ? sg.qsvcld + ((size_t)c * D_NV + nw - 1) * LEV1 : nullptr;
-            const double *gc = cld ? sg.gvcld + ((size_t)c * D_NV + nw - 1) * LEV1 : nullptr;
-            const double tr0 = K.tauray[nw - 1];
-            auto check = [&](int i) {
-                if (V) {
-                    if (!db) {
-                        chk.finite(qx[i]);
-                        chk.finite(qs[i]);
-                        chk.finite(gv[i]);
-                    }
-                    if (cld) {
-                        chk.finite(qxc[i]);
-                        chk.finite(qsc[i]);
-                        chk.finite(gc[i]);
-                    }
-                }
-            };
-            auto lvl = [&](int k, double &tr, double &tl, double &tc, double &g1, double &g2) {
-                tr = tr0 * s.dpr[k];
-                const double taeros = s.tref_v[k] * qx[(k - 1) * ks];
-                const double tcloud = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
-                s.ray(k, nw) = tr + taeros + tcloud;
-                tl = s.tref_v[k] * qs[(k - 1) * ks];
-                tc = s.tref_c[k] * (cld ? qsc[k - 1] : 0.0);
-                g1 = gv[(k - 1) * ks];
-                g2 = cld ? gc[k - 1] : 0.0;
-                check(k - 1);
-            };
-            bool usual = true;
-            double tra, tla, tca, ga, gca;
-            if (l == 0) {
-                lvl(2, tra, tla, tca, ga, gca);
-                check(0);
-            } else if (l <= L) {
-                const int k = 2 * l + 1;
-                double trb, tlb, tcb, gb, gcb;
-                lvl(k, tra, tla, tca, ga, gca);
-                lvl(k + 1, trb, tlb, tcb, gb, gcb);
-                const double cb = (ga * tla + gb * tlb + gca * tca + gcb * tcb) / (tra + trb + tla + tlb + tca + tcb);
-                s.lay_v[l * D_NV + nw - 1].cosb = cb;
-                s.lay_v[l * D_NV + nw - 1].cbs = cb / (1.0 + cb);   // code/getdetau.f90:29-56
-                const double wn = tla + tlb + tca + tcb + (tra + trb) * R4(0.9999);
-                s.lay_v[l * D_NV + nw - 1].wnum = wn;
-                usual = usual_layer(cb, wn);
-            } else {
-                const int k = LEV;
-                lvl(k, tra, tla, tca, ga, gca);
-                const double cb = (ga * tla + gca * tca) / (tra + tla + tca);
-                s.lay_v[l * D_NV + nw - 1].cosb = cb;
-                s.lay_v[l * D_NV + nw - 1].cbs = cb / (1.0 + cb);
-                const double wn = tla + tca + tra * R4(0.9999);
-                s.lay_v[l * D_NV + nw - 1].wnum = wn;
-                usual = usual_layer(cb, wn);
-                check(LEV);
-            }
-            if (!usual) atomicOr(s.odd, 1 << (nw - 1));
-        } else if (it < nitem_v + nitem_i) {
-            const int j = it - nitem_v;
-            const int l = j / D_NI, nw = j % D_NI + 1;
-            const double *db = sg.dust_band;
-            const int ks = db ? 0 : 1;
-            const double *qx = db ? db + 3 * D_NV + nw - 1 : sg.qxidst + ((size_t)c * D_NI + nw - 1) * LEV1;
-            const double *qs = db ? db + 3 * D_NV + D_NI + nw - 1
-                                  : sg.qsidst + ((size_t)c * D_NI + nw - 1) * LEV1;
-            const double *gi = db ? db + 3 * D_NV + 2 * D_NI + nw - 1
-                                  : sg.gidst + ((size_t)c * D_NI + nw - 1) * LEV1;
-            const double *qxc = cld ? sg.qxicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
-            const double *qsc = cld ? sg.qsicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
-            const double *gc = cld ? sg.gicld + ((size_t)c * D_NI + nw - 1) * LEV1 : nullptr;
-            auto ext = [&](int k) {   // TAEROS, TCLOUD at level k <= LEV
-                s.ext(k, nw).x = s.tref_i[k] * qx[(k - 1) * ks];
-                s.ext(k, nw).y = s.tref_c[k] * (cld ? qxc[k - 1] : 0.0);
-            };
-            auto check = [&](int i) {
-                if (V) {
-                    if (!db) {
-                        chk.finite(qx[i]);
-                        chk.finite(qs[i]);
-                        chk.finite(gi[i]);
-                    }
-                    if (cld) {
-                        chk.finite(qxc[i]);
-                        chk.finite(qsc[i]);
-                        chk.finite(gc[i]);
-                    }
-                }
-            };
-            if (l == 0) {
-                ext(2);
-                check(0);
-                check(1);
-            } else {
-                const int k = 2 * l + 1;
-                ext(k);
-                if (k + 1 <= LEV) ext(k + 1);
-                check(k - 1);
-                check(k);
-                const double tla = s.tref_i[k] * qs[(k - 1) * ks], tlb = s.tref_i[k + 1] * qs[k * ks];
-                const double tca = s.tref_c[k] * (cld ? qsc[k - 1] : 0.0);
-                const double tcb = s.tref_c[k + 1] * (cld ? qsc[k] : 0.0);
-                const double tauac = tla + tlb + tca + tcb;
-                s.lay_i[l * D_NI + nw - 1].wnum = tauac;
-                double cb = 0.0;
-                if (tauac > 0.0)
-                    cb = (gi[(k - 1) * ks] * tla + gi[k * ks] * tlb + (cld ? gc[k - 1] : 0.0) * tca +
-                          (cld ? gc[k] : 0.0) * tcb) /
-                         (tla + tlb + tca + tcb);
-                s.lay_i[l * D_NI + nw - 1].cosb = cb;
-                // Planck source terms (gfluxi.f90:219-239)
-                const int na = planck_index(l < NL ? tlev[2 * l - 1] : tlev[2 * l + 1 - 1], status);
-                const int nb = planck_index(l < NL ? tlev[2 * l + 2 - 1] : tlev[2 * l - 1], status);
-                const double pa = planck[(na - 1) * D_NI + nw - 1], pb = planck[(nb - 1) * D_NI + nw - 1];
-                const double pd = l < NL ? pb - pa : pa - pb;
-                s.lay_i[l * D_NI + nw - 1].pdif = pd;
-                s.lay_i[l * D_NI + nw - 1].b0 = l < NL ? pa : pb;
-                if (!usual_layer(cb, tauac) || (pd != 0.0 && out_of_range(pd)))
-                    atomicOr(s.odd, 1 << (D_NV + nw - 1));
-            }
+    const bool vis = b < D_NV;
+    const int nb = vis ? D_NV : D_NI, w = vis ? b : b - D_NV;   // 0-based band of the family
+    // dust properties of level k at q[(k - 1) * ks] (ks = 0: band constants)
+    const double *db = sg.dust_band;
+    const int ks = db ? 0 : 1;
+    const size_t row = ((size_t)c * nb + w) * LEV1;
+    const double *qx, *qs, *qg, *cx = nullptr, *cs = nullptr, *cg = nullptr;
+    if (vis) {
+        qx = db ? db + w : sg.qxvdst + row;
+        qs = db ? db + D_NV + w : sg.qsvdst + row;
+        qg = db ? db + 2 * D_NV + w : sg.gvdst + row;
+        if (cld) { cx = sg.qxvcld + row; cs = sg.qsvcld + row; cg = sg.gvcld + row; }
+    } else {
+        qx = db ? db + 3 * D_NV + w : sg.qxidst + row;
+        qs = db ? db + 3 * D_NV + D_NI + w : sg.qsidst + row;
+        qg = db ? db + 3 * D_NV + 2 * D_NI + w : sg.gidst + row;
+        if (cld) { cx = sg.qxicld + row; cs = sg.qsicld + row; cg = sg.gicld + row; }
+    }
+    struct Lv {
+        double qx, qs, g, cx, cs, cg;
+    };
+    auto read = [&](int k) {   // level k <= LEV1
+        Lv v;
+        v.qx = qx[(k - 1) * ks];
+        v.qs = qs[(k - 1) * ks];
+        v.g = qg[(k - 1) * ks];
+        v.cx = cld ? cx[k - 1] : 0.0;
+        v.cs = cld ? cs[k - 1] : 0.0;
+        v.cg = cld ? cg[k - 1] : 0.0;
+        chk.finite(v.qx);
+        chk.finite(v.qs);
+        chk.finite(v.g);
+        chk.finite(v.cx);
+        chk.finite(v.cs);
+        chk.finite(v.cg);
+        return v;
+    };
+    const int ka = l ? 2 * l + 1 : 2;   // the item's first level
+    const Lv A = read(ka);
+    Lv B = {};
+    if (l) B = read(ka + 1);             // the layer's second level; LEV+1 for l = NL
+    else if (V) read(1);
+    bool usual = true;
+    if (vis) {
+        const double tr0 = K.tauray[w];
+        VisLayer r;
+        r.cosb = r.wnum = r.cbs = r.pad = 0.0;
+        const double tra = tr0 * s.dpr[ka];
+        const double raya = tra + s.tref_v[ka] * A.qx + s.tref_c[ka] * A.cx;
+        const double tla = s.tref_v[ka] * A.qs, tca = s.tref_c[ka] * A.cs;
+        r.ray[0] = l ? raya : 0.0;
+        r.ray[1] = l ? 0.0 : raya;
+        if (l && l <= L) {
+            const int kb = ka + 1;
+            const double trb = tr0 * s.dpr[kb];
+            r.ray[1] = trb + s.tref_v[kb] * B.qx + s.tref_c[kb] * B.cx;
+            const double tlb = s.tref_v[kb] * B.qs, tcb = s.tref_c[kb] * B.cs;
+            r.cosb = (A.g * tla + B.g * tlb + A.cg * tca + B.cg * tcb) / (tra + trb + tla + tlb + tca + tcb);
+            r.wnum = tla + tlb + tca + tcb + (tra + trb) * R4(0.9999);
+        } else if (l) {
+            r.cosb = (A.g * tla + A.cg * tca) / (tra + tla + tca);
+            r.wnum = tla + tca + tra * R4(0.9999);
+        }
+        if (l) {
+            r.cbs = r.cosb / (1.0 + r.cosb);   // code/getdetau.f90:29-56
+            usual = usual_layer(r.cosb, r.wnum);
+        }
+        s.vis(l, w + 1) = r;
+    } else {
+        const double *tlev = sg.tlev + (size_t)c * LEV;
+        IrLayer r;
+        r.cosb = r.wnum = r.b0 = r.pdif = 0.0;
+        const double2 exta = make_double2(s.tref_i[ka] * A.qx, s.tref_c[ka] * A.cx);   // TAEROS, TCLOUD
+        r.ext[0] = exta;
+        r.ext[1] = l ? make_double2(0.0, 0.0) : exta;
+        if (l) {
+            const int kb = ka + 1;
+            if (kb <= LEV) r.ext[1] = make_double2(s.tref_i[kb] * B.qx, s.tref_c[kb] * B.cx);
+            const double tla = s.tref_i[ka] * A.qs, tlb = s.tref_i[kb] * B.qs;
+            const double tca = s.tref_c[ka] * A.cs, tcb = s.tref_c[kb] * B.cs;
+            const double tauac = tla + tlb + tca + tcb;
+            if (tauac > 0.0)
+                r.cosb = (A.g * tla + B.g * tlb + A.cg * tca + B.cg * tcb) / (tla + tlb + tca + tcb);
+            r.wnum = tauac;
+            // Planck source terms (gfluxi.f90:219-239)
+            const int na = planck_index(l < NL ? tlev[2 * l - 1] : tlev[2 * l + 1 - 1], status);
+            const int nt = planck_index(l < NL ? tlev[2 * l + 2 - 1] : tlev[2 * l - 1], status);
+            const double pa = planck[(na - 1) * D_NI + w], pb = planck[(nt - 1) * D_NI + w];
+            r.pdif = l < NL ? pb - pa : pa - pb;
+            r.b0 = l < NL ? pa : pb;
+            usual = usual_layer(r.cosb, tauac) && (r.pdif == 0.0 || !out_of_range(r.pdif));
         } else {
             // IR boundary terms (sfluxi.f90:51-62)
-            const int nw = it - nitem_v - nitem_i + 1;
             const int nts = planck_index(tlev[LEV - 1], status);
             const int ntt = planck_index(tlev[2 - 1], status);
-            s.bsurf_i[nw - 1] = (1.0 - sg.albi[c]) * planck[(nts - 1) * D_NI + nw - 1];
-            s.pltop_i[nw - 1] = planck[(ntt - 1) * D_NI + nw - 1];
+            s.bsurf_i[w] = (1.0 - sg.albi[c]) * planck[(nts - 1) * D_NI + w];
+            s.pltop_i[w] = planck[(ntt - 1) * D_NI + w];
         }
+        s.ir(l, w + 1) = r;
     }
+    if (!usual) atomicOr(s.odd, 1 << b);
     chk.report(status);
 }
 
@@ -295,8 +256,9 @@ __device__ inline void stage_column(const SegDev &sg, int c, const RtConst &K,
     const int LEV1 = 2 * sg.L + 4;
     for (int k = 2 + (int)threadIdx.x; k <= LEV1; k += blockDim.x) stage_level<false>(sg, c, K, s, k, status);
     __syncthreads();
-    const int n = stage_band_items(sg.L);
-    for (int it = threadIdx.x; it < n; it += blockDim.x) stage_band<false>(sg, c, K, planck, s, it, status);
+    const int n = (sg.L + 2) * (D_NV + D_NI);
+    for (int it = threadIdx.x; it < n; it += blockDim.x)
+        stage_band<false>(sg, c, K, planck, s, it / (sg.L + 2), it % (sg.L + 2), status);
 }
 
 }  // namespace mgcm
