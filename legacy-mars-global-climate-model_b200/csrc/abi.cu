@@ -87,6 +87,8 @@ __global__ void rt_dsolflux_kernel(int ncol, const double *__restrict__ sol,
                                    const double *__restrict__ detau,
                                    const double *__restrict__ dndiffv,
                                    double *__restrict__ dnvflux, const RtConst K);
+size_t dsolflux_ctas(int ncol);
+constexpr int DSOLFLUX_THREADS = 128;
 template <bool VIS, bool F32, int T>
 __global__ void rt_solve_oc(const SegTable *__restrict__ st, int col_begin, int max_nl,
                             unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ ktab,
@@ -1813,7 +1815,7 @@ int mgcm_rt_dsolflux(mgcm_rt_handle *h, int ncol, int device_ptrs, const double 
         CK(cudaMemcpyAsync(pn, dndiffv, n * 8, cudaMemcpyHostToDevice, st));
         ds = p; da = pa; dd = pd; dn = pn; dout = po;
     }
-    rt_dsolflux_kernel<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, ds, da, dd, dn, dout, h->K);
+    rt_dsolflux_kernel<<<(unsigned)dsolflux_ctas(ncol), DSOLFLUX_THREADS, 0, st>>>(ncol, ds, da, dd, dn, dout, h->K);
     CK(cudaGetLastError());
     if (!device_ptrs) CK(cudaMemcpyAsync(dnvflux, dout, (size_t)ncol * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

@@ -567,30 +567,60 @@ const void *reduce_kernel(int rb) {
 
 // Partial radiation: DIRECTSOL from DETAU (code/dsolflux.f:28-45) and
 // DNVFLUX = DNDIFFV + DIRECTSOL (code/comp3.f:335-351).
-__global__ void rt_dsolflux_kernel(int ncol, const double *__restrict__ sol,
-                                   const double *__restrict__ acosz,
-                                   const double *__restrict__ detau,
-                                   const double *__restrict__ dndiffv,
-                                   double *__restrict__ dnvflux, const RtConst K) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncol) return;
-    const double u0 = acosz[c];
-    double ds = 0.0;
-    if (u0 >= R4(1.0e-5)) {
-        const double *de = detau + (size_t)c * 119;
-        for (int nw = 1; nw <= D_NV; ++nw) {
-            const double factor = u0 * sol[nw - 1];
-            for (int ng = 1; ng <= D_NG - 1; ++ng) {
-                const double d = de[(nw - 1) + 7 * (ng - 1)];
-                if (d <= 5.0) ds = ds + factor * mgcm_rt_exp(-d / u0) * K.gweight[ng - 1] * (1.0 - K.fzerov[nw - 1]);
+//
+// A CTA takes 32 columns: its threads read the columns' DETAU coalesced and
+// put the 119 terms of each into shared memory, then a thread per column
+// adds them in the reference's order (band by band; a term of DETAU > 5
+// counts as +0).  Night columns are not read.
+constexpr int DSOL_COLS = 32, DSOL_THREADS = 128, DSOL_ROW = NSYS_V + 2;   // odd pitch: no bank conflicts
+constexpr int DSOL_MLP = 10;   // DETAU values a thread has in flight
+
+__global__ void __launch_bounds__(DSOL_THREADS)
+rt_dsolflux_kernel(int ncol, const double *__restrict__ sol, const double *__restrict__ acosz,
+                   const double *__restrict__ detau, const double *__restrict__ dndiffv,
+                   double *__restrict__ dnvflux, const RtConst K) {
+    __shared__ double term[DSOL_COLS * DSOL_ROW], u0s[DSOL_COLS], rcp[DSOL_COLS];
+    const int t = threadIdx.x, c0 = blockIdx.x * DSOL_COLS, nc = min(DSOL_COLS, ncol - c0);
+    if (t < nc) {
+        u0s[t] = acosz[c0 + t];
+        rcp[t] = 1.0 / u0s[t];
+    }
+    __syncthreads();
+    for (int i0 = t; i0 < nc * NSYS_V; i0 += DSOL_MLP * DSOL_THREADS) {
+        double dv[DSOL_MLP];
+#pragma unroll
+        for (int q = 0; q < DSOL_MLP; ++q) {
+            const int i = i0 + q * DSOL_THREADS;
+            dv[q] = i < nc * NSYS_V && u0s[i / NSYS_V] >= R4(1.0e-5) ? detau[(size_t)c0 * NSYS_V + i] : 6.0;
+        }
+#pragma unroll
+        for (int q = 0; q < DSOL_MLP; ++q) {
+            const int i = i0 + q * DSOL_THREADS;
+            if (i >= nc * NSYS_V) break;
+            const int c = i / NSYS_V, e = i - c * NSYS_V, ng = e / D_NV, nw = e - ng * D_NV;
+            const double u0 = u0s[c], d = dv[q];
+            double v = 0.0;
+            if (d <= 5.0) {
+                // the quotient and the exponential without their special cases
+                // where the operands allow it (rt_fastmath.cuh)
+                const bool usual = d > 0x1p-300 && u0 < 0x1p300;
+                const double x = usual ? -quot(d, u0, rcp[c]) : -d / u0;
+                const double w = fabs(x) < 700.0 ? exp_r(x) : mgcm_rt_exp(x);
+                v = u0 * sol[nw] * w;
+                v = ng < D_NG - 1 ? v * K.gweight[ng] * (1.0 - K.fzerov[nw]) : v * K.fzerov[nw];
             }
-            const double d = de[(nw - 1) + 7 * 16];
-            if (d <= 5.0) ds = ds + factor * mgcm_rt_exp(-d / u0) * K.fzerov[nw - 1];
+            term[c * DSOL_ROW + nw * D_NG + ng] = v;
         }
     }
-    dnvflux[c] = dndiffv[c] + ds;
+    __syncthreads();
+    if (t < nc) {
+        double ds = 0.0;
+        if (u0s[t] >= R4(1.0e-5))
+            for (int q = 0; q < NSYS_V; ++q) ds = ds + term[t * DSOL_ROW + q];
+        dnvflux[c0 + t] = dndiffv[c0 + t] + ds;
+    }
 }
-
+size_t dsolflux_ctas(int ncol) { return (size_t)(ncol + DSOL_COLS - 1) / DSOL_COLS; }
 
 // Integer bins as the pipeline uses them, for the bit-exact check of
 // tpindex (code/tpindex.f90:72-134) and of the Planck index INT(T*10-499)
