@@ -884,14 +884,26 @@ int issue_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt_batch_
 }
 
 // Device-pointer batches.  The columns are split into up to SYNC_SLOTS parts
-// of at least SPLIT_COLS columns that run concurrently on the synchronous
-// slots -- the first on the caller's stream, the others on their slots'
-// streams, forked from and joined back into it -- so the parts' kernels share
-// the SMs, which these latency-bound kernels use better than one call's
-// kernels (64,800 columns: 12.66 ms in one call; as 2 / 3 / 4 concurrent
-// calls 12.2 / 12.0 / 11.9 ms).  The fused form, a persistent kernel that
-// fills the GPU by itself, runs unsplit.
-constexpr int SPLIT_COLS = 12288;
+// that run concurrently on the synchronous slots -- the first on the caller's
+// stream, the others on their slots' streams, forked from and joined back
+// into it -- so the parts' kernels share the SMs, which these latency-bound
+// kernels use better than one call's kernels.  The fused form, a persistent
+// kernel that fills the GPU by itself, runs unsplit.
+//
+// Parts by layers in the call (columns x (L + 1)); us at 1 / 2 / 3 / 4 parts:
+//   2,160 x 24: 458 / 458 / 468 / 473            4,096 x 24: 764 / 692 / 716 / 741
+//   8,192 x 24: 1,396 / 1,258 / 1,250 / 1,313    8,640 x 36: 2,325 / 2,129 / 2,132 / 2,304
+//   16,200 x 24: 2,574 / 2,366 / 2,380 / 2,341   16,200 x 48: 6,334 / 5,866 / 5,847 / 5,834
+constexpr long long SPLIT2_LAYERS = 80000, SPLIT4_LAYERS = 400000;
+int parts_of_layers(long long layers) {
+    return layers < SPLIT2_LAYERS ? 1 : (layers < SPLIT4_LAYERS ? 2 : SYNC_SLOTS);
+}
+int parts_of(const mgcm_rt_handle *h, int nbatch, const mgcm_rt_batch_in *in) {
+    long long layers = 0;
+    for (int b = 0; b < nbatch; ++b) layers += (long long)sizes_of(in[b]).ncol * sizes_of(in[b]).nl;
+    return h->fused ? 1 : parts_of_layers(layers);
+}
+
 
 // Segment table of the global columns [b0, b1) of the batches, every
 // per-column pointer shifted to the segment's first column in the range;
@@ -942,7 +954,7 @@ int run_device(mgcm_rt_handle *h, int nbatch, const mgcm_rt_batch_in *in, mgcm_r
     if (!h->user_stream) {
         if (const int rc = after_legacy_stream(s0, st)) return rc;
     }
-    const int nparts = h->fused ? 1 : std::max(1, std::min(SYNC_SLOTS, total / SPLIT_COLS));
+    const int nparts = parts_of(h, nbatch, in);
     if (nparts > 1) {
         CK(cudaEventRecord(h->fork, st));
         for (int p = 1; p < nparts; ++p) CK(cudaStreamWaitEvent(h->slots[p]->stream, h->fork, 0));
@@ -1394,7 +1406,9 @@ int run_tracers(mgcm_rt_handle *h, const mgcm_rt_batch_tracers &in, mgcm_rt_batc
     long long systems = 0;
     int nk = 0, k = 0;
     bool used[JOB_SLOTS] = {};
-    const std::vector<int> ends = in.device_ptrs ? job_ends(in.ncol, 4 * SYNC_JOB_COLS, 0)
+    // device inputs: as many concurrent jobs as a device-pointer call has parts
+    const int parts = parts_of_layers((long long)in.ncol * (in.nlayers + 1));
+    const std::vector<int> ends = in.device_ptrs ? job_ends(in.ncol, std::min(4 * SYNC_JOB_COLS, (in.ncol + parts - 1) / parts), 0)
                                                  : job_ends(in.ncol, SYNC_JOB_COLS, SYNC_RAMP_COLS);
     int c0 = 0;
     for (const int c1 : ends) {
@@ -2077,7 +2091,7 @@ int mgcm_rt_graph_create(mgcm_rt_handle *h, int nbatch, const mgcm_rt_batch_in *
         delete g;
         return MGCM_RT_EINVAL;
     }
-    g->nparts = h->fused ? 1 : std::max(1, std::min(SYNC_SLOTS, total / SPLIT_COLS));
+    g->nparts = parts_of(h, nbatch, in);
     for (int p = 0; p < g->nparts; ++p)
         if (slot_init(g->part(p))) {
             g->nparts = p + 1;   // slot_free the ones begun
