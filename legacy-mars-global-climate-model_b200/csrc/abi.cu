@@ -1373,10 +1373,10 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
         rt_prep<<<pg, PREP_THREADS, 0, st>>>(ps);
         CK(cudaGetLastError());
     }
-    // a warp per column, AERO_WARPS columns per CTA, up to 8 CTAs per SM resident
-    const int ag = (int)std::min<long long>(((long long)n + AERO_WARPS - 1) / AERO_WARPS,
-                                            (long long)h->num_sms * 8);
-    rt_aerosol<<<ag, 32 * AERO_WARPS, 0, st>>>(as, h->aero, h->d_mie);
+    // a warp per task (rt_aerosol)
+    const long long tasks = (long long)n * ((L + 15) / 16) * (as.active_dust + as.cloudon);
+    const int ag = (int)std::min<long long>((tasks + AERO_WARPS - 1) / AERO_WARPS, 1 << 20);
+    if (tasks) rt_aerosol<<<ag, 32 * AERO_WARPS, 0, st>>>(as, h->aero, h->d_mie);
     CK(cudaGetLastError());
     rc = launch_all(h, sl, st, (int)n, nl, 1 << 30);
     if (rc) return rc;

@@ -11,13 +11,18 @@
 // TAUREF.  Built with --fmad=false; powers, logs, exps and DERF come from
 // include/mgcm_rt_math.h, so the results equal the CPU oracle's bit for bit.
 //
-// One warp per column.  A lane per layer applies the routines' thresholds
-// and computes the size parameters of the layers that pass them; a lane per
-// level writes every other level (prescribed dust, or the defaults, and
-// levels 1-3 and L_LEVELS+1 always); then each layer with aerosol is
-// computed across the warp: 21 lanes evaluate the DERF bin edges at once and
-// 12 lanes form the band sums (the per-layer chain of 21 DERFs was the cost
-// of a thread-per-layer form).  Every level is written exactly once.
+// One warp per family and 16 layers (32 levels) of a column.  A lane per layer
+// applies the routines' thresholds and computes the size parameters; then the
+// lanes take (layer, bin edge) items: the DERF arguments first, sorted into
+// the ones its series and its continued fraction evaluate so that a warp runs
+// one of the two on full lanes, then (layer, band) items for the band sums,
+// and last a lane per level writes every array contiguously (the layer's
+// properties, or the routines' defaults).  Bound by the FP64 work of the
+// DERFs (80 steps of the continued fraction for half of the 21 edges of a
+// layer; issue 43%).  4,050 x 24 columns of dust and ice: 381 -> 181 us
+// against going layer by layer across a column's warp -- 21 lanes for the
+// edges, both DERF branches in one warp, 12 lanes for the bands, two levels
+// written per array.
 #include "rt_aerosol.cuh"
 #include "../../include/mgcm_rt_math.h"
 
@@ -83,188 +88,150 @@ __device__ bool layer_mie(const AeroConst &K, double ma, double mcor, double nb,
     return true;
 }
 
-// The optical properties of one layer that passed the thresholds, spread
-// over the warp: lanes 0..20 evaluate the 21 DERF bin edges, lanes 0..6 /
-// 7..11 form the visible / IR band sums over the 20 bins in the routine's
-// order, for both of the layer's levels (k0 = 2l+2, k0+1; their sums are
-// the same numbers), then QEXTREF and TAUREF per level.
+constexpr int AERO_CHUNK = 16;              // layers at a time
+constexpr int AERO_EDGES = AERO_NBIN + 1;
+constexpr int AERO_BANDS = AERO_NV + AERO_NI;
+
+// One warp's shared memory.
+struct AeroWarp {
+    LayerMie lm[AERO_CHUNK];
+    double e[AERO_CHUNK * AERO_EDGES];              // DERF arguments, values, then bin weights
+    double opt[AERO_CHUNK][AERO_BANDS][3];          // QEXT, QSCAT, G per layer and band
+    unsigned short item[AERO_CHUNK * AERO_EDGES];   // DERF items: series from the front, fraction from the back
+    unsigned char layer[AERO_CHUNK];                // the chunk's layers with aerosol
+};
+
+// Layers 16q+1 .. 16q+16 of a column and their levels; with q = 0 also levels
+// 1-3 and L_LEVELS+1, which always hold the defaults.
 template <bool CLD>
-__device__ void layer_optics(int lane, const AeroConst &K, const double *__restrict__ mie, int L, int l,
-                             const double *pl, const LayerMie &m, double *tauref, double *qextref,
-                             double *qxv, double *qsv, double *gv, double *qxi, double *qsi, double *gi) {
+__device__ void layer_chunk(int lane, const AeroConst &K, const double *__restrict__ mie, int L, int q,
+                            const double *pl, const double *ma, const double *mcor, const double *nb, AeroWarp &w,
+                            double *tauref, double *qextref, double *qxv, double *qsv, double *gv, double *qxi,
+                            double *qsi, double *gi) {
     const unsigned full = 0xffffffffu;
-    const int lev1 = 2 * L + 4;
+    const int lev = 2 * L + 3, lev1 = lev + 1;
     const double GRAVc = 3.72;
     const double dev = CLD ? r4(0.3087) : r4(0.63676);
     const double dev2 = 1.0 / ((double)sqrtf(2.0f) * dev);
-    double e = 0.0;
-    if (lane <= AERO_NBIN) e = mgcm_rt_erf(mgcm_rt_ln(K.radb[lane] * m.rs_inv) * dev2);
-    const double ehi = __shfl_down_sync(full, e, 1);
-    const double surf = 0.5 * (ehi - e);   // bin `lane` (lanes 0..19)
-    // mie layout: dust [3][bin][7] vis, [3][bin][5] IR; ice [3][ratio][bin][7], [3][ratio][bin][5]
-    const bool vis = lane < AERO_NV, ir = lane >= AERO_NV && lane < AERO_NV + AERO_NI;
-    const int iw = vis ? lane : lane - AERO_NV, nb = vis ? AERO_NV : AERO_NI;
-    const double *tab;
-    size_t sq;
-    if (vis) {
-        tab = CLD ? mie + AERO_DST_SIZE + (size_t)(m.irap - 1) * AERO_NBIN * AERO_NV : mie;
-        sq = CLD ? (size_t)AERO_NRATIO * AERO_NBIN * AERO_NV : (size_t)AERO_NBIN * AERO_NV;
-    } else {
-        tab = CLD ? mie + AERO_DST_SIZE + 3 * AERO_NRATIO * AERO_NBIN * AERO_NV +
-                        (size_t)(m.irap - 1) * AERO_NBIN * AERO_NI
-                  : mie + 3 * AERO_NBIN * AERO_NV;
-        sq = CLD ? (size_t)AERO_NRATIO * AERO_NBIN * AERO_NI : (size_t)AERO_NBIN * AERO_NI;
-    }
-    double x = 0.0, sc = 0.0, g = 0.0;
-    for (int i = 0; i < AERO_NBIN; ++i) {
-        const double sf = __shfl_sync(full, surf, i);
-        if (vis || ir) {
-            x = x + sf * __ldg(tab + i * nb + iw);
-            sc = sc + sf * __ldg(tab + sq + i * nb + iw);
-            g = g + sf * __ldg(tab + 2 * sq + i * nb + iw);
+    bool on = false;
+    const int l = AERO_CHUNK * q + lane + 1;
+    if (lane < AERO_CHUNK && l <= L) on = layer_mie<CLD>(K, ma[l - 1], CLD ? mcor[l - 1] : 0.0, nb[l - 1], w.lm[lane]);
+    const unsigned mask = __ballot_sync(full, on);
+    const unsigned below = (1u << lane) - 1u;
+    if (on) w.layer[__popc(mask & below)] = (unsigned char)lane;
+    __syncwarp();
+    const int non = __popc(mask), nedge = non * AERO_EDGES;
+    // DERF arguments, sorted by the branch mgcm_rt_erf takes
+    int na = 0, nf = 0;
+    for (int i0 = 0; i0 < nedge; i0 += 32) {
+        const int i = i0 + lane;
+        bool ser = false, frac = false;
+        if (i < nedge) {
+            const int r = i / AERO_EDGES;
+            const double x = mgcm_rt_ln(K.radb[i - r * AERO_EDGES] * w.lm[w.layer[r]].rs_inv) * dev2;
+            const double ax = fabs(x);
+            ser = ax < 1.5;
+            frac = !ser && !(ax >= 6.0);
+            w.e[i] = ser || frac ? x : mgcm_rt_erf(x);
         }
+        const unsigned ms = __ballot_sync(full, ser), mf = __ballot_sync(full, frac);
+        if (ser) w.item[na + __popc(ms & below)] = (unsigned short)i;
+        if (frac) w.item[AERO_CHUNK * AERO_EDGES - 1 - nf - __popc(mf & below)] = (unsigned short)i;
+        na += __popc(ms);
+        nf += __popc(mf);
     }
-    const int k0 = 2 * l + 2;
-    if (vis || ir) {
-        const double scl = fmin(sc, r4(0.99999) * x);
-        double *X = vis ? qxv : qxi, *S = vis ? qsv : qsi, *G = vis ? gv : gi;
-        for (int k = k0; k <= k0 + 1; ++k) {
-            X[iw * lev1 + k - 1] = x;
-            S[iw * lev1 + k - 1] = scl;
-            G[iw * lev1 + k - 1] = g;
+    __syncwarp();
+    for (int i = lane; i < na; i += 32) w.e[w.item[i]] = mgcm_rt_erf(w.e[w.item[i]]);
+    for (int i = lane; i < nf; i += 32) {
+        const int j = w.item[AERO_CHUNK * AERO_EDGES - 1 - i];
+        w.e[j] = mgcm_rt_erf(w.e[j]);
+    }
+    __syncwarp();
+    // bin weights in place of the edges below them
+    for (int i0 = 0; i0 < nedge; i0 += 32) {
+        const int i = i0 + lane;
+        const double s = i + 1 < nedge ? 0.5 * (w.e[i + 1] - w.e[i]) : 0.0;
+        __syncwarp();
+        if (i < nedge) w.e[i] = s;
+        __syncwarp();
+    }
+    // band sums over the 20 bins in the routine's order (the layer's two
+    // levels have the same); mie layout: dust [3][bin][7] vis, [3][bin][5]
+    // IR; ice [3][ratio][bin][7], [3][ratio][bin][5]
+    for (int i = lane; i < non * AERO_BANDS; i += 32) {
+        const int r = i / AERO_BANDS, b = i - r * AERO_BANDS;
+        const bool vis = b < AERO_NV;
+        const int iw = vis ? b : b - AERO_NV, nbd = vis ? AERO_NV : AERO_NI, ly = w.layer[r];
+        const double *tab;
+        size_t sq;
+        if (vis) {
+            tab = CLD ? mie + AERO_DST_SIZE + (size_t)(w.lm[ly].irap - 1) * AERO_NBIN * AERO_NV : mie;
+            sq = CLD ? (size_t)AERO_NRATIO * AERO_NBIN * AERO_NV : (size_t)AERO_NBIN * AERO_NV;
+        } else {
+            tab = CLD ? mie + AERO_DST_SIZE + 3 * AERO_NRATIO * AERO_NBIN * AERO_NV +
+                            (size_t)(w.lm[ly].irap - 1) * AERO_NBIN * AERO_NI
+                      : mie + 3 * AERO_NBIN * AERO_NV;
+            sq = CLD ? (size_t)AERO_NRATIO * AERO_NBIN * AERO_NI : (size_t)AERO_NBIN * AERO_NI;
         }
+        double x = 0.0, sc = 0.0, g = 0.0;
+        const double *sf = w.e + r * AERO_EDGES;
+#pragma unroll 4
+        for (int n = 0; n < AERO_NBIN; ++n) {
+            const double f = sf[n];
+            x = x + f * __ldg(tab + n * nbd + iw);
+            sc = sc + f * __ldg(tab + sq + n * nbd + iw);
+            g = g + f * __ldg(tab + 2 * sq + n * nbd + iw);
+        }
+        w.opt[ly][b][0] = x;
+        w.opt[ly][b][1] = fmin(sc, r4(0.99999) * x);
+        w.opt[ly][b][2] = g;
     }
-    const double q6 = __shfl_sync(full, x, 5);   // QXV of L_NREFV = 6
-    if (lane < 2) {
-        const int k = k0 + lane;
+    __syncwarp();
+    auto level = [&](int k, int ly, bool act) {
+        const double q6 = act ? w.opt[ly][5][0] : 1.0;   // QXV of L_NREFV = 6
         qextref[k - 1] = q6;
-        const double mass = 100.0 * (pl[k - 1] - pl[k - 2]) / GRAVc;
-        tauref[k - 1] = m.ao * qextref[k - 1] * mass;
-    }
-}
-
-// Prescribed dust on level k (1-based): band constants, TAUREF as given.
-__device__ void prescribed_level(const AeroConst &K, int lev1, int k, const double *tin, double *tauref,
-                                 double *qextref, double *qxv, double *qsv, double *gv, double *qxi,
-                                 double *qsi, double *gi) {
-    qextref[k - 1] = K.qextv[5];
-    tauref[k - 1] = k == lev1 ? 0.0 : tin[k - 1];
-    for (int i = 0; i < AERO_NV; ++i) {
-        qxv[i * lev1 + k - 1] = K.qextv[i];
-        qsv[i * lev1 + k - 1] = K.qscatv[i];
-        gv[i * lev1 + k - 1] = K.gv[i];
-    }
-    for (int i = 0; i < AERO_NI; ++i) {
-        qxi[i * lev1 + k - 1] = K.qexti[i];
-        qsi[i * lev1 + k - 1] = K.qscati[i];
-        gi[i * lev1 + k - 1] = K.gi[i];
-    }
-}
-
-__device__ void default_level(int lev1, int k, double *tauref, double *qextref, double *qxv, double *qsv,
-                              double *gv, double *qxi, double *qsi, double *gi) {
-    qextref[k - 1] = 1.0;
-    tauref[k - 1] = 0.0;
-    for (int i = 0; i < AERO_NV; ++i) {
-        qxv[i * lev1 + k - 1] = 1.0;
-        qsv[i * lev1 + k - 1] = 1.0 * r4(0.99);
-        gv[i * lev1 + k - 1] = 0.0;
-    }
-    for (int i = 0; i < AERO_NI; ++i) {
-        qxi[i * lev1 + k - 1] = 1.0;
-        qsi[i * lev1 + k - 1] = 1.0 * r4(0.99);
-        gi[i * lev1 + k - 1] = 0.0;
-    }
+        tauref[k - 1] = act ? w.lm[ly].ao * q6 * (100.0 * (pl[k - 1] - pl[k - 2]) / GRAVc) : 0.0;
+        for (int b = 0; b < AERO_BANDS; ++b) {
+            const bool vis = b < AERO_NV;
+            const int o = (vis ? b : b - AERO_NV) * lev1 + k - 1;
+            (vis ? qxv : qxi)[o] = act ? w.opt[ly][b][0] : 1.0;
+            (vis ? qsv : qsi)[o] = act ? w.opt[ly][b][1] : 1.0 * r4(0.99);
+            (vis ? gv : gi)[o] = act ? w.opt[ly][b][2] : 0.0;
+        }
+    };
+    const int k = 4 + 2 * AERO_CHUNK * q + lane, ly = lane >> 1;
+    if (k <= lev) level(k, ly, (mask >> ly) & 1u);
+    if (q == 0 && lane < 4) level(lane < 3 ? lane + 1 : lev1, 0, false);
+    __syncwarp();   // the shared arrays are rewritten by the next chunk
 }
 
 }  // namespace
 
-constexpr int AERO_MAXL = 99;   // MGCM_RT_MAX_LAYERS
-
-__global__ void __launch_bounds__(32 * AERO_WARPS, 8)   // 64 registers
-rt_aerosol(const AeroSeg a, const AeroConst K, const double *__restrict__ mie) {
-    __shared__ LayerMie lm[AERO_WARPS][2][AERO_MAXL];
-    const unsigned full = 0xffffffffu;
+__global__ void __launch_bounds__(32 * AERO_WARPS, 6)
+rt_aerosol(const AeroSeg a, const __grid_constant__ AeroConst K, const double *__restrict__ mie) {
+    __shared__ AeroWarp ws[AERO_WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int L = a.L, lev = 2 * L + 3, lev1 = lev + 1;
-    for (long long cc = (long long)blockIdx.x * AERO_WARPS + wid; cc < a.ncol;
-         cc += (long long)gridDim.x * AERO_WARPS) {
-        const size_t c = (size_t)cc;
+    // a warp's task is one chunk of one family of a column, the dust (more
+    // layers) first
+    const int nq = (L + AERO_CHUNK - 1) / AERO_CHUNK;
+    const long long per = (long long)a.ncol * nq, tasks = per * (a.active_dust + a.cloudon);   // prescribed dust: none
+    for (long long i = (long long)blockIdx.x * AERO_WARPS + wid; i < tasks; i += (long long)gridDim.x * AERO_WARPS) {
+        const long long j = i % per;
+        const size_t c = (size_t)(j / nq);
+        const int q = (int)(j % nq);
         const double *pl = a.plev + c * lev;
-        // dust arrays (absent for prescribed dust read as band constants)
-        double *tr = nullptr, *qr = nullptr, *xv = nullptr, *sv = nullptr, *gv = nullptr;
-        double *xi = nullptr, *si = nullptr, *gi = nullptr;
-        if (a.tauref) {
-            tr = a.tauref + c * lev1;
-            qr = a.qextrefdst + c * lev1;
-            xv = a.qxvdst + c * AERO_NV * lev1;
-            sv = a.qsvdst + c * AERO_NV * lev1;
-            gv = a.gvdst + c * AERO_NV * lev1;
-            xi = a.qxidst + c * AERO_NI * lev1;
-            si = a.qsidst + c * AERO_NI * lev1;
-            gi = a.gidst + c * AERO_NI * lev1;
-        }
-        double *tc = nullptr, *qc = nullptr, *cxv = nullptr, *csv = nullptr, *cgv = nullptr;
-        double *cxi = nullptr, *csi = nullptr, *cgi = nullptr;
-        if (a.cloudon) {
-            tc = a.taurefcld + c * lev1;
-            qc = a.qextrefcld + c * lev1;
-            cxv = a.qxvcld + c * AERO_NV * lev1;
-            csv = a.qsvcld + c * AERO_NV * lev1;
-            cgv = a.gvcld + c * AERO_NV * lev1;
-            cxi = a.qxicld + c * AERO_NI * lev1;
-            csi = a.qsicld + c * AERO_NI * lev1;
-            cgi = a.gicld + c * AERO_NI * lev1;
-        }
-        // the layers that pass OPT_DST's / OPT_CLD's thresholds, a lane per layer
-        unsigned dmask[4] = {0u, 0u, 0u, 0u}, cmask[4] = {0u, 0u, 0u, 0u};
-        for (int base = 0; base < L; base += 32) {
-            const int l = base + lane + 1;
-            bool d_on = false, c_on = false;
-            if (l <= L) {
-                LayerMie m;
-                if (a.active_dust && layer_mie<false>(K, a.dust_mass[c * L + l - 1], 0.0,
-                                                      a.dust_number[c * L + l - 1], m)) {
-                    lm[wid][0][l - 1] = m;
-                    d_on = true;
-                }
-                if (a.cloudon && layer_mie<true>(K, a.ice_mass[c * L + l - 1], a.ice_core[c * L + l - 1],
-                                                 a.ice_number[c * L + l - 1], m)) {
-                    lm[wid][1][l - 1] = m;
-                    c_on = true;
-                }
-            }
-            dmask[base >> 5] = __ballot_sync(full, d_on);
-            cmask[base >> 5] = __ballot_sync(full, c_on);
-        }
-        __syncwarp();
-        // every other level: prescribed dust or the routines' defaults (levels
-        // 1-3 and L_LEVELS+1 always), a lane per level
-        const double *tin = a.tauref_in ? a.tauref_in + c * lev1 : nullptr;
-        for (int k = lane + 1; k <= lev1; k += 32) {
-            const int l = (k >= 4 && k <= lev) ? (k - 2) / 2 : 0;
-            const bool d_act = l && ((dmask[(l - 1) >> 5] >> ((l - 1) & 31)) & 1u);
-            const bool c_act = l && ((cmask[(l - 1) >> 5] >> ((l - 1) & 31)) & 1u);
-            if (!a.active_dust) {
-                if (tr) prescribed_level(K, lev1, k, tin, tr, qr, xv, sv, gv, xi, si, gi);
-            } else if (!d_act) {
-                default_level(lev1, k, tr, qr, xv, sv, gv, xi, si, gi);
-            }
-            if (a.cloudon && !c_act) default_level(lev1, k, tc, qc, cxv, csv, cgv, cxi, csi, cgi);
-        }
-        // the layers with aerosol, one at a time across the warp
-        for (int w = 0; w < 4; ++w) {
-            for (unsigned bits = dmask[w]; bits; bits &= bits - 1u) {
-                const int l = 32 * w + __ffs(bits);
-                layer_optics<false>(lane, K, mie, L, l, pl, lm[wid][0][l - 1], tr, qr, xv, sv, gv, xi, si, gi);
-            }
-            for (unsigned bits = cmask[w]; bits; bits &= bits - 1u) {
-                const int l = 32 * w + __ffs(bits);
-                layer_optics<true>(lane, K, mie, L, l, pl, lm[wid][1][l - 1], tc, qc, cxv, csv, cgv, cxi, csi,
-                                   cgi);
-            }
-        }
-        __syncwarp();   // lm is rewritten for the next column
+        if (a.active_dust && i < per)
+            layer_chunk<false>(lane, K, mie, L, q, pl, a.dust_mass + c * L, nullptr, a.dust_number + c * L, ws[wid],
+                               a.tauref + c * lev1, a.qextrefdst + c * lev1, a.qxvdst + c * AERO_NV * lev1,
+                               a.qsvdst + c * AERO_NV * lev1, a.gvdst + c * AERO_NV * lev1,
+                               a.qxidst + c * AERO_NI * lev1, a.qsidst + c * AERO_NI * lev1,
+                               a.gidst + c * AERO_NI * lev1);
+        else
+            layer_chunk<true>(lane, K, mie, L, q, pl, a.ice_mass + c * L, a.ice_core + c * L, a.ice_number + c * L,
+                              ws[wid], a.taurefcld + c * lev1, a.qextrefcld + c * lev1, a.qxvcld + c * AERO_NV * lev1,
+                              a.qsvcld + c * AERO_NV * lev1, a.gvcld + c * AERO_NV * lev1, a.qxicld + c * AERO_NI * lev1,
+                              a.qsicld + c * AERO_NI * lev1, a.gicld + c * AERO_NI * lev1);
     }
 }
 

@@ -29,6 +29,6 @@ struct AeroSeg {
 };
 
 constexpr int AERO_WARPS = 4;   // columns (warps) per CTA of rt_aerosol
-__global__ void rt_aerosol(const AeroSeg a, const AeroConst K, const double *__restrict__ mie);
+__global__ void rt_aerosol(const AeroSeg a, const __grid_constant__ AeroConst K, const double *__restrict__ mie);
 
 }  // namespace mgcm
