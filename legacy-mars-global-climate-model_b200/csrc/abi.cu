@@ -56,6 +56,10 @@ __global__ void rt_fp64_solve_vis(const SegTable *__restrict__ st, int col_begin
                                   const double *__restrict__ ktab, const __grid_constant__ RtConst K,
                                   const int *__restrict__ list, const unsigned int *count,
                                   double *__restrict__ fl, double *__restrict__ sc);
+__global__ void rt_vis_dense(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
+                             unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ kv,
+                             const __grid_constant__ RtConst K, double *__restrict__ fl, double *__restrict__ sc,
+                             unsigned long long *nsys);
 __global__ void rt_ir_dense(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                             unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ ktab,
                             const __grid_constant__ RtConst K, double *__restrict__ fl, double *__restrict__ sc,
@@ -581,11 +585,15 @@ int configure_kernels(int device) {
     // the solvers use no shared memory: the whole unified L1 goes to the
     // per-system arrays
     for (const void *f : {(const void *)rt_fp64_solve_vis, (const void *)rt_ir_dense,
-                          (const void *)rt_mixed_solve_vis})
+                          (const void *)rt_mixed_solve_vis, (const void *)rt_vis_dense})
         CK(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0));
     done[device] = true;
     return MGCM_RT_OK;
 }
+
+// FP64 chunks of up to this many columns per SM screen and solve their visible
+// systems in one kernel (rt_vis_dense).
+constexpr int DENSE_V_COLS_PER_SM = 3;
 
 size_t pipe_bytes_per_col(int max_nl, size_t *stride_out = nullptr) {
     const size_t stride = (col_smem_bytes(max_nl, false) + 255) / 256 * 256;
@@ -681,9 +689,13 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         };
         if (dense_ir)
             if (const int frc = fork()) return frc;
-        (mixed ? rt_fp64_screen<true> : rt_fp64_screen<false>)<<<g1, SCREEN_THREADS, 0, dense_ir ? vst : st>>>(
-            sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_kv, h->d_ki, h->K, list_v, list_i, counts, sl.d_nsys,
-            mixed ? h->d_kvf : nullptr, groups);
+        // small calls screen and solve the visible systems in one kernel too
+        const int dense_v = dense_ir && !mixed && (c1 - c0) <= DENSE_V_COLS_PER_SM * h->num_sms;
+        const int dense = (dense_ir ? DENSE_I : 0) | (dense_v ? DENSE_V : 0);
+        if (!dense_v)
+            (mixed ? rt_fp64_screen<true> : rt_fp64_screen<false>)<<<g1, SCREEN_THREADS, 0, dense_ir ? vst : st>>>(
+                sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_kv, h->d_ki, h->K, list_v, list_i, counts, sl.d_nsys,
+                mixed ? h->d_kvf : nullptr, groups);
         if (!dense_ir)
             if (const int frc = fork()) return frc;
         // MIXED: FP32 visible opacities; the IR family is FP64 in both modes.
@@ -723,7 +735,10 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
             else MGCM_QUAD(13);
 #undef MGCM_QUAD
         } else {
-            if (mixed)
+            if (dense_v)
+                rt_vis_dense<<<((c1 - c0) * NSYS_V + 127) / 128, 128, 0, vst>>>(
+                    sl.d_segs, c0, c1, max_nl, blocks, stride, h->d_kv, h->K, fl_v, sc_v, sl.d_nsys);
+            else if (mixed)
                 rt_mixed_solve_vis<<<g2, 128, 0, vst>>>(sl.d_segs, c0, max_nl, blocks, stride, h->d_kvf, h->d_kv,
                                                         h->K, list_v, counts, fl_v, sc_v);
             else
@@ -742,10 +757,10 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
             const RtConst &K = h->K;
             void *args[] = {(void *)&segs, (void *)&c0, (void *)&c1, (void *)&max_nl, (void *)&blocks,
                             (void *)&stride, (void *)&K, (void *)&fl_v, (void *)&sc_v, (void *)&fl_i,
-                            (void *)&sc_i, (void *)&dense_ir};
+                            (void *)&sc_i, (void *)&dense};
             CK(cudaLaunchKernel(reduce_kernel(rb), dim3(g3), dim3(REDUCE_THREADS), args, rsm, st));
         }
-        nk += 5;
+        nk += dense_v ? 4 : 5;
         CK(cudaGetLastError());
     }
     return MGCM_RT_OK;
@@ -1635,6 +1650,7 @@ mgcm_rt_handle *mgcm_rt_create(const mgcm_rt_config *cfg, const char *data_dir, 
         size_t need = 0, cur = 0;
         for (const void *f : {(const void *)rt_fp64_kernel, (const void *)rt_fp64_solve_vis,
                               (const void *)rt_ir_dense, (const void *)rt_mixed_solve_vis,
+                              (const void *)rt_vis_dense,
                               (const void *)rt_fp64_screen<false>, (const void *)rt_fp64_screen<true>}) {
             cudaFuncAttributes fa{};
             if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) { *status = MGCM_RT_ECUDA; return nullptr; }

@@ -28,6 +28,9 @@ __host__ __device__ constexpr int group_end(int w) {
                                       : NSYS);
 }
 
+// Families whose systems sit at fixed list positions of their columns.
+constexpr int DENSE_I = 1, DENSE_V = 2;
+
 // Layers per lane of the four-lane solvers for a largest NL (0: NL > 52,
 // the one-thread-per-system solvers run).
 __host__ __device__ constexpr int quad_r_for(int nl) {

@@ -221,6 +221,38 @@ rt_fp64_solve_vis(const SegTable *__restrict__ st, int col_begin, int max_nl,
     }
 }
 
+// K1 and K2 in one for small calls: screen and solve the visible systems of a
+// chunk, one thread per system, at list position (column) * 119 + system.
+// Half of a day column's systems pass the screen, so most warps carry idle
+// lanes through the solve; but where all of them are resident at once that
+// costs nothing, and the call is spared a kernel and a second pass A in its
+// longest chain of dependent kernels.  FP64 only: MIXED solves contract
+// multiply-adds (rt_mixed.cu), and a column's result must not depend on the
+// size of the call.  60 / 200 / 400 x 24 columns: 191 / 198 / 229 -> 163 / 179 /
+// 220 us; 800: 269 -> 311, so three columns per SM is the limit.
+__global__ void __launch_bounds__(128, MGCM_VIS_SOLVE_MINB)
+rt_vis_dense(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
+             unsigned char *__restrict__ blocks, size_t stride, const double *__restrict__ kv,
+             const __grid_constant__ RtConst K, double *__restrict__ fl,
+             double *__restrict__ sc, unsigned long long *nsys) {
+    SolveLocal w;
+    unsigned int nsolved = 0;
+    const int n = (col_end - col_begin) * NSYS_V;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int cc = i / NSYS_V, g = col_begin + cc;
+        const SegDev &sg = st->seg[find_seg(st, g)];
+        const int c = g - sg.col0;
+        if (!(sg.acosz[c] >= R4(1.0e-5))) continue;
+        double *row = fl + row_base(i, max_nl);
+        nsolved += fast_vis<false, true>(sg, c, i - cc * NSYS_V, blocks + (size_t)cc * stride, max_nl, K, kv, nullptr, w, row,
+                                       row + (size_t)max_nl * ROW_BLK, sc + sc_base(i));
+    }
+    if (nsys) {
+        for (int o = 16; o > 0; o >>= 1) nsolved += __shfl_down_sync(0xffffffffu, nsolved, o);
+        if ((threadIdx.x & 31) == 0 && nsolved) atomicAdd(nsys, (unsigned long long)nsolved);
+    }
+}
+
 // K2: screen and solve the IR systems of a chunk, one thread per system, at
 // list position (column in the chunk) * 85 + system.  Nine tenths of them
 // pass TLIMIT, so a list of the kept ones would fill 8% more lanes but take
@@ -297,8 +329,8 @@ template __global__ void rt_quad_solve<false, 13>(QUAD_ARGS);
 // the system at position p is fl[row_base(p) + 32 k] (k < max_nl: upward
 // midpoint flux of layer k+1; max_nl + k: downward), scalar q
 // sc[sc_base(p) + 32 q].  A column's kept systems sit in ascending (band,
-// Gauss) order, in one run of positions per screening group (visible) or at
-// 85 positions a column (rt_ir_dense).
+// Gauss) order, in one run of positions per screening group or, per `dense`,
+// at 119 (DENSE_V, rt_vis_dense) and 85 (DENSE_I, rt_ir_dense) positions a column.
 //
 // The rows of up to 16 systems at a time come into shared memory with
 // asynchronous copies, half a warp along the systems for the upward and half
@@ -381,7 +413,7 @@ __global__ void __launch_bounds__(32)
 rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                unsigned char *__restrict__ blocks, size_t stride, const __grid_constant__ RtConst K,
                const double *__restrict__ fl_v, const double *__restrict__ sc_v,
-               const double *__restrict__ fl_i, const double *__restrict__ sc_i, int dense_ir) {
+               const double *__restrict__ fl_i, const double *__restrict__ sc_i, int dense) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x;
     RedSys *sys = reinterpret_cast<RedSys *>(smem_raw);
@@ -435,7 +467,9 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
                     const int base = __shfl_sync(0xffffffffu, gbase, vis ? w : 4 + w);
                     const int before = __popc(m & ((1u << lane) - 1u));
                     if ((m >> lane) & 1u)
-                        sys[nrow + before].pos = !vis && dense_ir ? (g - col_begin) * NSYS_I + 32 * w + lane : base + before;
+                        sys[nrow + before].pos = dense & (vis ? DENSE_V : DENSE_I)
+                                                     ? (g - col_begin) * (vis ? NSYS_V : NSYS_I) + 32 * w + lane
+                                                     : base + before;
                     nrow += __popc(m);
                 }
                 warp_multipliers(mine, vis, K, sys);

@@ -422,20 +422,12 @@ struct VisPassA {
     }
 };
 
-// Screen of system t of a day column: DETAU, CUMTAUV and the TLIMIT decision
-// (code/sfluxv.f90:60-75); true when the system is to be solved.
-template <bool F32>
-__device__ __forceinline__ bool fast_vis_screen(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
-                                                const ColSmem &s, const RtConst &K, const double *__restrict__ kv,
-                                                const float *__restrict__ kvf, SolveLocal &w,
-                                                unsigned int &nsolved) {
-    VisPassA<false, F32> a;
-    a.run(sg, t, s, kv, kvf, w);
+// The TLIMIT decision of system t of a day column after its pass A, with
+// DETAU and CUMTAUV (code/sfluxv.f90:60-75); true when it is to be solved.
+template <class PassA>
+__device__ __forceinline__ bool vis_decision(const PassA &a, const SegDev &sg, int c, int t, const ColSmem &s,
+                                             const RtConst &K) {
     const int nb = t / D_NG, ng = t - nb * D_NG;
-    if (a.odd) {
-        nsolved += general_vis<1, F32>(sg, c, t, block, max_nl, K, kv, kvf, w.g, nullptr, nullptr, nullptr);
-        return s.skip[t] == 0;
-    }
     const size_t o = (size_t)c * NSYS_V + nb + D_NV * ng;
     sg.cumtauv[o] = a.tclev;
     if (ng < D_NG - 1 && K.fzerov[nb] >= R4(0.99)) {
@@ -445,13 +437,30 @@ __device__ __forceinline__ bool fast_vis_screen(const SegDev &sg, int c, int t, 
     sg.detau[o] = a.tau;
     const bool skip = ng < D_NG - 1 && a.taugsurf < TLIMITS;
     s.skip[t] = skip ? 1 : 0;
-    nsolved += skip ? 0 : 1;
     return !skip;
 }
 
-// Solve of a kept visible system.
+// Screen of system t of a day column; true when it is to be solved.
 template <bool F32>
-__device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
+__device__ __forceinline__ bool fast_vis_screen(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
+                                                const ColSmem &s, const RtConst &K, const double *__restrict__ kv,
+                                                const float *__restrict__ kvf, SolveLocal &w,
+                                                unsigned int &nsolved) {
+    VisPassA<false, F32> a;
+    a.run(sg, t, s, kv, kvf, w);
+    if (a.odd) {
+        nsolved += general_vis<1, F32>(sg, c, t, block, max_nl, K, kv, kvf, w.g, nullptr, nullptr, nullptr);
+        return s.skip[t] == 0;
+    }
+    const bool keep = vis_decision(a, sg, c, t, s, K);
+    nsolved += keep ? 1 : 0;
+    return keep;
+}
+
+// Solve of a visible system the screen kept; with DENSE of any system of a day
+// column, the decision taken after pass A.  Returns whether it was solved.
+template <bool F32, bool DENSE = false>
+__device__ __forceinline__ bool fast_vis(const SegDev &sg, int c, int t, unsigned char *block, int max_nl,
                                          const RtConst &K, const double *__restrict__ kv,
                                          const float *__restrict__ kvf, SolveLocal &w, double *fmp, double *fmm,
                                          double *sc) {
@@ -460,6 +469,13 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
     const double u0 = sg.acosz[c], rsf = sg.als[c], f0pi = sg.sol[nb];
     VisPassA<true, F32> a;
     a.run(sg, t, s, kv, kvf, w);
+    if (DENSE) {
+        if (a.odd) {
+            if (!general_vis<1, F32>(sg, c, t, block, max_nl, K, kv, kvf, w.g, nullptr, nullptr, nullptr)) return false;
+        } else if (!vis_decision(a, sg, c, t, s, K)) {
+            return false;
+        }
+    }
     // u0 in [2^-30, 2^30), the band's sun 0 or in [2^-60, 2^60)
     bool odd = a.odd || hi32(u0) - 0x3e100000u >= 0x03c00000u || (f0pi != 0.0 && hi32(f0pi) - 0x3c300000u >= 0x07800000u);
     if (!odd) {
@@ -559,10 +575,11 @@ __device__ __forceinline__ void fast_vis(const SegDev &sg, int c, int t, unsigne
                 if (n == NL) sc[2 * ROW_BLK] = m;
                 fmm[(size_t)(n - 1) * ROW_BLK] = m + u0 * f0pi * et;
             }
-            return;
+            return true;
         }
     }
     general_vis<2, F32>(sg, c, t, block, max_nl, K, kv, kvf, w.g, fmp, fmm, sc);
+    return true;
 }
 
 }  // namespace fp64
