@@ -22,12 +22,12 @@ namespace fp64 {
 // a thread indexes them with one register, in 16-byte accesses: the rows 2l-1
 // and 2l of DSOLVER (AS, DS) and
 //   IR       DTAUKI of the layer's two levels;
-//   visible  (W0, DTAU), then (LAMDA, GAMA); TAU at the top and the middle; (AM, AP).
+//   visible  W0, DTAU; TAU at the top and the middle.
 struct alignas(16) IrSlot {
     double2 odd, even, pair;
 };
 struct alignas(16) VisSlot {
-    double2 odd, even, pair, depth, src;
+    double2 odd, even, pair, depth;
 };
 union SolveLocal {
     SysLocal g;   // the general solve's
@@ -483,25 +483,29 @@ __device__ __forceinline__ bool fast_vis(const SegDev &sg, int c, int t, unsigne
         const double rcp_u0 = rcp_n(u0), rcp_u02 = 1.0 / (u0 * u0);
         const double s3 = (double)sqrtf(3.0f), s3h = (double)(sqrtf(3.0f) * 0.5f);
         const double bsurf = rsf * u0 * f0pi * beam(a.tau, u0, rcp_u0);
-        // pass C; pair becomes (LAMDA, GAMA), src = (AM, AP)
-        auto coef = [&](int l, double2 p, double cb, double et_top, double et_bot) {
-            Lay y;
-            const double w0 = p.x;
+        // LAMDA, GAMA, AM, AP of a layer (code/gfluxv.f90:108-150).  Passes C
+        // and D both evaluate them: cheaper than 32 more bytes per layer
+        // through local memory.
+        auto lay4 = [&](double w0, double cb, double &lam, double &gama, double &am, double &ap) {
             const double g1 = s3h * (2.0 - w0 * (1.0 + cb));
             const double g2 = (s3 * w0 * 0.5) * (1.0 - cb);
             const double g3 = 0.5 * (1.0 - s3 * cb * u0);
             const double l2 = g1 * g1 - g2 * g2;
             odd |= hi32(l2) - 0x2d300000u >= 0x25800000u || out_of_range(g2);
-            const double lam = sqrt_n(l2);
-            y.gama = quot(g1 - lam, g2, rcp_s(g2));
+            lam = sqrt_n(l2);
+            gama = quot(g1 - lam, g2, rcp_s(g2));
             const double g4 = 1.0 - g3;
             double denom = lam * lam - rcp_u02;
             if (denom == 0.0) denom = R4(1.E-10);
             const double rd = rcp_s(denom);
-            const double am = quot(f0pi * w0 * (g4 * (g1 + rcp_u0) + g2 * g3), denom, rd);
-            const double ap = quot(f0pi * w0 * (g3 * (g1 - rcp_u0) + g2 * g4), denom, rd);
-            w.vis[l].pair = make_double2(lam, y.gama);
-            w.vis[l].src = make_double2(am, ap);
+            am = quot(f0pi * w0 * (g4 * (g1 + rcp_u0) + g2 * g3), denom, rd);
+            ap = quot(f0pi * w0 * (g3 * (g1 - rcp_u0) + g2 * g4), denom, rd);
+        };
+        // pass C
+        auto coef = [&](double2 p, double cb, double et_top, double et_bot) {
+            Lay y;
+            double lam, am, ap;
+            lay4(p.x, cb, lam, y.gama, am, ap);
             y.cpm1 = ap * et_top;
             y.cmm1 = am * et_top;
             y.cp = ap * et_bot;
@@ -510,7 +514,7 @@ __device__ __forceinline__ bool fast_vis(const SegDev &sg, int c, int t, unsigne
             return y;
         };
         double et_bot = beam(a.tau, u0, rcp_u0), et_top = beam(w.vis[NL].depth.x, u0, rcp_u0);
-        Lay hi = coef(NL, w.vis[NL].pair, lay->cbs, et_top, et_bot);
+        Lay hi = coef(w.vis[NL].pair, lay->cbs, et_top, et_bot);
         double as, ds;
         bottom_row_v(hi, bsurf, rsf, as, ds);
         w.vis[NL].even = make_double2(as, ds);
@@ -528,7 +532,7 @@ __device__ __forceinline__ bool fast_vis(const SegDev &sg, int c, int t, unsigne
             et_top = beam(d, u0, rcp_u0);
             --lay;
             if (n > 1) prefetch_l1(&lay[-1].cbs);
-            const Lay lo = coef(n, cur, lay->cbs, et_top, et_bot);
+            const Lay lo = coef(cur, lay->cbs, et_top, et_bot);
             double ao, dd;
             fast_rows(lo, hi, as, ds, ao, dd, odd);
             w.vis[n + 1].odd = make_double2(ao, dd);
@@ -544,18 +548,22 @@ __device__ __forceinline__ bool fast_vis(const SegDev &sg, int c, int t, unsigne
         if (!odd) {
             // pass D
             double xprev = 0.0;
-            double2 n1 = w.vis[1].odd, n2 = w.vis[1].even, nl = w.vis[1].pair, ns = w.vis[1].src, nt = w.vis[1].depth;
+            double2 n1 = w.vis[1].odd, n2 = w.vis[1].even, nt = w.vis[1].depth;
+            double nw = w.vis[1].pair.x;
 #pragma unroll 1
             for (int n = 1; n <= NL; ++n) {
                 const double2 r1 = n1, r2 = n2, t2 = nt;
-                const double lam = nl.x, gama = nl.y, am = ns.x, ap = ns.y;
+                const double w0 = nw;
                 if (n < NL) {
                     n1 = w.vis[n + 1].odd;
                     n2 = w.vis[n + 1].even;
-                    nl = w.vis[n + 1].pair;
-                    ns = w.vis[n + 1].src;
+                    nw = w.vis[n + 1].pair.x;
                     nt = w.vis[n + 1].depth;
+                    prefetch_l1(&lay[1].cbs);
                 }
+                double lam, gama, am, ap;
+                lay4(w0, lay->cbs, lam, gama, am, ap);
+                ++lay;
                 const double xa = n == 1 ? r1.y : r1.y - r1.x * xprev;
                 const double xb = r2.y - r2.x * xa;
                 xprev = xb;
