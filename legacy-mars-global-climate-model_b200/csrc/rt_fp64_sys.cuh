@@ -13,12 +13,12 @@ constexpr double PI_D = 3.1415926535897932;
 constexpr double TLIMITS = 1.0e-3;
 constexpr double TLIMITI = 5.0e-3;
 
-// Resident CTAs per SM (128 threads) asked of the solve kernels: 64 registers
-// for the IR solve, 72 for the visible ones.  64,800 x 24 FP64 call: IR at 5 /
-// 6 / 7 / 8 CTAs 10.59 / 10.54 / 10.34 / 10.29 ms, visible at 6 / 7 / 8
-// 10.49 / 10.34 / 10.46 ms.
+// Resident CTAs per SM (128 threads) asked of the solve kernels: 72 registers.
+// 64,800 x 24 FP64 calls back to back, at the 1 kW power limit: IR at 6 / 7 /
+// 8 CTAs 9.39 / 9.40 / 9.52 ms (8 spill more, which costs power), 32,400 x 48
+// 12.15 / 11.84 / 11.95 ms; visible at 6 / 7 9.54 / 9.52 ms.
 #ifndef MGCM_IR_SOLVE_MINB
-#define MGCM_IR_SOLVE_MINB 8
+#define MGCM_IR_SOLVE_MINB 7
 #endif
 #ifndef MGCM_VIS_SOLVE_MINB
 #define MGCM_VIS_SOLVE_MINB 7   // the FP64 and the MIXED visible solve
