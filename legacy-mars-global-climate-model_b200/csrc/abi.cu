@@ -81,9 +81,8 @@ __global__ void rt_mixed_solve_vis(const SegTable *__restrict__ st, int col_begi
                                    const __grid_constant__ RtConst K, const int *__restrict__ list,
                                    const unsigned int *count, double *__restrict__ fl,
                                    double *__restrict__ sc);
-size_t reduce_smem_bytes(int max_nl);
+size_t reduce_smem_bytes(int max_nl, int warps);
 const void *reduce_kernel(int rb);
-constexpr int REDUCE_THREADS = 32;   // rt_fp64_reduce: a warp, and CTA, per column
 constexpr int STAGE_THREADS = 256, SCREEN_THREADS = 128;
 int reduce_rows_per_chunk();
 __global__ void rt_dsolflux_kernel(int ncol, const double *__restrict__ sol,
@@ -298,7 +297,7 @@ struct Slot {
     uint32_t *d_status = nullptr, *h_status = nullptr;
     unsigned long long *d_nsys = nullptr, *h_nsys = nullptr;
     Arena stage, pipe, aero;   // aero: per-level aerosol arrays of tracer jobs
-    int occ_nl = 0, occ_rb = 0, occ_stage = 1, occ_screen = 1, occ_solve = 1, occ_quad = 1, occ_reduce = 1;
+    int occ_nl = 0, occ_rb = 0, occ_rw = 0, occ_stage = 1, occ_screen = 1, occ_solve = 1, occ_quad = 1, occ_reduce = 1;
     bool busy = false;
     Job job;
     int kernels = 0;
@@ -638,11 +637,23 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
     double *sc_i = reinterpret_cast<double *>(take(r_i * 32));
     unsigned int *counts = reinterpret_cast<unsigned int *>(take(256));
     const int rb = sl.tune.rb > 0 ? sl.tune.rb : reduce_rows_per_chunk();
-    const size_t rsm = reduce_smem_bytes(max_nl);
+    // reduce: a CTA per column, of one warp; of two, a family each, where all
+    // columns are resident even so (60 / 200 / 400 / 592 x 24 columns: 167 / 182 /
+    // 222 / 247 -> 155 / 169 / 210 / 238 us a call; 540 x 48, not all resident:
+    // 509 -> 520)
+    int rw = 1;
+    if (chunk <= 4 * h->num_sms) {
+        int two = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, reduce_kernel(rb), 64, reduce_smem_bytes(max_nl, 2));
+        // (the carve-out preference, half of the shared memory, halves it)
+        if (chunk <= std::max(two / 2, 1) * h->num_sms) rw = 2;
+    }
+    const size_t rsm = reduce_smem_bytes(max_nl, rw);
     const bool mixed = h->cfg.precision == MGCM_RT_MIXED;
-    if (sl.occ_nl != max_nl || sl.occ_rb != rb) {
+    if (sl.occ_nl != max_nl || sl.occ_rb != rb || sl.occ_rw != rw) {
         sl.occ_nl = max_nl;
         sl.occ_rb = rb;
+        sl.occ_rw = rw;
         int a = 1, b = 1, c = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, mixed ? rt_fp64_screen<true> : rt_fp64_screen<false>,
                                                       SCREEN_THREADS, 0);
@@ -657,7 +668,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
         else if (qr == 10) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qo, rt_quad_solve<false, 10>, 128, 0);
         else if (qr == 13) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qo, rt_quad_solve<false, 13>, 128, 0);
         sl.occ_quad = std::max(qo, 1);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, reduce_kernel(rb), REDUCE_THREADS, rsm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, reduce_kernel(rb), 32 * rw, rsm);
         sl.occ_screen = std::max(a, 1);
         sl.occ_solve = std::max(b, 1);
         sl.occ_reduce = std::max(c, 1);
@@ -764,7 +775,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
             void *args[] = {(void *)&segs, (void *)&c0, (void *)&c1, (void *)&max_nl, (void *)&blocks,
                             (void *)&stride, (void *)&K, (void *)&fl_v, (void *)&sc_v, (void *)&fl_i,
                             (void *)&sc_i, (void *)&dense};
-            CK(cudaLaunchKernel(reduce_kernel(rb), dim3(g3), dim3(REDUCE_THREADS), args, rsm, st));
+            CK(cudaLaunchKernel(reduce_kernel(rb), dim3(g3), dim3(32 * rw), args, rsm, st));
         }
         nk += dense_v ? 4 : 5;
         CK(cudaGetLastError());

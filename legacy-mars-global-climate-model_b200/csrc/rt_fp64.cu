@@ -352,15 +352,14 @@ struct alignas(16) RedSys {
     int pos, fac;
 };
 
-// Shared memory of one warp (= CTA): one family's kept systems, FMNET per
-// level of both families and the two factors of the heating rate, the top
-// values, and the staged rows: NL + 2 items, upward and downward.
-__host__ __device__ inline size_t red_fixed_bytes(int max_nl) {
-    const size_t b = (size_t)NSYS_V * sizeof(RedSys) + (size_t)(4 * (max_nl + 1) + 2) * 8;
-    return (b + 15) / 16 * 16;
+// Shared memory of a CTA: FMNET per level of both families, the two factors
+// of the heating rate and the top values; then per warp one family's kept
+// systems and the staged rows: NL + 2 items, upward and downward.
+__host__ __device__ inline size_t red_col_bytes(int max_nl) {
+    return ((size_t)(4 * (max_nl + 1) + 2) * 8 + 15) / 16 * 16;
 }
 __host__ __device__ inline size_t red_warp_bytes(int max_nl) {
-    return red_fixed_bytes(max_nl) + (size_t)2 * (max_nl + 2) * RED_PITCH * 8;
+    return (size_t)NSYS_V * sizeof(RedSys) + (size_t)2 * (max_nl + 2) * RED_PITCH * 8;
 }
 
 // Multipliers of one family of a column, one lane per band: `mine` holds, on
@@ -409,17 +408,19 @@ __device__ __forceinline__ void copy8_async(double *dst, const double *src) {
 }
 
 template <int RB>   // systems whose staged values are read before they are summed
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(64)
 rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int max_nl,
                unsigned char *__restrict__ blocks, size_t stride, const __grid_constant__ RtConst K,
                const double *__restrict__ fl_v, const double *__restrict__ sc_v,
                const double *__restrict__ fl_i, const double *__restrict__ sc_i, int dense) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x;
-    RedSys *sys = reinterpret_cast<RedSys *>(smem_raw);
-    double *fmv = reinterpret_cast<double *>(sys + NSYS_V), *fmi = fmv + max_nl + 1;   // [1..NL]
+    // one warp per column, or two with a family each (small calls)
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const bool two = blockDim.x > 32;
+    double *fmv = reinterpret_cast<double *>(smem_raw), *fmi = fmv + max_nl + 1;   // [1..NL]
     double *pnl = fmi + max_nl + 1, *den = pnl + max_nl + 1, *misc = den + max_nl + 1;
-    double *buf = reinterpret_cast<double *>(smem_raw + red_fixed_bytes(max_nl));
+    RedSys *sys = reinterpret_cast<RedSys *>(smem_raw + red_col_bytes(max_nl) + wid * red_warp_bytes(max_nl));
+    double *buf = reinterpret_cast<double *>(sys + NSYS_V);
 
     for (int g = col_begin + blockIdx.x; g < col_end; g += gridDim.x) {
         const SegDev &sg = st->seg[find_seg(st, g)];
@@ -447,7 +448,7 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
         const int gbase = lane < SCREEN_GROUPS ? s.meta[2 * lane] : 0;   // list positions of the groups
         // what the heating rates need besides the fluxes (code/comp3.f:765-771)
         const double *plev = sg.plev + (size_t)c * LEV;
-        for (int l = 1 + lane; l <= NL; l += 32) {
+        for (int l = 1 + threadIdx.x; l <= NL; l += blockDim.x) {
             const int k = 2 * l;
             const double ptrop = sg.ptrop;
             const double ym = k == 2 ? ptrop * 100.0 / 3.72 : (plev[k + 1 - 1] - plev[k - 1 - 1]) * 100.0 / 3.72;
@@ -455,7 +456,7 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
             pnl[l] = sg.sigma[k - 1] * (sg.pcol[c] - ptrop) + ptrop;
             den[l] = 735.94 * ym * om;
         }
-        for (int fam = 0; fam < 2; ++fam) {
+        for (int fam = two ? wid : 0; fam < (two ? wid + 1 : 2); ++fam) {
             const bool vis = fam == 0;
             const unsigned mine = vis ? mine_v : mine_i;
             // the family's kept systems in order (none at night for the
@@ -564,7 +565,8 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
             __syncwarp();   // sys is rewritten by the next family
         }
         // divergences and heating rates (code/comp3.f:677-681,735-738,765-771)
-        for (int l = 1 + lane; l <= NL; l += 32) {
+        if (two) __syncthreads();
+        for (int l = 1 + threadIdx.x; l <= NL; l += blockDim.x) {
             const double sun = day ? (l == 1 ? fmv[1] - misc[0] : fmv[l] - fmv[l - 1]) : 0.0;
             const double irt = l == 1 ? fmi[1] - misc[1] : fmi[l] - fmi[l - 1];
             const double sunlte = sun * 2.2e4 * pnl[l] / (1.0 + 2.2e4 * pnl[l]);
@@ -573,7 +575,9 @@ rt_fp64_reduce(const SegTable *__restrict__ st, int col_begin, int col_end, int 
             sg.irtotal[o] = irt;
             sg.qrad[o] = (sunlte + irt) / den[l];
         }
-        __syncwarp();   // the shared arrays are rewritten by the next column
+        // the shared arrays are rewritten by the next column
+        if (two) __syncthreads();
+        else __syncwarp();
     }
 }
 
@@ -587,8 +591,8 @@ template __global__ void rt_fp64_reduce<4>(REDUCE_ARGS);
 template __global__ void rt_fp64_reduce<8>(REDUCE_ARGS);
 #undef REDUCE_ARGS
 
-// Shared memory of a reduce CTA (one warp).
-size_t reduce_smem_bytes(int max_nl) { return red_warp_bytes(max_nl); }
+// Shared memory of a reduce CTA of `warps` warps.
+size_t reduce_smem_bytes(int max_nl, int warps) { return red_col_bytes(max_nl) + warps * red_warp_bytes(max_nl); }
 // Systems whose staged values a lane reads before it sums them, by default.
 int reduce_rows_per_chunk() { return 4; }
 // The reduce kernel of a launch, rb in {1, 2, 4, 8} (other values round down).
@@ -606,32 +610,55 @@ const void *reduce_kernel(int rb) {
 // put the 119 terms of each into shared memory, then a thread per column
 // adds them in the reference's order (band by band; a term of DETAU > 5
 // counts as +0).  Night columns are not read.
+static_assert(NSYS_V <= 128, "a thread per element sets up the tables");
 constexpr int DSOL_COLS = 32, DSOL_THREADS = 128, DSOL_ROW = NSYS_V + 2;   // odd pitch: no bank conflicts
-constexpr int DSOL_MLP = 10;   // DETAU values a thread has in flight
+constexpr int DSOL_MLP = 8;   // DETAU values a thread has in flight
 
 __global__ void __launch_bounds__(DSOL_THREADS)
 rt_dsolflux_kernel(int ncol, const double *__restrict__ sol, const double *__restrict__ acosz,
                    const double *__restrict__ detau, const double *__restrict__ dndiffv,
                    double *__restrict__ dnvflux, const RtConst K) {
     __shared__ double term[DSOL_COLS * DSOL_ROW], u0s[DSOL_COLS], rcp[DSOL_COLS];
+    __shared__ int day[DSOL_COLS], nday;   // the tile's day columns
+    // per element of DETAU's (Gauss, band) order: SOL, the two weights in the
+    // reference's order, and the place in the summation order
+    __shared__ double sl[NSYS_V], wa[NSYS_V], wb[NSYS_V];
+    __shared__ int at[NSYS_V];
     const int t = threadIdx.x, c0 = blockIdx.x * DSOL_COLS, nc = min(DSOL_COLS, ncol - c0);
-    if (t < nc) {
-        u0s[t] = acosz[c0 + t];
-        rcp[t] = 1.0 / u0s[t];
+    if (t < 32) {
+        const double u0 = t < nc ? acosz[c0 + t] : 0.0;
+        const bool on = u0 >= R4(1.0e-5);
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) {
+            const int q = __popc(m & ((1u << t) - 1u));
+            day[q] = t;
+            u0s[q] = u0;
+            rcp[q] = 1.0 / u0;
+        }
+        if (t == 0) nday = __popc(m);
+        if (t < nc && !on) dnvflux[c0 + t] = dndiffv[c0 + t] + 0.0;
+    }
+    if (t < NSYS_V) {
+        const int ng = t / D_NV, nw = t - ng * D_NV;
+        sl[t] = sol[nw];
+        wa[t] = ng < D_NG - 1 ? K.gweight[ng] : K.fzerov[nw];
+        wb[t] = ng < D_NG - 1 ? 1.0 - K.fzerov[nw] : 1.0;
+        at[t] = nw * D_NG + ng;
     }
     __syncthreads();
-    for (int i0 = t; i0 < nc * NSYS_V; i0 += DSOL_MLP * DSOL_THREADS) {
+    const int n = nday * NSYS_V;
+    for (int i0 = t; i0 < n; i0 += DSOL_MLP * DSOL_THREADS) {
         double dv[DSOL_MLP];
 #pragma unroll
         for (int q = 0; q < DSOL_MLP; ++q) {
-            const int i = i0 + q * DSOL_THREADS;
-            dv[q] = i < nc * NSYS_V && u0s[i / NSYS_V] >= R4(1.0e-5) ? detau[(size_t)c0 * NSYS_V + i] : 6.0;
+            const int i = i0 + q * DSOL_THREADS, c = i / NSYS_V;
+            dv[q] = i < n ? detau[(size_t)(c0 + day[c]) * NSYS_V + (i - c * NSYS_V)] : 6.0;
         }
 #pragma unroll
         for (int q = 0; q < DSOL_MLP; ++q) {
             const int i = i0 + q * DSOL_THREADS;
-            if (i >= nc * NSYS_V) break;
-            const int c = i / NSYS_V, e = i - c * NSYS_V, ng = e / D_NV, nw = e - ng * D_NV;
+            if (i >= n) break;
+            const int c = i / NSYS_V, e = i - c * NSYS_V;
             const double u0 = u0s[c], d = dv[q];
             double v = 0.0;
             if (d <= 5.0) {
@@ -640,18 +667,16 @@ rt_dsolflux_kernel(int ncol, const double *__restrict__ sol, const double *__res
                 const bool usual = d > 0x1p-300 && u0 < 0x1p300;
                 const double x = usual ? -quot(d, u0, rcp[c]) : -d / u0;
                 const double w = fabs(x) < 700.0 ? exp_r(x) : mgcm_rt_exp(x);
-                v = u0 * sol[nw] * w;
-                v = ng < D_NG - 1 ? v * K.gweight[ng] * (1.0 - K.fzerov[nw]) : v * K.fzerov[nw];
+                v = u0 * sl[e] * w * wa[e] * wb[e];
             }
-            term[c * DSOL_ROW + nw * D_NG + ng] = v;
+            term[c * DSOL_ROW + at[e]] = v;
         }
     }
     __syncthreads();
-    if (t < nc) {
+    if (t < nday) {
         double ds = 0.0;
-        if (u0s[t] >= R4(1.0e-5))
-            for (int q = 0; q < NSYS_V; ++q) ds = ds + term[t * DSOL_ROW + q];
-        dnvflux[c0 + t] = dndiffv[c0 + t] + ds;
+        for (int q = 0; q < NSYS_V; ++q) ds = ds + term[t * DSOL_ROW + q];
+        dnvflux[c0 + day[t]] = dndiffv[c0 + day[t]] + ds;
     }
 }
 size_t dsolflux_ctas(int ncol) { return (size_t)(ncol + DSOL_COLS - 1) / DSOL_COLS; }
