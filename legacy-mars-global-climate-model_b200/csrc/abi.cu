@@ -297,6 +297,7 @@ struct Slot {
     uint32_t *d_status = nullptr, *h_status = nullptr;
     unsigned long long *d_nsys = nullptr, *h_nsys = nullptr;
     Arena stage, pipe, aero;   // aero: per-level aerosol arrays of tracer jobs
+    int two_nl = 0, two_cols = 0;   // columns up to which the reduce takes two warps each
     int occ_nl = 0, occ_rb = 0, occ_rw = 0, occ_stage = 1, occ_screen = 1, occ_solve = 1, occ_quad = 1, occ_reduce = 1;
     bool busy = false;
     Job job;
@@ -641,13 +642,13 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
     // columns are resident even so (60 / 200 / 400 / 592 x 24 columns: 167 / 182 /
     // 222 / 247 -> 155 / 169 / 210 / 238 us a call; 540 x 48, not all resident:
     // 509 -> 520)
-    int rw = 1;
-    if (chunk <= 4 * h->num_sms) {
+    if (sl.two_nl != max_nl) {
+        sl.two_nl = max_nl;
         int two = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, reduce_kernel(rb), 64, reduce_smem_bytes(max_nl, 2));
-        // (the carve-out preference, half of the shared memory, halves it)
-        if (chunk <= std::max(two / 2, 1) * h->num_sms) rw = 2;
+        sl.two_cols = std::max(two / 2, 1) * h->num_sms;   // the carve-out, half of the shared memory, halves it
     }
+    const int rw = chunk <= std::min(sl.two_cols, 4 * h->num_sms) ? 2 : 1;
     const size_t rsm = reduce_smem_bytes(max_nl, rw);
     const bool mixed = h->cfg.precision == MGCM_RT_MIXED;
     if (sl.occ_nl != max_nl || sl.occ_rb != rb || sl.occ_rw != rw) {
