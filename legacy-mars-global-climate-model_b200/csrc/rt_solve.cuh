@@ -4,11 +4,16 @@
 // system that leaves it anywhere (`odd`) is redone by the general solve.
 //
 // Range: the stage marks bands with |COSBAR| >= 1 or an unusual scattering
-// numerator (usual_layer); pass A checks that the layer's optical depth is
-// below 2^100 and its albedo in [0, 1), pass C every eliminated denominator
-// (and, visible, the root and the divisor of GAMA).  What else is divided by
-// or rooted then lies in range: 1 - W0 COSB >= 2^-53, and ALPHA within 2^27
-// of 1, EP in [1, exp(35)].
+// numerator (usual_layer); pass A checks that the optical depths of the
+// layer's two levels (visible: and of level 2) are in [0, 2^99) (unusual_depth)
+// and its albedo in [0, 1), pass C every eliminated denominator (and, visible,
+// the root and the divisor of GAMA).  What else is divided by or rooted then
+// lies in range: 1 - W0 COSB >= 2^-53, and ALPHA within 2^27 of 1.  Every
+// depth from the top down to a middle of a layer is a sum of depths that are
+// not negative, so the exponents of the layers' middles are in [0, 35], EP in
+// [1, exp(35)], and those of the beam in [-35, 0].  The sign of the sum of a
+// layer's depths is not enough: with -3000 and 3005 the middle's exponent is
+// -3000, exp_r wraps, and finite values come out for infinities.
 //
 // IR solve of 8,192 x 24 columns: 896 instructions issued per layer and warp
 // in the general arithmetic, 617 in this one.
@@ -35,6 +40,10 @@ union SolveLocal {
     VisSlot vis[D_MAXNL + 1];
     __device__ SolveLocal() {}
 };
+
+// An optical depth outside [0, 2^99): negative (-0 too), infinite or NaN.
+__device__ __forceinline__ bool unusual_depth(double d) { return hi32(d) >= 0x46200000u; }
+__device__ __forceinline__ bool unusual_depths(double a, double b) { return max(hi32(a), hi32(b)) >= 0x46200000u; }
 
 // The general solves, out of line: systems out of range only.  They carve the
 // column block themselves, so that the callers' ColSmem stays in registers.
@@ -202,7 +211,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
             const bool thick = dtsum > tiny;
             const double dt = thick ? dtsum : tiny, ydt = rcp_n(dt);
             const double w0 = thick ? quot(r.wnum, dt, ydt) : 0.0;
-            if (hi32(dt) >= 0x46300000u || hi32(w0) >= 0x3ff00000u) flags |= 1;   // DTAUI < 2^100, 0 <= WBARI < 1
+            if (hi32(w0) >= 0x3ff00000u) flags |= 1;   // 0 <= WBARI < 1
             dt1 = dt;
             Lay y;
             double lam, term;
@@ -222,6 +231,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
         taug = tg;
         flags |= hi32(tg) & 0x80000000u;
         double da = gas ? tg + e.x + e.y : e.x + e.y;
+        if (unusual_depth(da)) flags |= 1;
         w.ir[NL].pair = make_double2(da, 0.0);
         Lay hi = coef(*r, da);
         double as, ds;
@@ -244,6 +254,7 @@ __device__ __forceinline__ int fast_ir(const SegTable *__restrict__ st, int col_
                 da = e1.x + e1.y;
                 db = e2.x + e2.y;
             }
+            if (unusual_depths(da, db)) flags |= 1;
             w.ir[n].pair = make_double2(da, db);
             if (n > 1) {
                 prefetch_l1(r - 1);
@@ -362,6 +373,7 @@ struct VisPassA {
         };
         odd = (*s.odd >> nb) & 1;
         const double tc2 = 0.0 + level(2, lay->ray[1]);
+        odd |= unusual_depth(tc2);
         double tc = tc2, fprev = 0.0;
 #pragma unroll 1
         for (int l = 1; l <= NL; ++l) {
@@ -391,17 +403,19 @@ struct VisPassA {
                     da = lay->ray[0];
                     db = lay->ray[1];
                 }
+                odd |= unusual_depths(da, db);
                 tcA = tc + da;
                 tcB = tcA + db;
                 dt = da + db;
             } else {
                 dt = da = level(k, lay->ray[0]);
+                odd |= unusual_depth(da);
                 tcA = tcB = tc + da;
             }
             const double cosb = lay->cosb;
             const double wb = quot(lay->wnum, dt, rcp_n(dt));
             const double f = 1.0 - wb * (cosb * cosb);
-            odd |= hi32(dt) - 0x2d300000u >= 0x19000000u || hi32(wb) >= 0x3ff00000u;   // [2^-300, 2^100), [0, 1)
+            odd |= hi32(dt) < 0x2d300000u || hi32(wb) >= 0x3ff00000u;   // below 2^-300; outside [0, 1)
             const double dtl = dt * f;
             if (KEEP) {
                 double m = 0.0;
