@@ -10,20 +10,34 @@
 // flag per system) and send such systems through the general code.
 //
 // Every result is the correctly rounded one, so it equals the operators
-// `/` and sqrt() -- and the CPU oracle -- bit for bit:
-//   rcp_n   Newton-Raphson on the hardware approximation (rcp.approx.ftz.f64),
-//           then y' = y + y (1 - b y) with fused multiply-adds, which rounds
-//           1/b correctly from any y within one ulp (P. Markstein,
-//           "Computation of elementary functions on the IBM RISC System/6000
-//           processor", IBM J. Res. Dev. 34(1), 1990) but for a significand of
-//           all ones -- 1 - W0 COSB and 1 + ALPHA of a thin layer -- where
-//           only the upper neighbour y does: hence the iterate rounded up;
-//   quot    q = a y, q' = q + y (a - b q) with y = 1/b rounded: correctly rounded (same paper),
-//           so quotients over one divisor share its reciprocal;
-//   sqrt_n  coupled Newton iterations for sqrt(x) and 1/(2 sqrt(x)) from
-//           rsqrt.approx.ftz.f64, then g' = g + h (x - g g).
-// Compared with CUDA's operators on 6e9 random and structured operands
-// (significands near 1 and near 2, few bits, squares of midpoints): no difference.
+// `/` and sqrt() -- and the CPU oracle -- bit for bit.  "Near a midpoint" below
+// is a value so close to the middle of two doubles that the error stated could
+// change its rounding; u is the distance of the two.
+//   rcp_n   Newton-Raphson, y <- y + y (1 - b y), from the hardware approximation
+//           (rcp.approx.ftz.f64): two steps leave a relative error of 2^-80
+//           before the second one's rounding, upwards, so y is 1/b or up to one
+//           u above it.  The third step is P. Markstein's ("Computation of
+//           elementary functions on the IBM RISC System/6000 processor", IBM J.
+//           Res. Dev. 34(1), 1990): 1 - b y is exact, and y + y (1 - b y) lies
+//           b (y - 1/b)^2 below 1/b.  For a b in [1, 2) 1/b is N 2^-106 / b from
+//           its midpoint, N a whole number, not 0, so it matters for N = 1 .. 4
+//           alone; there y, rounded up, is u/2 = 2^-54 above 1/b, and b^2 / 4 < N.
+//           (Rounded to nearest, y would be u/2 below 1/b for the significand of
+//           all ones -- 1 - W0 COSB and 1 + ALPHA of a thin layer -- and stay.)
+//   quot    q = a y, q' = q + y (a - b q) with y = 1/b rounded (same paper).
+//           q' before its rounding is off a/b by |a/b - q| |b y - 1|, at most
+//           3 b 2^-108 for a < b in [1, 2), u = 2^-53.  a/b is N 2^-106 / b from
+//           its midpoint, so it matters for |N| <= 3 alone; there a y, off by
+//           less than u, rounds to one of the two doubles beside a/b, u/2 from
+//           it, and b^2 / 4 < |N|.  For a >= b both u and the distance are twice
+//           as large, the error of a y is below u/2, and the same holds.  So
+//           quotients over one divisor share its reciprocal;
+//   sqrt_n  Goldschmidt's coupled iterations for sqrt(x) and 1/(2 sqrt(x)) from
+//           rsqrt.approx.ftz.f64, then g' = g + h (x - g g) (P. Markstein,
+//           "Software division and square root using Goldschmidt's algorithms",
+//           6th Conference on Real Numbers and Computers, 2004).
+// tests/test_arithmetic_gpu.py compares them with CUDA's operators, at random
+// operands and at those whose exact results lie nearest to midpoints.
 // exp_r is mgcm_rt_exp (include/mgcm_rt_math.h), operation for operation:
 // rounding to an integer by adding 1.5 2^52, S_j = RN(lead + trail) being
 // lead itself, the scaling by 2^m an addition to the exponent.
@@ -43,9 +57,8 @@ __device__ __forceinline__ bool out_of_range(double x) {
 __device__ __forceinline__ double rcp_n(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    double e = __fma_rn(-b, y, 1.0);
-    e = __fma_rn(e, e, e);
-    y = __fma_ru(y, e, y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    y = __fma_ru(y, __fma_rn(-b, y, 1.0), y);
     return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
 }
 
