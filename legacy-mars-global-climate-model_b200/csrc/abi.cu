@@ -1054,11 +1054,12 @@ int finish_pending(mgcm_rt_handle *h) {
     return status_to_code(stw);
 }
 
-// Column ranges (ends) of a synchronous host-buffer call over n columns: jobs
-// of up to max_job columns.  With first > 0 the jobs ramp up (first, 2 first,
-// ... below max_job) and back down at the end, so the first host-to-device
-// copy and the last device-to-host copy, which no kernel overlaps, are short;
-// the middle is split evenly.
+// Column ranges (ends) of a synchronous call over n columns, split evenly.
+// first = 0: jobs of at most max_job columns.  first > 0 (host buffers): the
+// jobs ramp up (first, 2 first, ... below max_job) and back down at the end, so
+// the first host-to-device copy and the last device-to-host copy, which no
+// kernel overlaps, are short; calls too small for that run as jobs of up to
+// half more than max_job columns rather than with a small last one.
 std::vector<int> job_ends(int n, int max_job, int first) {
     std::vector<int> ramp, ends;
     int ramp_cols = 0;
@@ -1073,8 +1074,7 @@ std::vector<int> job_ends(int n, int max_job, int first) {
         for (int j = 0; j < nj; ++j) ends.push_back(c += mid / nj + (j < mid % nj ? 1 : 0));
         for (auto it = ramp.rbegin(); it != ramp.rend(); ++it) ends.push_back(c += *it);
     } else {
-        // even jobs, up to half larger than max_job rather than a small last one
-        const int nj = std::max(1, (n + max_job / 2) / max_job);
+        const int nj = std::max(1, (n + (first > 0 ? max_job / 2 : max_job - 1)) / max_job);
         for (int j = 0; j < nj && n > 0; ++j) ends.push_back(c += n / nj + (j < n % nj ? 1 : 0));
     }
     return ends;

@@ -1,0 +1,70 @@
+"""Calls that fit a handle's HBM budget by their size keep fitting it: no job
+of a device call is larger than the library's limit."""
+import numpy as np
+import pytest
+
+from mgcm_rt import abi
+
+pytestmark = pytest.mark.gpu
+
+JOB, SLOTS = 32768, 4   # columns per job of a device tracer call at most, jobs in flight
+
+
+def _tracers(n, L, seed=5):
+    """n columns on the device with clear skies and prescribed dust: one ordinary column, repeated."""
+    import torch
+    lev = 2 * L + 3
+    plev = np.geomspace(0.01, 7.0, lev)
+    col = dict(plev=plev, pmid=plev, tlev=np.linspace(160.0, 220.0, lev), tmid=np.linspace(160.0, 220.0, lev),
+               qh2o=np.full(lev, 1e-4), tauref=np.full(lev + 1, 0.01), acosz=0.5, als=0.2, albi=0.05, pcol=plev[-1],
+               detau=np.zeros((17, 7)), cumtauv=np.zeros((17, 7)))
+    b = {k: torch.from_numpy(np.asarray(v, dtype=np.float64)).cuda().expand(*((n,) + np.shape(v))).contiguous()
+         for k, v in col.items()}
+    b.update(ncol=n, L=L, ptrop=0.0008, active_dust=0, cloudon=0,
+             sigma=torch.linspace(0.0, 1.0, lev, dtype=torch.float64).cuda(),
+             sol=torch.full((7,), 50.0, dtype=torch.float64).cuda())
+    return b
+
+
+@pytest.fixture(scope="module")
+def tables(data_dir, tmp_path_factory):
+    """The k tables, with Mie tables of one value each: the tracer calls ask for them."""
+    import shutil
+    from mgcm_rt import data
+    d = tmp_path_factory.mktemp("tables")
+    for name in data.REQUIRED:
+        shutil.copy(data_dir / name, d / name)
+    for name, n in ((data.ICE_VIS_FILE, 15 * 20 * 3 * 7), (data.ICE_IR_FILE, 15 * 20 * 3 * 5),
+                    ("Dust_vis_wolff2010_JD_12bands.dat", 20 * 3 * 7), ("Dust_ir_wolff2010_JD_12bands.dat", 20 * 3 * 5)):
+        (d / name).write_text("0.5\n" * n)
+    return d
+
+
+def _radiation(tables, L, budget=0):
+    return abi.Radiation(tables, max_layers=L, precision=abi.FP64, hbm_budget=budget)
+
+
+def _used(tables, L, call):
+    rt = _radiation(tables, L)
+    try:
+        call(rt)
+        return rt.stats()["hbm_used"]
+    finally:
+        rt.close()
+
+
+def test_device_tracer_jobs_stay_within_their_limit(tables):
+    """The budget of as many jobs as run at once, each of the largest size,
+    holds a call of any size."""
+    most = _tracers(180000, 1)
+
+    def call(rt, n):
+        b = {k: v[:n] if hasattr(v, "shape") and v.shape[0] == 180000 else v for k, v in most.items()}
+        out = rt.run_tracers(dict(b, ncol=n), inplace=True)
+        assert bool((out["fluxdni"] == out["fluxdni"][0]).all())   # one column, n times
+    rt = _radiation(tables, 1, _used(tables, 1, lambda rt: call(rt, SLOTS * JOB)))
+    try:
+        for n in (SLOTS * JOB, SLOTS * JOB + 1, 147455, 180000):
+            call(rt, n)
+    finally:
+        rt.close()
