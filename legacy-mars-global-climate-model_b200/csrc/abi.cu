@@ -299,6 +299,7 @@ struct Slot {
     Arena stage, pipe, aero;   // aero: per-level aerosol arrays of tracer jobs
     int two_nl = 0, two_cols = 0;   // columns up to which the reduce takes two warps each
     int occ_nl = 0, occ_rb = 0, occ_rw = 0, occ_stage = 1, occ_screen = 1, occ_solve = 1, occ_quad = 1, occ_reduce = 1;
+    bool served = false;   // the serving thread's
     bool busy = false;
     Job job;
     int kernels = 0;
@@ -490,9 +491,8 @@ int after_legacy_stream(Slot &sl, cudaStream_t st) {
     return MGCM_RT_OK;
 }
 
-// Grows an arena within the handle's HBM budget (arenas never shrink).
-int arena_ensure(mgcm_rt_handle *h, Arena &a, size_t bytes, cudaStream_t s) {
-    if (a.bytes >= bytes) return MGCM_RT_OK;
+// Grows an arena within the handle's HBM budget.
+int arena_grow(mgcm_rt_handle *h, Arena &a, size_t bytes, cudaStream_t s) {
     std::lock_guard<std::mutex> lk(h->mem_mu);
     if (h->used - a.bytes + bytes > h->budget) return MGCM_RT_ENOMEM;
     if (a.ptr) {
@@ -502,10 +502,48 @@ int arena_ensure(mgcm_rt_handle *h, Arena &a, size_t bytes, cudaStream_t s) {
     }
     a.ptr = nullptr;
     a.bytes = 0;
-    if (cudaMalloc(&a.ptr, bytes) != cudaSuccess) return MGCM_RT_ENOMEM;
+    if (cudaMalloc(&a.ptr, bytes) != cudaSuccess) {
+        a.ptr = nullptr;
+        (void)cudaGetLastError();   // reported here, not by the next launch
+        return MGCM_RT_ENOMEM;
+    }
     a.bytes = bytes;
     h->used += bytes;
     return MGCM_RT_OK;
+}
+
+// Frees the arenas of the synchronous slots other than sl, after the work on
+// them; false if there are none, or (serving thread) if a synchronous call is
+// under way.
+bool release_arenas(mgcm_rt_handle *h, const Slot &sl) {
+    std::unique_lock<std::mutex> lk(h->mu, std::defer_lock);
+    if (sl.served && !lk.try_lock()) return false;   // other callers hold it
+    bool freed = false;
+    for (auto &s : h->slots) {
+        if (s.get() == &sl) continue;
+        for (Arena *a : {&s->stage, &s->pipe, &s->aero})
+            if (a->ptr) {
+                cudaStreamSynchronize(s->stream);
+                if (s == h->slots[0]) cudaStreamSynchronize(sync_stream(h));
+                cudaFree(a->ptr);
+                std::lock_guard<std::mutex> mk(h->mem_mu);
+                h->used -= a->bytes;
+                *a = Arena{};
+                freed = true;
+            }
+    }
+    return freed;
+}
+
+// An arena of slot sl with room for `bytes`.  Arenas are kept from call to
+// call, and calls of other sizes split over the slots in other ways (15,900 x
+// 24 columns into 2 parts, 16,200 x 24 into 4), so that what the slots keep can
+// add up to more than the largest call needs: where the budget (or the
+// device) has no room left, the idle slots' arenas are given back first.
+int arena_ensure(mgcm_rt_handle *h, Slot &sl, Arena &a, size_t bytes, cudaStream_t s) {
+    if (a.bytes >= bytes) return MGCM_RT_OK;
+    const int rc = arena_grow(h, a, bytes, s);
+    return rc == MGCM_RT_ENOMEM && release_arenas(h, sl) ? arena_grow(h, a, bytes, s) : rc;
 }
 
 // The input checks as a kernel of their own, for the forms without rt_stage.
@@ -625,7 +663,7 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
     const size_t need = al((size_t)chunk * stride) + al(n_v * 4) + al(n_i * 4) + al(r_v * row) +
                         al(r_i * row) + al(r_v * 32) + al(r_i * 32) + 256;
     (void)per_col;
-    int rc = arena_ensure(h, sl.pipe, need, st);
+    int rc = arena_ensure(h, sl, sl.pipe, need, st);
     if (rc) return rc;
     unsigned char *p = static_cast<unsigned char *>(sl.pipe.ptr);
     auto take = [&](size_t b) { unsigned char *r = p; p += al(b); return r; };
@@ -801,7 +839,7 @@ int launch_fused(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int ncols, int ma
     size_t stride = 0;
     pipe_bytes_per_col(max_nl, &stride);
     const size_t cta = (fused_scratch_per_cta(sh.tc, max_nl, stride) + 255) / 256 * 256;
-    const int rc = arena_ensure(h, sl.pipe, cta * grid + 256, st);
+    const int rc = arena_ensure(h, sl, sl.pipe, cta * grid + 256, st);
     if (rc) return rc;
     unsigned char *scr = static_cast<unsigned char *>(sl.pipe.ptr);
     unsigned int *ctr = reinterpret_cast<unsigned int *>(scr + cta * grid);
@@ -878,7 +916,7 @@ int issue_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt_batch_
         arrs = arrays_of(in, out, z, sd);
         size_t bytes = ((z.lev + 8) * 8 + 255) / 256 * 256;
         for (const auto &a : arrs) bytes += ((a.per_col * n * 8 + 255) / 256) * 256;
-        const int rc = arena_ensure(h, sl.stage, bytes, st);
+        const int rc = arena_ensure(h, sl, sl.stage, bytes, st);
         if (rc) return rc;
         char *base = static_cast<char *>(sl.stage.ptr);
         size_t off = 0;
@@ -1318,7 +1356,7 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
     } else {
         size_t bytes = ((lev + 8) * 8 + 255) / 256 * 256;
         for (const auto &a : arrs) bytes += ((a.per_col * n * 8 + 255) / 256) * 256;
-        const int rc = arena_ensure(h, sl.stage, bytes, st);
+        const int rc = arena_ensure(h, sl, sl.stage, bytes, st);
         if (rc) return rc;
         char *base = static_cast<char *>(sl.stage.ptr);
         size_t off = 0;
@@ -1344,7 +1382,7 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
     const size_t per = (size_t)lev1 * (2 + 3 * (AERO_NV + AERO_NI));
     const size_t prep_per = stt ? (size_t)5 * lev + lev1 : 0;
     const size_t abytes = n * (per * ((in.active_dust ? 1 : 0) + (in.cloudon ? 1 : 0)) + prep_per) * 8;
-    int rc = arena_ensure(h, sl.aero, abytes, st);
+    int rc = arena_ensure(h, sl, sl.aero, abytes, st);
     if (rc) return rc;
     double *ap = static_cast<double *>(sl.aero.ptr);
     auto take = [&](size_t per_col) { double *r = ap; ap += per_col * n; return r; };
@@ -1565,6 +1603,7 @@ void worker_main(mgcm_rt_handle *h) {
             if (!free_slot && (int)h->sslots.size() < SERVE_SLOTS) {
                 auto s = std::make_unique<Slot>();
                 if (slot_init(*s) == MGCM_RT_OK) {
+                    s->served = true;
                     h->sslots.push_back(std::move(s));
                     free_slot = h->sslots.back().get();
                 }
@@ -1862,7 +1901,7 @@ int mgcm_rt_dsolflux(mgcm_rt_handle *h, int ncol, int device_ptrs, const double 
     if (!device_ptrs) {
         const size_t n = (size_t)ncol;
         const size_t bytes = 8 * (8 + n + 119 * n + n + n) + 5 * 256;
-        rc = arena_ensure(h, sl.stage, bytes, st);
+        rc = arena_ensure(h, sl, sl.stage, bytes, st);
         if (rc) return rc;
         double *p = static_cast<double *>(sl.stage.ptr);
         double *pa = p + 8, *pd = pa + n, *pn = pd + 119 * n, *po = pn + n;

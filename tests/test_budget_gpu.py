@@ -68,3 +68,75 @@ def test_device_tracer_jobs_stay_within_their_limit(tables):
             call(rt, n)
     finally:
         rt.close()
+
+
+@pytest.mark.parametrize("before, n", [(15900, 16200), (3300, 3199)])
+def test_earlier_calls_do_not_narrow_the_budget(tables, before, n):
+    """A call that fits the budget on a new handle fits it after a call that
+    was split into other parts: 15,900 x 24 columns run as 2 jobs, 16,200 as 4;
+    3,300 as 2, 3,199 as one."""
+    b = _tracers(max(before, n), 24)
+
+    def call(rt, m):
+        return rt.run_tracers(dict({k: v[:m] if hasattr(v, "shape") and v.shape[0] == b["ncol"] else v
+                                    for k, v in b.items()}, ncol=m), inplace=True)
+    budget = max(_used(tables, 24, lambda rt: call(rt, before)), _used(tables, 24, lambda rt: call(rt, n)))
+    rt = _radiation(tables, 24, budget)
+    try:
+        want = {k: v.cpu() for k, v in call(rt, before).items()}
+        for m in (n, before, n):
+            got = call(rt, m)
+            assert rt.stats()["hbm_used"] <= budget
+            for k, v in want.items():
+                assert bool((got[k].cpu()[:1] == v[:1]).all()), k
+    finally:
+        rt.close()
+
+
+def test_host_calls_after_one_another(data_dir):
+    """The same for host buffers: one job of 3,000 columns, then three of 2,000."""
+    from mgcm_rt import synth
+    b = synth.make_batch(6000, L=2, seed=8, cloud=False)
+    few = {k: v[:3000] if isinstance(v, np.ndarray) and v.shape[0] == 6000 else v for k, v in b.items()}
+    few["ncol"] = 3000
+    budget = _used(data_dir, 2, lambda rt: rt.run(b))
+    rt = _radiation(data_dir, 2, budget)
+    try:
+        a, c = rt.run(few), rt.run(b)
+        assert rt.stats()["hbm_used"] <= budget
+        for k, v in a.items():
+            assert np.array_equal(v, c[k][:3000]), k
+    finally:
+        rt.close()
+
+
+def test_request_after_calls(tables):
+    """A budget that holds a call and a request holds them after another call too."""
+    import torch
+    from mgcm_rt import synth
+    t = _tracers(16200, 24)
+    b = synth.make_batch(8000, L=24, seed=9, cloud=False)
+    b = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() if isinstance(v, np.ndarray) else v for k, v in b.items()}
+
+    def call(rt, m):
+        rt.run_tracers(dict({k: v[:m] if hasattr(v, "shape") and v.shape[0] == 16200 else v for k, v in t.items()},
+                            ncol=m), inplace=True)
+
+    def request(rt):
+        ticket, out = rt.submit(b)
+        rt.wait(ticket, 60.0)
+        return {k: v.cpu().numpy() for k, v in out.items()}
+    budget = _used(tables, 24, lambda rt: call(rt, 16200)) + _used(tables, 24, request)
+    rt = _radiation(tables, 24)
+    want = request(rt)
+    rt.close()
+    rt = _radiation(tables, 24, budget)
+    try:
+        call(rt, 15900)
+        call(rt, 16200)
+        for k, v in request(rt).items():
+            assert np.array_equal(v, want[k]), k
+        call(rt, 15900)
+        assert rt.stats()["hbm_used"] <= budget
+    finally:
+        rt.close()
