@@ -640,7 +640,7 @@ int configure_kernels(int device) {
 constexpr int DENSE_V_COLS_PER_SM = 3;
 
 size_t pipe_bytes_per_col(int max_nl, size_t *stride_out = nullptr) {
-    const size_t stride = (col_smem_bytes(max_nl, false) + 255) / 256 * 256;
+    const size_t stride = (col_block_bytes(max_nl) + 255) / 256 * 256;
     if (stride_out) *stride_out = stride;
     const size_t row = (size_t)2 * max_nl * sizeof(double);
     return stride + NSYS * (sizeof(int) + row + 4 * sizeof(double));

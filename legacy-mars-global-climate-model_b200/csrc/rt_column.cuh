@@ -63,15 +63,16 @@ struct ColSmem {
     VisLayer *lay_v;                    // [7][pitch]
     int pitch;                          // the launch's largest NL + 1
     double *bsurf_i, *pltop_i;          // [5]
-    // reduction staging
+    // reduction staging: null in the pipeline's and the fused kernel's blocks
+    // (col_block_bytes), whose fluxes go elsewhere
     double *fmp, *fmm;                  // [sys][l]
     double *sc0, *sc1, *sc2;            // [sys] FLUXUP, FLUXDN, DIFFV (vis) / FTOPUP (IR)
     unsigned char *skip;                // [sys] 0 = solved, 1 = TLIMIT skip, 2 = no work
     int *meta;                          // [2*SCREEN_GROUPS] list base/count of kept systems per group
     int *odd;                           // bands (bit nw-1 visible, 7+nw-1 IR) with a layer outside the
                                         // range of the solves' fast arithmetic (rt_solve.cuh)
-    double *fmnet_v, *fmnet_i;          // [l] reduced net fluxes for the divergences
-    double *misc;                       // [4] NFLUXTOPV, NFLUXTOPI
+    double *fmnet_v, *fmnet_i;          // [l] reduced net fluxes for the divergences (reduction staging)
+    double *misc;                       // [4] NFLUXTOPV, NFLUXTOPI (reduction staging)
     int day;
     // the records of layer l, IR / visible band nw (1-based)
     __device__ __forceinline__ IrLayer &ir(int l, int nw) const { return lay_i[(nw - 1) * pitch + l]; }
@@ -103,6 +104,11 @@ __host__ __device__ inline size_t col_smem_bytes(int nl, bool red_in_smem = true
     return b;
 }
 
+// The same as a block of global memory without the reduction staging.
+__host__ __device__ inline size_t col_block_bytes(int nl) {
+    return col_smem_bytes(nl, false) - (3 * NSYS + 2 * (nl + 1) + 4) * sizeof(double);
+}
+
 __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_global = nullptr,
                                      bool with_red = true) {
     ColSmem s;
@@ -122,7 +128,7 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
     s.bsurf_i = take(D_NI);
     s.pltop_i = take(D_NI);
     if (!with_red) {
-        s.fmp = s.fmm = nullptr;
+        s.fmp = s.fmm = s.sc0 = s.sc1 = s.sc2 = s.fmnet_v = s.fmnet_i = s.misc = nullptr;
     } else if (red_global) {
         s.fmp = red_global;
         s.fmm = red_global + (size_t)NSYS * nl;
@@ -130,12 +136,14 @@ __device__ inline ColSmem carve_smem(unsigned char *base, int nl, double *red_gl
         s.fmp = take((size_t)NSYS * nl);
         s.fmm = take((size_t)NSYS * nl);
     }
-    s.sc0 = take(NSYS);
-    s.sc1 = take(NSYS);
-    s.sc2 = take(NSYS);
-    s.fmnet_v = take(nl + 1);
-    s.fmnet_i = take(nl + 1);
-    s.misc = take(4);
+    if (with_red) {
+        s.sc0 = take(NSYS);
+        s.sc1 = take(NSYS);
+        s.sc2 = take(NSYS);
+        s.fmnet_v = take(nl + 1);
+        s.fmnet_i = take(nl + 1);
+        s.misc = take(4);
+    }
     int *ip = reinterpret_cast<int *>(d);
     s.skip = reinterpret_cast<unsigned char *>(ip);
     s.meta = reinterpret_cast<int *>(((reinterpret_cast<uintptr_t>(s.skip + NSYS) + 15) / 16) * 16);

@@ -140,3 +140,19 @@ def test_request_after_calls(tables):
         assert rt.stats()["hbm_used"] <= budget
     finally:
         rt.close()
+
+
+@pytest.mark.parametrize("L, budget", [(24, 115838464), (48, 213642752), (99, 421348864)])
+def test_scratch_of_a_column(data_dir, L, budget):
+    """1,000 columns fit the scratch that a column block of plain arrays (no
+    padded records) takes with the flux rows of its 204 systems."""
+    import torch
+    from mgcm_rt import synth
+    b = synth.make_batch(1000, L=L, seed=4, cloud=False)
+    b = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() if isinstance(v, np.ndarray) else v for k, v in b.items()}
+    rt = _radiation(data_dir, L, budget)
+    try:
+        ticket, _ = rt.submit(b)
+        rt.wait(ticket, 60.0)
+    finally:
+        rt.close()
