@@ -966,15 +966,14 @@ int issue_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt_batch_
 //   8,192 x 24: 1,396 / 1,258 / 1,250 / 1,313    8,640 x 36: 2,325 / 2,129 / 2,132 / 2,304
 //   16,200 x 24: 2,574 / 2,366 / 2,380 / 2,341   16,200 x 48: 6,334 / 5,866 / 5,847 / 5,834
 constexpr long long SPLIT2_LAYERS = 80000, SPLIT4_LAYERS = 400000;
-int parts_of_layers(long long layers) {
-    return layers < SPLIT2_LAYERS ? 1 : (layers < SPLIT4_LAYERS ? 2 : SYNC_SLOTS);
+int parts_of_layers(const mgcm_rt_handle *h, long long layers) {
+    return h->fused || layers < SPLIT2_LAYERS ? 1 : (layers < SPLIT4_LAYERS ? 2 : SYNC_SLOTS);
 }
 int parts_of(const mgcm_rt_handle *h, int nbatch, const mgcm_rt_batch_in *in) {
     long long layers = 0;
     for (int b = 0; b < nbatch; ++b) layers += (long long)sizes_of(in[b]).ncol * sizes_of(in[b]).nl;
-    return h->fused ? 1 : parts_of_layers(layers);
+    return parts_of_layers(h, layers);
 }
-
 
 // Segment table of the global columns [b0, b1) of the batches, every
 // per-column pointer shifted to the segment's first column in the range;
@@ -1487,7 +1486,7 @@ int run_tracers(mgcm_rt_handle *h, const mgcm_rt_batch_tracers &in, mgcm_rt_batc
     int nk = 0, k = 0;
     bool used[JOB_SLOTS] = {};
     // device inputs: as many concurrent jobs as a device-pointer call has parts
-    const int parts = parts_of_layers((long long)in.ncol * (in.nlayers + 1));
+    const int parts = parts_of_layers(h, (long long)in.ncol * (in.nlayers + 1));
     const std::vector<int> ends = in.device_ptrs ? job_ends(in.ncol, std::min(4 * SYNC_JOB_COLS, (in.ncol + parts - 1) / parts), 0)
                                                  : job_ends(in.ncol, host_job_cols(in.ncol), SYNC_RAMP_COLS);
     int c0 = 0;
