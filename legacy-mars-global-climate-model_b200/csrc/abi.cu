@@ -1459,7 +1459,7 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
     CK(cudaGetLastError());
     rc = launch_all(h, sl, st, (int)n, nl, 1 << 30);
     if (rc) return rc;
-    sl.kernels += stt ? 2 : 1;   // rt_aerosol (+ rt_prep)
+    sl.kernels += (tasks ? 1 : 0) + (stt ? 1 : 0);   // rt_aerosol, rt_prep
     if (!in.device_ptrs)
         for (auto &a : arrs)
             if (a.dir != 0)

@@ -27,3 +27,10 @@ def _cloudy(n):
 def test_fused_tracer_calls_run_unsplit(tables, n):
     """Input checks, aerosol optics and one persistent kernel."""
     assert _kernels(tables, _cloudy(n), solver=abi.SOLVER_FUSED) == 3
+
+
+def test_aerosol_kernel_counted_where_it_runs(tables):
+    """Prescribed dust and clear skies have no aerosol optics to compute: the
+    four kernels of a small call; with clouds rt_aerosol is the fifth."""
+    assert _kernels(tables, _tracers(60, 24)) == 4
+    assert _kernels(tables, _cloudy(60)) == 5
