@@ -297,7 +297,7 @@ struct Slot {
     uint32_t *d_status = nullptr, *h_status = nullptr;
     unsigned long long *d_nsys = nullptr, *h_nsys = nullptr;
     Arena stage, pipe, aero;   // aero: per-level aerosol arrays of tracer jobs
-    int two_nl = 0, two_cols = 0;   // columns up to which the reduce takes two warps each
+    int two_nl = 0, two_rb = 0, two_cols = 0;   // columns up to which the reduce takes two warps each
     int occ_nl = 0, occ_rb = 0, occ_rw = 0, occ_stage = 1, occ_screen = 1, occ_solve = 1, occ_quad = 1, occ_reduce = 1;
     bool served = false;   // the serving thread's
     bool busy = false;
@@ -680,8 +680,9 @@ int launch_pipeline(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, int total, int
     // columns are resident even so (60 / 200 / 400 / 592 x 24 columns: 167 / 182 /
     // 222 / 247 -> 155 / 169 / 210 / 238 us a call; 540 x 48, not all resident:
     // 509 -> 520)
-    if (sl.two_nl != max_nl) {
+    if (sl.two_nl != max_nl || sl.two_rb != rb) {
         sl.two_nl = max_nl;
+        sl.two_rb = rb;
         int two = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&two, reduce_kernel(rb), 64, reduce_smem_bytes(max_nl, 2));
         sl.two_cols = std::max(two / 2, 1) * h->num_sms;   // the carve-out, half of the shared memory, halves it
