@@ -1275,6 +1275,7 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
     as.L = L;
     as.active_dust = in.active_dust ? 1 : 0;
     as.cloudon = in.cloudon ? 1 : 0;
+    const double *tauref_in = nullptr;   // prescribed dust: TAUREF as given or prepared
     std::vector<ArrSpec> arrs;
     auto add_in = [&](const double *p, size_t per, const double **f) {
         if (p) arrs.push_back({p, nullptr, per, 0, const_cast<double **>(f)});
@@ -1285,14 +1286,14 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
     double *prep_want[6] = {};
     double **prep_field[6] = {const_cast<double **>(&sd.plev), const_cast<double **>(&sd.tlev),
                               const_cast<double **>(&sd.pmid), const_cast<double **>(&sd.tmid),
-                              const_cast<double **>(&sd.qh2o), const_cast<double **>(&as.tauref_in)};
+                              const_cast<double **>(&sd.qh2o), const_cast<double **>(&tauref_in)};
     if (!stt) {
         add_in(in.plev, lev, &sd.plev);
         add_in(in.tlev, lev, &sd.tlev);
         add_in(in.pmid, lev, &sd.pmid);
         add_in(in.tmid, lev, &sd.tmid);
         add_in(in.qh2o, lev, &sd.qh2o);
-        if (!in.active_dust) add_in(in.tauref, lev1, &as.tauref_in);
+        if (!in.active_dust) add_in(in.tauref, lev1, &tauref_in);
     } else {
         ps.ncol = (int)n;
         ps.L = L;
@@ -1398,7 +1399,7 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
         ps.pmid = const_cast<double *>(sd.pmid);
         ps.tmid = const_cast<double *>(sd.tmid);
         ps.qh2o = const_cast<double *>(sd.qh2o);
-        ps.tauref = const_cast<double *>(as.tauref_in);
+        ps.tauref = const_cast<double *>(tauref_in);
     }
     if (in.active_dust) {
         as.tauref = take(lev1);
@@ -1425,7 +1426,7 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
         sd.dust_band = h->d_mie + AERO_MIE_SIZE;
         as.tauref = nullptr;   // rt_aerosol leaves the dust alone
     }
-    sd.tauref = in.active_dust ? as.tauref : as.tauref_in;
+    sd.tauref = in.active_dust ? as.tauref : tauref_in;
     sd.qextrefdst = as.qextrefdst;
     sd.qxvdst = as.qxvdst;
     sd.qsvdst = as.qsvdst;
@@ -1762,12 +1763,6 @@ mgcm_rt_handle *mgcm_rt_create(const mgcm_rt_config *cfg, const char *data_dir, 
             AeroConst &A = h->aero;
             std::memcpy(A.radb, at.radb, sizeof(A.radb));
             for (int j = 0; j < AERO_NRATIO; ++j) A.cor_ratio[j] = (float)at.cor_ratio[j];
-            std::memcpy(A.qextv, at.qextv, sizeof(A.qextv));
-            std::memcpy(A.qscatv, at.qscatv, sizeof(A.qscatv));
-            std::memcpy(A.gv, at.gv, sizeof(A.gv));
-            std::memcpy(A.qexti, at.qexti, sizeof(A.qexti));
-            std::memcpy(A.qscati, at.qscati, sizeof(A.qscati));
-            std::memcpy(A.gi, at.gi, sizeof(A.gi));
             std::vector<double> mie;
             mie.reserve(AERO_MIE_SIZE);
             for (int m = 0; m < 3; ++m)
@@ -1785,8 +1780,8 @@ mgcm_rt_handle *mgcm_rt_create(const mgcm_rt_config *cfg, const char *data_dir, 
                     for (int i = 0; i < AERO_NBIN; ++i)
                         for (int l = 0; l < AERO_NI; ++l) mie.push_back(at.cld_i[m][j][i][l]);
             // then the prescribed dust band properties (SegDev::dust_band order)
-            for (const double *p : {A.qextv, A.qscatv, A.gv}) mie.insert(mie.end(), p, p + AERO_NV);
-            for (const double *p : {A.qexti, A.qscati, A.gi}) mie.insert(mie.end(), p, p + AERO_NI);
+            for (const double *p : {at.qextv, at.qscatv, at.gv}) mie.insert(mie.end(), p, p + AERO_NV);
+            for (const double *p : {at.qexti, at.qscati, at.gi}) mie.insert(mie.end(), p, p + AERO_NI);
             if (cudaMalloc(&h->d_mie, mie.size() * 8) ||
                 cudaMemcpy(h->d_mie, mie.data(), mie.size() * 8, cudaMemcpyHostToDevice))
                 return fail(MGCM_RT_ENOMEM);

@@ -14,21 +14,19 @@ constexpr int AERO_MIE_SIZE = AERO_DST_SIZE + 3 * AERO_NRATIO * AERO_NBIN * (AER
 struct AeroConst {
     double radb[AERO_NBIN + 1];    // radb_rt (code/initcld.f:141-156)
     float cor_ratio[AERO_NRATIO];  // REAL*4 core ratios (cldcommon_h)
-    double qextv[AERO_NV], qscatv[AERO_NV], gv[AERO_NV];   // prescribed dust (setrad)
-    double qexti[AERO_NI], qscati[AERO_NI], gi[AERO_NI];
 };
 
 // One batch: tracers in ([ncol][L]), full per-level arrays out (layout of
 // mgcm_rt_batch_in).  Device pointers.
 struct AeroSeg {
     int ncol, L, active_dust, cloudon;
-    const double *plev, *tauref_in;
+    const double *plev;
     const double *dust_mass, *dust_number, *ice_mass, *ice_core, *ice_number;
     double *tauref, *qextrefdst, *qxvdst, *qsvdst, *gvdst, *qxidst, *qsidst, *gidst;
     double *taurefcld, *qextrefcld, *qxvcld, *qsvcld, *gvcld, *qxicld, *qsicld, *gicld;
 };
 
-constexpr int AERO_WARPS = 4;   // columns (warps) per CTA of rt_aerosol
+constexpr int AERO_WARPS = 4;   // warps per CTA of rt_aerosol
 __global__ void rt_aerosol(const AeroSeg a, const __grid_constant__ AeroConst K, const double *__restrict__ mie);
 
 }  // namespace mgcm

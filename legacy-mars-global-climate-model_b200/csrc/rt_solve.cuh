@@ -379,7 +379,7 @@ struct VisPassA {
         for (int l = 1; l <= NL; ++l) {
             const int k = 2 * l + 1;
             ++lay;
-            if (true && l < NL) {
+            if (l < NL) {
                 prefetch_l1(lay + 1);
                 prefetch_l1(s.klev + k + 2);
             }
