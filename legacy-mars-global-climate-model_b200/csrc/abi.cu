@@ -1118,9 +1118,10 @@ std::vector<int> job_ends(int n, int max_job, int first) {
     return ends;
 }
 
-// Columns per job of a synchronous host-buffer call: an eighth of the call
-// within [2,048, SYNC_JOB_COLS], so that mid-sized calls overlap their copies
-// with kernels too (jobs of 8,192 -> this: tracers 16,200 x 24 4.99 -> 4.02 ms,
+// Columns per job that a synchronous host-buffer call asks for (job_ends): an
+// eighth of the call within [2,048, SYNC_JOB_COLS], so that mid-sized calls
+// overlap their copies with kernels too; up to 3,071 columns run as one job,
+// whose copies nothing overlaps (jobs of 8,192 -> this: tracers 16,200 x 24 4.99 -> 4.02 ms,
 // state 16,200 x 24 4.07 -> 3.61, arrays 6,000 x 36 5.42 -> 4.35; jobs of 1,024
 // and less are slower from 16,200 columns on).
 int host_job_cols(int n) { return std::min(SYNC_JOB_COLS, std::max(2048, (n + 7) / 8)); }
@@ -1473,8 +1474,8 @@ int issue_tracer_job(mgcm_rt_handle *h, Slot &sl, cudaStream_t st, const mgcm_rt
     return MGCM_RT_OK;
 }
 
-// Synchronous tracer (or state) batch: jobs alternate between the two
-// synchronous slots.
+// Synchronous tracer (or state) batch: jobs rotate over JOB_SLOTS synchronous
+// slots.
 int run_tracers(mgcm_rt_handle *h, const mgcm_rt_batch_tracers &in, mgcm_rt_batch_out &out,
                 const mgcm_rt_batch_state *stt = nullptr) {
     cudaStream_t ust = sync_stream(h);

@@ -340,8 +340,8 @@ template __global__ void rt_quad_solve<false, 13>(QUAD_ARGS);
 // the buffer without bank conflicts.  8,192 x 24 columns: 255 -> 191 us against
 // loading the rows lane by level straight from global memory, 32 cache lines
 // a value, which ran at 76% of the L1's tag rate; what bounds it now is the
-// latency of its short phases at 9 warps per SM (the carve-out set beside its
-// attributes; issue 27%, 2.3 TB/s).  32 systems at a time: the same at 24
+// latency of its short phases at 8 warps per SM (the carve-out set beside its
+// attributes; issue 29%, 2.4 TB/s).  32 systems at a time: the same at 24
 // layers, 1.5% slower calls at 48.
 constexpr int RED_LPL = (D_MAXNL + 2 + 31) / 32;   // items (levels and two scalar sums) per lane
 constexpr int RED_SYS = 16, RED_PITCH = RED_SYS + 1;   // systems staged at a time
